@@ -1,11 +1,10 @@
 // oic_align.cuh -- warp-cooperative banded prefix edit distance (furthest-reaching
 // diagonals) and the per-read-pair driver around it.
 //
-// One warp owns one read pair.  Lanes own diagonals of the current error row (lane l
-// takes d = Lc + l, Lc + l + 32, ...); the previous row lives in a shared-memory
-// buffer, every kept row is appended to the warp's traceback arena in HBM, and the
-// slides compare 32 bases per step on the 2-bit packed reads.  The arithmetic is the
-// reference's exactly -- integer rows, the same band pruning against Edit_Match_Limit,
+// One warp owns one read pair.  Lanes own diagonals of the current error row, 32 at a
+// time; the previous row lives in a shared-memory buffer, every kept row is appended to
+// the warp's traceback arena in HBM, and the slides compare 32 bases per step on the reads'
+// bit planes.  The arithmetic is the reference's exactly -- integer rows, the same band pruning against Edit_Match_Limit,
 // the same first-index tie breaks, and the branch-point test in IEEE double with
 // explicitly rounded multiply / subtract / divide (no FMA contraction), as an x86-64
 // build of canu computes it.
@@ -37,7 +36,8 @@ struct AlignCaps {
 struct WarpDP {
   WarpScratch        sc;
   AlignCaps          cap;
-  int               *smA, *smB;     // shared-memory row buffers (bandW ints each)
+  int               *smA, *smB;     // shared-memory row buffers of a group CTA (bandW ints each)
+  int                smOff;         // first int of the warp's slice of smemRows (one-warp rows)
   const int         *eml;           // Edit_Match_Limit
   DevParams          P;
   unsigned long long cells, slides, rows;
@@ -66,55 +66,70 @@ template <int STEP>
 __device__ __forceinline__ int warp_slide0(const SeqView &A, int a0, const SeqView &T, int t0, int m,
                                            unsigned long long &slides) {
   const int lane = threadIdx.x & 31;
-  int       base = 0;
-  while (base < m) {
-    int off = base + lane * 32;
-    int r   = 32;
-    if (off < m) r = match_run32<STEP>(A, a0 + STEP * off, T, t0 + STEP * off);
-    unsigned short_ = __ballot_sync(0xffffffffu, off < m && r < 32);
-    if (short_) {
-      int first = __ffs(short_) - 1;
-      int rr    = __shfl_sync(0xffffffffu, r, first);
-      int run   = base + first * 32 + rr;
-      run       = min(run, m);
-      if (lane == 0) slides += (unsigned long long)run;
-      return run;
+  int       run  = m;
+  for (int base = 0; base < m; base += 32 * 32) {
+    const int off = base + lane * 32;
+    const int r   = off < m ? __clz((int)mismatch32<STEP>(A, a0 + STEP * off, T, t0 + STEP * off)) : 32;
+    const unsigned stop = __ballot_sync(0xffffffffu, r < 32);
+    if (stop) {
+      const int f = __ffs((int)stop) - 1;
+      run         = min(base + f * 32 + __shfl_sync(0xffffffffu, r, f), m);
+      break;
     }
-    base += 32 * 32;
   }
-  if (lane == 0) slides += (unsigned long long)m;
-  return m;
+  if (lane == 0) slides += (unsigned long long)run;
+  return run;
 }
 
 // Traceback of Set_Right_Delta / Set_Left_Delta (prefixEditDistance-forward.C:32-71,
-// -reverse.C:36-93) from row e, diagonal d whose value is `last`.  Lane 0 only.
-// Pushes one entry per indel into out[]; returns the value reached on row 0.
+// -reverse.C:36-93) from row e, diagonal d whose value is `last`, by the whole warp (every
+// argument and result is warp-uniform).  Writes one entry per indel to out[] (by lane 0;
+// a __syncwarp before the caller reads them), their number to nOut; returns the value
+// reached on row 0.
+//
+// A step needs the row above at d - 1, d and d + 1 and moves d by at most one, so the
+// values that the next kTraceRows rows can need lie within a window of 32 diagonals: the
+// warp loads those windows together (one coalesced load per row, all in flight) and walks
+// them with shuffles.  One lane walking the arena by itself waited for an L2 round trip
+// per row.
+constexpr int kTraceRows = 8;
 static __device__ __noinline__ int trace_rows(const WarpDP &w, int e, int d, int last, int *out, int &nOut) {
-  // Pointers and the entry count in registers; the next row's header is loaded one
-  // step ahead (it does not depend on the path), so only the arena reads stay on the
-  // step-to-step dependency chain.
+  static_assert(kTraceRows + 1 <= 15, "the window holds d - kTraceRows - 1 .. d + kTraceRows + 1");
   const int4 *const rowHdr = w.sc.rowHdr;
   const int *const  arena  = w.sc.arena;
-  int  n     = 0;
-  int4 hNext = e > 0 ? rowHdr[e - 1] : make_int4(0, 0, 0, 0);
-  for (int k = e; k > 0; k--) {
-    const int4 h = hNext;
-    if (k > 1) hNext = rowHdr[k - 2];
-    const int off = h.x, L = h.y, R = h.z;
-    const int g0 = (d >= L && d <= R) ? arena[off + d - L] : -2;
-    const int gm = (d - 1 >= L && d - 1 <= R) ? arena[off + d - 1 - L] : -2;
-    const int gp = (d + 1 >= L && d + 1 <= R) ? arena[off + d + 1 - L] : -2;
-    int from = d, mx = 1 + g0;
-    if (gm > mx) { from = d - 1; mx = gm; }
-    if (1 + gp > mx) { from = d + 1; mx = 1 + gp; }
-    if (from == d - 1) {
-      out[n++] = mx - last - 1;
-      last     = gm;
-      d--;
-    } else if (from == d + 1) {
-      out[n++] = last - (mx - 1);
-      last     = gp;
-      d++;
+  const int         lane   = threadIdx.x & 31;
+  const int4        none   = make_int4(0, 1, 0, 0);   // an empty band
+  int  n = 0;
+  // Lane j holds the header of row k - 1 - j; the next block's are loaded a block ahead.
+  int4 hNext = lane < kTraceRows && e - 1 - lane >= 0 ? rowHdr[e - 1 - lane] : none;
+  for (int k = e; k > 0; k -= kTraceRows) {
+    const int4 h  = hNext;
+    const int  kn = k - kTraceRows - 1 - lane;
+    hNext         = lane < kTraceRows && kn >= 0 ? rowHdr[kn] : none;
+    const int d0  = d - 16, dd = d0 + lane;
+    int v[kTraceRows];
+#pragma unroll
+    for (int j = 0; j < kTraceRows; j++) {
+      const int off = __shfl_sync(0xffffffffu, h.x, j), L = __shfl_sync(0xffffffffu, h.y, j),
+                R   = __shfl_sync(0xffffffffu, h.z, j);
+      v[j] = (dd >= L && dd <= R) ? arena[off + dd - L] : -2;
+    }
+#pragma unroll
+    for (int j = 0; j < kTraceRows; j++) {
+      if (j < k) {
+        const int g0 = __shfl_sync(0xffffffffu, v[j], d - d0);
+        const int gm = __shfl_sync(0xffffffffu, v[j], d - 1 - d0);
+        const int gp = __shfl_sync(0xffffffffu, v[j], d + 1 - d0);
+        int from = 0, mx = 1 + g0;
+        if (gm > mx) { from = -1; mx = gm; }
+        if (1 + gp > mx) { from = 1; mx = 1 + gp; }
+        if (from) {
+          if (lane == 0) out[n] = from < 0 ? mx - last - 1 : last - (mx - 1);
+          last = from < 0 ? gm : gp;
+          d += from;
+          n++;
+        }
+      }
     }
   }
   nOut = n;
@@ -126,30 +141,43 @@ __device__ __forceinline__ int arena_get(const WarpDP &w, int e, int d) {
   return (d >= h.y && d <= h.z) ? w.sc.arena[h.x + d - h.y] : -2;
 }
 
-// Set_Right_Delta (forward.C:32-71) into sc.deltaR; lane 0.
+// Set_Right_Delta (forward.C:32-71) into sc.deltaR, whole warp.
 static __device__ __noinline__ void set_right_delta(WarpDP &w, int e, int d, int last) {
+  const int  lane  = threadIdx.x & 31;
+  int *const stack = w.sc.stack;
   int n;
-  int l = trace_rows(w, e, d, last, w.sc.stack, n);
-  w.sc.stack[n++] = l + 1;
-  int k           = 0;
-  for (int i = n - 1; i > 0; i--) {
-    int s = w.sc.stack[i - 1];
-    w.sc.deltaR[k++] = abs(w.sc.stack[i]) * ((s > 0) - (s < 0));
+  const int l = trace_rows(w, e, d, last, stack, n);
+  if (lane == 0) stack[n] = l + 1;
+  __syncwarp();
+  for (int k = lane; k < n; k += 32) {
+    const int s      = stack[n - 1 - k];
+    w.sc.deltaR[k]   = abs(stack[n - k]) * ((s > 0) - (s < 0));
   }
-  w.rightLen = n - 1;
+  w.rightLen = n;
+  __syncwarp();
 }
 
-// Set_Left_Delta (reverse.C:36-93) into sc.deltaL; lane 0.
+// Set_Left_Delta (reverse.C:36-93) into sc.deltaL, whole warp.
 static __device__ __noinline__ void set_left_delta(WarpDP &w, int e, int d, int last, int &leftover, int &tEnd, int tLen) {
+  const int  lane = threadIdx.x & 31;
+  int *const ld   = w.sc.deltaL;
   int n;
-  leftover  = trace_rows(w, e, d, last, w.sc.deltaL, n);
-  int *ld   = w.sc.deltaL;
+  leftover = trace_rows(w, e, d, last, ld, n);
+  __syncwarp();
   if (n > 1 && ld[0] == 1 && tEnd + tLen > 0) {
-    ld[0] = (ld[1] > 0) ? ld[1] + 1 : ld[1] - 1;
-    for (int i = 2; i < n; i++) ld[i - 1] = ld[i];
+    const int l1 = ld[1];
+    __syncwarp();
+    for (int i0 = 2; i0 < n; i0 += 32) {   // drop the first entry
+      const int i = i0 + lane;
+      const int v = i < n ? ld[i] : 0;
+      __syncwarp();
+      if (i < n) ld[i - 1] = v;
+      __syncwarp();
+    }
+    if (lane == 0) ld[0] = (l1 > 0) ? l1 + 1 : l1 - 1;
     n--;
     tEnd--;
-    if (n == 0) leftover++;
+    __syncwarp();
   }
   w.leftLen = n;
 }
@@ -230,8 +258,8 @@ struct RowsOut {
   int  status;
   u32  err;
   int  e, dEnd, eDone;       // end row, first diagonal reaching an end, last kept row
-  int  Lc, Rc, prevBase;     // band of row e and the base of row e-1
-  int *prev, *cur;           // row e-1 and row e buffers
+  int  Rc;                   // right edge of the end row's computed band
+  int  rowEnd, ppEnd;        // value of the end row at dEnd, of the row before it at dEnd + 1
   unsigned long long cells, rows;
 };
 
@@ -241,7 +269,6 @@ struct GroupJob {
   SeqView A, T;
   int     a0, t0;
   int     m, n, errorLimit, step, u;
-  int     first16;           // slides start with the 16-base compare (slide_first16)
   int    *rowA, *rowB;       // row buffers (rowA holds row 0)
 };
 struct GroupShared {
@@ -256,117 +283,300 @@ __device__ __forceinline__ void group_bar(int id, int nThr) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(nThr) : "memory");
 }
 
-// The row loop by one warp.  Row 0 (value r0) is in prev[2].  FIRST16: slides start
-// with a 16-base compare (see slide()).
-template <int STEP, bool FIRST16>
-__device__ __forceinline__ RowsOut warp_rows(WarpDP &w, const SeqView &Aref, int a0, int m, const SeqView &Tref,
-                                             int t0, int n, int errorLimit) {
-  const SeqView A = Aref, T = Tref;   // in registers for the slides
+// Shared memory of a warp's row loop, in ints: two rows of kRowW diagonals, each with
+// kRowPad ints behind it, and the RowJob.
+constexpr int kRowW      = 512;
+constexpr int kRowPad    = 8;
+constexpr int kRowStride = kRowW + kRowPad;
+
+// A row loop's arguments, state between calls and results, in shared memory: what it needs
+// rarely or only for addresses stays out of its registers.
+struct RowJob {
+  SeqView    A, T;
+  int       *arena;
+  int4      *rowHdr;
+  const int *eml;
+  int        a0, t0, step;
+  int        arenaCap, bufW;
+  int        e, L, R, off, base;   // the row to compute; kept band, place and buffer origin of the row before it
+  int        dEnd, Rc, rowEnd, ppEnd;
+  u32        cells;
+  u32        slides[32];           // per lane
+};
+constexpr int kJobInts      = (sizeof(RowJob) + 15) / 16 * 4;
+constexpr int kWarpSmemInts = 2 * kRowStride + kJobInts;
+static_assert(2 * kRowStride % 4 == 0, "RowJob starts on 16 bytes");
+
+extern __shared__ __align__(16) int smemRows[];
+
+// Mismatch mask of 32 bases of A from base ga and T from base gt on in read order (the
+// caller passes the window's low ends); bit 31 is the first base in the direction of the
+// extension.  fwd: forward extension.
+template <bool HASN>
+__device__ __forceinline__ int match_len(const RowJob &job, const uint2 *Ap, int ga, const uint2 *Tp, int gt, bool fwd) {
+  const uint2 x = load_planes(Ap, ga), y = load_planes(Tp, gt);
+  u32 m = (x.x ^ y.x) | (x.y ^ y.y);
+  if (HASN) m = drop_n(m, job.A.nm, ga, job.T.nm, gt);
+  return __clz((int)(fwd ? __brev(m) : m));
+}
+
+// Rows e, e + 1, ... by one warp, from the kept band [L, R] of row e - 1 in the buffer
+// `prev` (first diagonal `base`, arena place `off`).  Buffers of bufW ints.  Returns a
+// RowsOut status, or kRowsWiden when the band outgrew the buffers: row e - 1 is then in the
+// buffer of its parity, and the caller continues in wider ones (WIDE: those in HBM).  A row
+// buffer holds diagonal d at index d - base + 2, with the two diagonals on each side of the
+// kept band set to -2 as the reference does (forward.C:150-153), so the neighbour reads
+// need no bounds tests.
+//
+// What bounds it: instruction issue (64 % of the slots) and the latency of a row.  A row of
+// the 0.5 % reads is 33 diagonals and issues 350 warp instructions, of which the leading
+// diagonal's long slide is a third; with the interleaved 2-bit words, a window of 32 bases
+// cost 60 instructions, the row 520, and the longest slide ran alone, 32 bases per step
+// (150 Mbp of those reads: DP 648 -> 426 ms; 20 Mbp of 2 % reads 346 -> 321 ms).
+// Both directions run the same instructions, and 64 diagonals at a time share one copy of
+// the code for long slides: with a copy per direction and chunk the loop missed the
+// instruction cache (6.9 stall cycles per issue; DP 601 ms).  Keeping each diagonal's
+// mismatch mask from row to row does not pay: inside the band every diagonal moves as fast
+// as the alignment does, so a mask of 32 bases is used up in a row or two (519 ms).
+enum { kRowsWiden = 3 };
+template <bool HASN, bool WIDE>
+static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *rowsG, const int m, const int n,
+                                            const int errorLimit) {
   const int lane = threadIdx.x & 31;
-  RowsOut o;
-  o.status = kRowsDone;
-  o.err = 0;
-  o.e = o.dEnd = o.eDone = 0;
-  o.cells = o.rows = 0;
-  // Row buffers hold diagonal d at index d - base + 2.  Before a row is computed the
-  // two diagonals on each side of the previous row's kept band are set to -2, as the
-  // reference does (forward.C:150-153), so the neighbour reads need no bounds tests.
-  // Loop invariants and the slide counter in registers: the loop stores through
-  // generic pointers, which the compiler cannot tell apart from the WarpDP on the stack.
-  int *const         arena    = w.sc.arena;
-  int4 *const        rowHdr   = w.sc.rowHdr;
-  int *const         rowsG    = w.sc.rowsG;
-  const int *const   eml      = w.eml;
-  const int          rowCap   = w.cap.rowCap;
-  const int          rowsGW   = w.cap.rowsGW;
-  const int          arenaCap = w.cap.arenaCap;
-  unsigned long long slides   = 0;
-  int *prev = w.smA, *cur = w.smB;
-  int  bufW = w.cap.bandW;
-  int  used = 1, prevBase = 0, L = 0, R = 0;
-  for (int e = 1; e <= errorLimit; e++) {
-    if (e >= rowCap) { o.status = kRowsErr; o.err = kErrRowsFull; break; }
+  int *prev = WIDE ? rowsG : smemRows + smOff, *cur = WIDE ? rowsG + job.bufW : prev + kRowStride;
+  const uint2 *const Ap = job.A.p, *const Tp = job.T.p;
+  int *const arena = job.arena;
+  const int  sgn = job.step;
+  const bool fwd = sgn > 0;
+  const int  a0 = job.a0 - (fwd ? 0 : 31), t0 = job.t0 - (fwd ? 0 : 31);
+  const int  bufW = job.bufW, arenaCap = job.arenaCap;
+  int e = job.e, L = job.L, R = job.R, off = job.off, base = job.base;
+  int lim = e <= errorLimit ? job.eml[e] : 0;
+  u32 cells = 0, slides = 0;
+  int status = kRowsDone;
+  for (; e <= errorLimit; e++) {
+    if (off + R - L + 1 > arenaCap) { status = kRowsErr; break; }
     const int Lc = max(L - 1, -e), Rc = min(R + 1, e);
     const int width = Rc - Lc + 1;
-    if (width + 4 > bufW) {
-      // The band outgrew the shared-memory rows: continue in the warp's HBM rows.
-      if (bufW == rowsGW || width + 4 > rowsGW || !rowsG) { o.status = kRowsErr; o.err = kErrBandWide; break; }
-      int *gA = rowsG, *gB = rowsG + rowsGW;
-      for (int i = lane; i < bufW; i += 32) gA[i] = prev[i];
-      __syncwarp();
-      prev = gA;
-      cur  = gB;
-      bufW = rowsGW;
-    }
-
-    const int lim = eml[e];
-    if (lane < 4) prev[(lane < 2 ? L - 2 + lane : R - 1 + lane) - prevBase + 2] = -2;
-    __syncwarp();
-    const int *pv = prev + (2 - prevBase);   // pv[d] = row e-1 at diagonal d
-    int       *cv = cur + (2 - Lc);          // cv[d] = row e at diagonal d
-    int myEnd = INT_MAX, myL = INT_MAX, myR = INT_MIN;
-    for (int d = Lc + lane; d <= Rc; d += 32) {
-      const int p0 = pv[d], pm = pv[d - 1], pp = pv[d + 1];
-      int row = 1 + p0;
-      if (pm > row) row = pm;
-      if (1 + pp > row) row = 1 + pp;
-      const int room = min(m - row, n - row - d);
-      if (room > 0) row += slide<STEP, FIRST16>(A, a0, T, t0, row, d, room, slides);
-      cv[d] = row;
-      if ((row == m || row + d == n) && d < myEnd) myEnd = d;
+    if (width + 4 > bufW) { status = kRowsWiden; break; }
+    const int limNext = e < errorLimit ? job.eml[e + 1] : 0;
+    const int *pv = prev + (2 - base);        // pv[d] = row e-1 at diagonal d
+    int       *cv = cur + (2 - Lc);           // cv[d] = row e at diagonal d
+    int       *av = arena + (off - L);        // av[d]: row e-1's place in the arena
+    int L2 = INT_MAX, R2 = INT_MIN, prevMax = -1, dEnd = INT_MAX;
+#pragma unroll 1
+    for (int c = Lc; c <= Rc; c += 64) {
+      const bool two = c + 32 <= Rc;
+      const int  da = min(c + lane, Rc), db = min(c + 32 + lane, Rc);
+      const bool ina = c + lane <= Rc, inb = c + 32 + lane <= Rc;
+      int pa = pv[da + 1], pb = 0, ra, rb = 0, ka, kb = 0;   // row e-1 at d + 1; value; room to the nearer end
+      {
+        const int p0 = pv[da];
+        ra = max(max(p0, pa) + 1, pv[da - 1]);
+        if (ina && da >= L && da <= R) {      // keep row e-1 for the traceback
+          av[da]  = p0;
+          prevMax = max(prevMax, p0);
+        }
+        ka = min(m - ra, n - da - ra);        // >= 0: no cell of row e-1 is at an end
+      }
+      if (two) {
+        const int p0 = pv[db];
+        pb = pv[db + 1];
+        rb = max(max(p0, pb) + 1, pv[db - 1]);
+        if (inb && db <= R) {                 // db > Lc + 31 >= L
+          av[db]  = p0;
+          prevMax = max(prevMax, p0);
+        }
+        kb = min(m - rb, n - db - rb);
+      }
+      int sa = match_len<HASN>(job, Ap, a0 + sgn * ra, Tp, t0 + sgn * (ra + da), fwd), sb = 0;
+      if (two) sb = match_len<HASN>(job, Ap, a0 + sgn * rb, Tp, t0 + sgn * (rb + db), fwd);
+      unsigned moreA = __ballot_sync(0xffffffffu, ina && sa == 32 && ka > 32);
+      unsigned moreB = __ballot_sync(0xffffffffu, inb && sb == 32 && kb > 32);
+      while (moreA | moreB) {
+        // One lane's slide goes on: the warp looks at 32 windows of 32 bases per step.
+        const bool second = moreA == 0;
+        const unsigned w = second ? moreB : moreA;
+        const int  q  = __ffs((int)w) - 1;
+        const int  r0 = __shfl_sync(0xffffffffu, second ? rb : ra, q);
+        const int  rq = __shfl_sync(0xffffffffu, second ? kb : ka, q);
+        const int  dq = c + q + (second ? 32 : 0);
+        if (second) moreB = w & (w - 1);
+        else moreA = w & (w - 1);
+        for (int run = 32;; run += 1024) {
+          const int at = run + 32 * lane;
+          int len = 0;
+          if (at < rq) len = match_len<HASN>(job, Ap, a0 + sgn * (r0 + at), Tp, t0 + sgn * (r0 + at + dq), fwd);
+          const unsigned stop = __ballot_sync(0xffffffffu, len < 32);
+          if (stop) {
+            const int f   = __ffs((int)stop) - 1;
+            const int all = run + 32 * f + __shfl_sync(0xffffffffu, len, f);
+            if (lane == q) {
+              if (second) sb = all;
+              else sa = all;
+            }
+            break;
+          }
+        }
+      }
+      sa = min(sa, ka);
+      ra += sa;
+      unsigned keepB = 0, endB = 0;
       // pruneAlign (prefixEditDistance.H:249-258): extra = max(d, 0) on both band edges
-      if (!(row + max(d, 0) < lim)) {
-        if (myL == INT_MAX) myL = d;
-        myR = d;
+      const unsigned keepA = __ballot_sync(0xffffffffu, ina && ra + max(da, 0) >= lim);
+      const unsigned endA  = __ballot_sync(0xffffffffu, ina && sa == ka);   // at the end of A or T
+      if (ina) {
+        cv[da] = ra;
+        slides += (u32)sa;
+      }
+      if (two) {
+        sb = min(sb, kb);
+        rb += sb;
+        keepB = __ballot_sync(0xffffffffu, inb && rb + max(db, 0) >= lim);
+        endB  = __ballot_sync(0xffffffffu, inb && sb == kb);
+        if (inb) {
+          cv[db] = rb;
+          slides += (u32)sb;
+        }
+      }
+      if ((endA | endB) && dEnd == INT_MAX) {
+        const int f = __ffs((int)(endA ? endA : endB)) - 1;
+        dEnd = c + f + (endA ? 0 : 32);
+        if (lane == f) {
+          job.rowEnd = endA ? ra : rb;
+          job.ppEnd  = endA ? pa : pb;
+        }
+      }
+      const u64 keep = (u64)keepA | ((u64)keepB << 32);
+      if (keep) {
+        if (L2 == INT_MAX) L2 = c + __ffsll((long long)keep) - 1;
+        R2 = c + 63 - __clzll((long long)keep);
       }
     }
-    __syncwarp();
-    o.rows++;
-    const int dEnd = __reduce_min_sync(0xffffffffu, myEnd);
+    // Row e-1's header, with its largest value (forward.C:284-289) for max_score_rows.
+    prevMax = __reduce_max_sync(0xffffffffu, prevMax);
+    if (lane == 0) job.rowHdr[e - 1] = make_int4(off, L, R, prevMax);
     if (dEnd != INT_MAX) {
-      o.cells += (unsigned long long)(dEnd - Lc + 1);
-      o.status   = kRowsEnd;
-      o.e        = e;
-      o.dEnd     = dEnd;
-      o.Lc       = Lc;
-      o.Rc       = Rc;
-      o.prevBase = prevBase;
-      o.prev     = prev;
-      o.cur      = cur;
+      cells += (u32)(dEnd - Lc + 1);
+      status = kRowsEnd;
+      if (lane == 0) {
+        job.dEnd = dEnd;
+        job.Rc   = Rc;
+      }
       break;
     }
-    o.cells += (unsigned long long)width;
-
+    cells += (u32)width;
     // The kept band is [first, last] unpruned diagonal (forward.C:245-280).
-    const int L2 = __reduce_min_sync(0xffffffffu, myL);
     if (L2 == INT_MAX) break;
-    const int R2 = __reduce_max_sync(0xffffffffu, myR);
-
-    // Keep the band for the traceback, and take its largest value on the way
-    // (forward.C:284-289); the Max_Score test that uses it runs once after the rows
-    // (max_score_rows).
-    const int cnt = R2 - L2 + 1;
-    if (used + cnt > arenaCap) { o.status = kRowsErr; o.err = kErrArenaFull; break; }
-    int myV = -1;
-    for (int d = L2 + lane; d <= R2; d += 32) {
-      const int v = cv[d];
-      myV         = max(myV, v);
-      arena[used + d - L2] = v;
-    }
-    const int rowMax = __reduce_max_sync(0xffffffffu, myV);
-    if (lane == 0) rowHdr[e] = make_int4(used, L2, R2, rowMax);
-    used += cnt;
+    __syncwarp();
+    if (lane < 4) cv[lane < 2 ? L2 - 2 + lane : R2 - 1 + lane] = -2;
+    off += R - L + 1;
     int *t = prev;
     prev   = cur;
     cur    = t;
-    prevBase = Lc;
-    L        = L2;
-    R        = R2;
-    o.eDone  = e;
+    base   = Lc;
+    L      = L2;
+    R      = R2;
+    lim    = limNext;
     __syncwarp();
   }
-  w.slides += slides;
-  return o;
+  if (e > errorLimit) {
+    // The error limit: the last row has not been kept yet.
+    if (off + R - L + 1 > arenaCap) status = kRowsErr;
+    else {
+      const int *pv = prev + (2 - base);
+      int prevMax = -1;
+      for (int d = L + lane; d <= R; d += 32) {
+        const int v = pv[d];
+        arena[off + d - L] = v;
+        prevMax            = max(prevMax, v);
+      }
+      prevMax = __reduce_max_sync(0xffffffffu, prevMax);
+      if (lane == 0) job.rowHdr[errorLimit] = make_int4(off, L, R, prevMax);
+    }
+  }
+  __syncwarp();
+  if (lane == 0) {
+    job.e    = e;
+    job.L    = L;
+    job.R    = R;
+    job.off  = off;
+    job.base = base;
+    job.cells += cells;
+  }
+  job.slides[lane] += slides;
+  __syncwarp();
+  return status;
+}
+
+// The row loop by one warp: rows in shared memory, and in the warp's HBM rows from the row
+// on whose band has outgrown them.  r0: row 0's value.
+static __device__ __noinline__ void warp_rows(WarpDP &w, RowsOut &o, int step, const SeqView &A, int a0, int m,
+                                              const SeqView &T, int t0, int n, int errorLimit, int r0) {
+  const int  lane = threadIdx.x & 31;
+  int *const bufA = smemRows + w.smOff, *const bufB = bufA + kRowStride;
+  RowJob    &job  = *(RowJob *)(bufB + kRowStride);
+  const int  rowCap = w.cap.rowCap, gw = w.cap.rowsGW;
+  int *const rowsG  = w.sc.rowsG;
+  const bool hasN   = A.nm || T.nm;
+  if (lane < 5) bufA[lane] = lane == 2 ? r0 : -2;
+  if (lane == 0) {
+    job.A        = A;
+    job.T        = T;
+    job.arena    = w.sc.arena;
+    job.rowHdr   = w.sc.rowHdr;
+    job.eml      = w.eml;
+    job.a0       = a0;
+    job.t0       = t0;
+    job.step     = step;
+    job.arenaCap = w.cap.arenaCap;
+    job.bufW     = kRowW;
+    job.e        = 1;
+    job.L = job.R = job.off = job.base = 0;
+    job.cells    = 0;
+  }
+  job.slides[lane] = 0;
+  __syncwarp();
+  // Row rowCap has no header: the loop stops before it.
+  const bool capped = errorLimit >= rowCap;
+  const int  limit  = capped ? rowCap - 1 : errorLimit;
+  u32 err = kErrArenaFull;
+  int st  = hasN ? row_loop<true, false>(job, w.smOff, rowsG, m, n, limit)
+                 : row_loop<false, false>(job, w.smOff, rowsG, m, n, limit);
+  if (st == kRowsWiden) {
+    if (job.R - job.L + 7 > gw || !rowsG) {
+      st  = kRowsErr;
+      err = kErrBandWide;
+    } else {
+      const int *src = (job.e & 1) ? bufA : bufB;   // even rows are in bufA
+      for (int i = lane; i < kRowW; i += 32) rowsG[i] = src[i];
+      if (lane == 0) job.bufW = gw;
+      __syncwarp();
+      st = hasN ? row_loop<true, true>(job, w.smOff, rowsG, m, n, limit)
+                : row_loop<false, true>(job, w.smOff, rowsG, m, n, limit);
+      if (st == kRowsWiden) {
+        st  = kRowsErr;
+        err = kErrBandWide;
+      }
+    }
+  }
+  const int e = job.e;
+  if (capped && e > limit && st == kRowsDone) {
+    st  = kRowsErr;
+    err = kErrRowsFull;
+  }
+  o.status = st;
+  o.err    = st == kRowsErr ? err : 0;
+  o.e      = e;
+  o.eDone  = e - 1;      // rows below e are kept
+  o.dEnd   = job.dEnd;
+  o.Rc     = job.Rc;
+  o.rowEnd = job.rowEnd;
+  o.ppEnd  = job.ppEnd;
+  o.cells  = job.cells;
+  o.rows   = (unsigned)(e <= limit && st != kRowsErr ? e : e - 1);   // row e itself was computed when the loop ended in it
+  w.slides += job.slides[lane];
+  __syncwarp();
 }
 
 // The row loop by every thread of the CTA (nThr threads, tid = threadIdx.x).  Thread t
@@ -374,7 +584,7 @@ __device__ __forceinline__ RowsOut warp_rows(WarpDP &w, const SeqView &Aref, int
 // neighbour values of row e-1 are read once for U cells and U slides are in flight.
 // Every decision is made on CTA-reduced values, so all threads take the same path and
 // meet the same barriers.
-template <int STEP, int U, bool FIRST16>
+template <int STEP, int U>
 static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpScratch &sc, const AlignCaps &cap,
                                                   const int *eml, int tid, int nThr, int (*red)[4],
                                                   unsigned long long &slides) {
@@ -385,7 +595,7 @@ static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpS
   RowsOut o;
   o.status = kRowsDone;
   o.err = 0;
-  o.e = o.dEnd = o.eDone = 0;
+  o.e = o.dEnd = o.eDone = o.Rc = o.rowEnd = o.ppEnd = 0;
   o.cells = o.rows = 0;
   // Every thread has read the job before warp 0 can post the next one.
   group_bar(2, nThr);
@@ -423,7 +633,7 @@ static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpS
           if (q[k] > row) row = q[k];
           if (1 + q[k + 2] > row) row = 1 + q[k + 2];
           const int room = min(m - row, n - row - d);
-          if (room > 0) row += slide<STEP, FIRST16>(A, a0, T, t0, row, d, room, slides);
+          if (room > 0) row += slide<STEP>(A, a0, T, t0, row, d, room, slides);
           cv[d] = row;
           if ((row == m || row + d == n) && d < myEnd) myEnd = d;
           if (!(row + max(d, 0) < lim)) {
@@ -456,11 +666,9 @@ static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpS
       o.status   = kRowsEnd;
       o.e        = e;
       o.dEnd     = dEnd;
-      o.Lc       = Lc;
       o.Rc       = Rc;
-      o.prevBase = prevBase;
-      o.prev     = prev;
-      o.cur      = cur;
+      o.rowEnd   = cv[dEnd];
+      o.ppEnd    = pv[dEnd + 1];
       break;
     }
     o.cells += (unsigned long long)width;
@@ -500,18 +708,14 @@ static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpS
 static __device__ __forceinline__ RowsOut group_rows_any(const GroupJob &j, const WarpScratch &sc,
                                                          const AlignCaps &cap, const int *eml, int tid, int nThr,
                                                          int (*red)[4], unsigned long long &slides) {
-#define OIC_GROUP_ROWS(S, U)                                                                  \
-  return j.first16 ? group_rows<S, U, true>(j, sc, cap, eml, tid, nThr, red, slides)          \
-                   : group_rows<S, U, false>(j, sc, cap, eml, tid, nThr, red, slides)
   if (j.step > 0) {
-    if (j.u == 4) OIC_GROUP_ROWS(+1, 4);
-    if (j.u == 2) OIC_GROUP_ROWS(+1, 2);
-    OIC_GROUP_ROWS(+1, 1);
+    if (j.u == 4) return group_rows<+1, 4>(j, sc, cap, eml, tid, nThr, red, slides);
+    if (j.u == 2) return group_rows<+1, 2>(j, sc, cap, eml, tid, nThr, red, slides);
+    return group_rows<+1, 1>(j, sc, cap, eml, tid, nThr, red, slides);
   }
-  if (j.u == 4) OIC_GROUP_ROWS(-1, 4);
-  if (j.u == 2) OIC_GROUP_ROWS(-1, 2);
-  OIC_GROUP_ROWS(-1, 1);
-#undef OIC_GROUP_ROWS
+  if (j.u == 4) return group_rows<-1, 4>(j, sc, cap, eml, tid, nThr, red, slides);
+  if (j.u == 2) return group_rows<-1, 2>(j, sc, cap, eml, tid, nThr, red, slides);
+  return group_rows<-1, 1>(j, sc, cap, eml, tid, nThr, red, slides);
 }
 
 // Worker warps of a group CTA: run the row loops warp 0 posts until it posts exit.
@@ -531,9 +735,11 @@ static __device__ __noinline__ void group_worker(GroupShared &gs, const WarpScra
 // view A, T likewise.  The row loop runs on this warp, or on the whole CTA when w.gs is
 // set (warp 0 of a group CTA); the rest runs on this warp.  Returns the error count;
 // the outputs are warp-uniform.  On a capacity overflow sets w.err and returns 0.
-template <int STEP, bool GROUP, bool FIRST16 = false>
+// endOnly: the caller uses the outputs only when the end is reached (toEnd); otherwise
+// they are not computed.
+template <int STEP, bool GROUP>
 static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, int a0, int m, const SeqView &T, int t0, int n,
-                              int errorLimit, int &aEnd, int &tEnd, int &leftover, bool &toEnd) {
+                              int errorLimit, bool endOnly, int &aEnd, int &tEnd, int &leftover, bool &toEnd) {
   const int lane = threadIdx.x & 31;
   const double BMV = w.P.branchMatchValue;
 
@@ -548,16 +754,12 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
     return 0;
   }
 
-  if (lane == 0) {
-    w.sc.arena[0]  = r0;
-    w.sc.rowHdr[0] = make_int4(0, 0, 0, 0);
-    w.smA[2]       = r0;
-  }
-  __syncwarp();
-
   RowsOut o;
   if (GROUP) {
     if (lane == 0) {
+      w.sc.arena[0]  = r0;
+      w.sc.rowHdr[0] = make_int4(0, 0, 0, 0);
+      w.smA[2]       = r0;
       GroupJob &j  = w.gs->job;
       j.A          = A;
       j.T          = T;
@@ -568,7 +770,6 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
       j.errorLimit = errorLimit;
       j.step       = STEP;
       j.u          = w.gU;
-      j.first16    = slide_first16(w.P.maxErate);
       j.rowA       = w.smA;
       j.rowB       = w.smB;
       w.gs->cmd    = kGroupRows;
@@ -578,12 +779,16 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
     const GroupJob j = w.gs->job;
     o = group_rows_any(j, w.sc, w.cap, w.eml, lane, w.gThreads, w.gs->red, w.slides);
   } else {
-    o = warp_rows<STEP, FIRST16>(w, A, a0, m, T, t0, n, errorLimit);
+    warp_rows(w, o, STEP, A, a0, m, T, t0, n, errorLimit, r0);
   }
   w.cells += o.cells;
   w.rows += o.rows;
   if (o.status == kRowsErr) {
     w.err |= o.err;
+    return 0;
+  }
+  if (endOnly && o.status != kRowsEnd) {
+    toEnd = false;
     return 0;
   }
 
@@ -592,10 +797,8 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
   max_score_rows(w, o.eDone, maxScore, msLen, msD, msE);
 
   if (o.status == kRowsEnd) {
-    const int  e   = o.e;
-    const int *pv  = o.prev + (2 - o.prevBase);
-    const int *cv  = o.cur + (2 - o.Lc);
-    const int  row = cv[o.dEnd];
+    const int e   = o.e;
+    const int row = o.rowEnd;
     // Branch-point test in IEEE double on lane 0 (the FP64 pipe is narrow); the other
     // lanes take its decision.
     int abort_ = 0;
@@ -611,22 +814,21 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
       int d = o.dEnd;
       if (STEP > 0) {
         // Force the last error to be a mismatch (forward.C:215-221).
-        if (row == m && 1 + pv[d + 1] == row && d < o.Rc) d++;
+        if (row == m && 1 + o.ppEnd == row && d < o.Rc) d++;
         aEnd = row;
         tEnd = row + d;
-        if (lane == 0) set_right_delta(w, e, d, row);
-        w.rightLen = __shfl_sync(0xffffffffu, w.rightLen, 0);
+        set_right_delta(w, e, d, row);
       } else {
         aEnd = -row;
         tEnd = -row - d;
-        if (lane == 0) set_left_delta(w, e, d, row, leftover, tEnd, n);
-        w.leftLen = __shfl_sync(0xffffffffu, w.leftLen, 0);
-        leftover  = __shfl_sync(0xffffffffu, leftover, 0);
-        tEnd      = __shfl_sync(0xffffffffu, tEnd, 0);
+        set_left_delta(w, e, d, row, leftover, tEnd, n);
       }
       toEnd = true;
-      __syncwarp();
       return e;
+    }
+    if (endOnly) {
+      toEnd = false;
+      return 0;
     }
   }
 
@@ -634,29 +836,20 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
   // 306-313): the alignment ends at the Max_Score row.
   aEnd = STEP * msLen;
   tEnd = STEP * (msLen + msD);
-  __syncwarp();
-  if (lane == 0) {
-    const int last = arena_get(w, msE, msD);
-    if (STEP > 0) set_right_delta(w, msE, msD, last);
-    else set_left_delta(w, msE, msD, last, leftover, tEnd, n);
-  }
-  if (STEP > 0) w.rightLen = __shfl_sync(0xffffffffu, w.rightLen, 0);
-  else {
-    w.leftLen = __shfl_sync(0xffffffffu, w.leftLen, 0);
-    leftover  = __shfl_sync(0xffffffffu, leftover, 0);
-    tEnd      = __shfl_sync(0xffffffffu, tEnd, 0);
-  }
+  const int last = arena_get(w, msE, msD);
+  if (STEP > 0) set_right_delta(w, msE, msD, last);
+  else set_left_delta(w, msE, msD, last, leftover, tEnd, n);
   toEnd = false;
-  __syncwarp();
   return msE;
 }
 
-static __device__ __forceinline__ void warp_dp_init(WarpDP &w, const WarpScratch &sc, const AlignCaps &cap, int *smA,
-                                                    int *smB, const int *eml, const DevParams &P) {
+static __device__ __forceinline__ void warp_dp_init(WarpDP &w, const WarpScratch &sc, const AlignCaps &cap, int smOff,
+                                                    const int *eml, const DevParams &P) {
   w.sc       = sc;
   w.cap      = cap;
-  w.smA      = smA;
-  w.smB      = smB;
+  w.smOff    = smOff;
+  w.smA      = smemRows + smOff;             // a group CTA's two rows of cap.bandW
+  w.smB      = w.smA + cap.bandW;
   w.eml      = eml;
   w.P        = P;
   w.cells    = 0;
@@ -673,8 +866,12 @@ enum { kNone = 0, kLeftBranch = 1, kRightBranch = 2, kDovetail = 3 };
 
 // Extend_Alignment (prefixEditDistance-extend.C:36-183), one warp.  The merged delta
 // ends up in sc.deltaL[0 .. leftLen).  Outputs are warp-uniform.
-template <bool GROUP, bool FIRST16 = false>
-static __device__ __noinline__ int warp_extend(WarpDP &w, const SeqView &S, int sLen, const SeqView &T, int tLen, int mStart,
+// dovetailOnly: the caller uses the outputs only when both ends are reached.  The left
+// side is then not extended after the right side has failed, and a side that fails is not
+// traced: pairs that share only a repeat fail on one side in nearly every extension, and
+// on repeat-rich low-error reads they are nine tenths of the cells.
+template <bool GROUP>
+static __device__ __noinline__ int warp_extend(WarpDP &w, bool dovetailOnly, const SeqView &S, int sLen, const SeqView &T, int tLen, int mStart,
                            int mOffset, int mLen, int &sLo, int &sHi, int &tLo, int &tHi, int &errors) {
   const int lane = threadIdx.x & 31;
   int  rightErrors = 0, leftErrors = 0, leftover = 0;
@@ -692,15 +889,16 @@ static __device__ __noinline__ int warp_extend(WarpDP &w, const SeqView &S, int 
     sHi = tHi = 0;
     rToEnd    = true;
   } else if (sRightLen <= tRightLen) {
-    rightErrors = warp_prefix_dp<+1, GROUP, FIRST16>(w, S, sRightBegin, sRightLen, T, tRightBegin, tRightLen, errorLimit, sHi, tHi,
-                                     leftover, rToEnd);
+    rightErrors = warp_prefix_dp<+1, GROUP>(w, S, sRightBegin, sRightLen, T, tRightBegin, tRightLen, errorLimit,
+                                     dovetailOnly, sHi, tHi, leftover, rToEnd);
     if (w.err) return kNone;
     for (int i = lane; i < w.rightLen; i += 32) w.sc.deltaR[i] = -w.sc.deltaR[i];
   } else {
-    rightErrors = warp_prefix_dp<+1, GROUP, FIRST16>(w, T, tRightBegin, tRightLen, S, sRightBegin, sRightLen, errorLimit, tHi, sHi,
-                                     leftover, rToEnd);
+    rightErrors = warp_prefix_dp<+1, GROUP>(w, T, tRightBegin, tRightLen, S, sRightBegin, sRightLen, errorLimit,
+                                     dovetailOnly, tHi, sHi, leftover, rToEnd);
     if (w.err) return kNone;
   }
+  if (dovetailOnly && !rToEnd) return kNone;
   __syncwarp();
   sHi += sRightBegin - 1;
   tHi += tRightBegin - 1;
@@ -710,15 +908,16 @@ static __device__ __noinline__ int warp_extend(WarpDP &w, const SeqView &S, int 
     sLo = tLo = 0;
     lToEnd    = true;
   } else if (sRightBegin <= tRightBegin) {
-    leftErrors = warp_prefix_dp<-1, GROUP, FIRST16>(w, S, sLeftBegin, sLeftBegin + 1, T, tLeftBegin, tLeftBegin + 1,
-                                    errorLimit - rightErrors, sLo, tLo, leftover, lToEnd);
+    leftErrors = warp_prefix_dp<-1, GROUP>(w, S, sLeftBegin, sLeftBegin + 1, T, tLeftBegin, tLeftBegin + 1,
+                                    errorLimit - rightErrors, dovetailOnly, sLo, tLo, leftover, lToEnd);
     if (w.err) return kNone;
   } else {
-    leftErrors = warp_prefix_dp<-1, GROUP, FIRST16>(w, T, tLeftBegin, tLeftBegin + 1, S, sLeftBegin, sLeftBegin + 1,
-                                    errorLimit - rightErrors, tLo, sLo, leftover, lToEnd);
+    leftErrors = warp_prefix_dp<-1, GROUP>(w, T, tLeftBegin, tLeftBegin + 1, S, sLeftBegin, sLeftBegin + 1,
+                                    errorLimit - rightErrors, dovetailOnly, tLo, sLo, leftover, lToEnd);
     if (w.err) return kNone;
     for (int i = lane; i < w.leftLen; i += 32) w.sc.deltaL[i] = -w.sc.deltaL[i];
   }
+  if (dovetailOnly && !lToEnd) return kNone;
   __syncwarp();
   sLo += sLeftBegin + 1;
   tLo += tLeftBegin + 1;

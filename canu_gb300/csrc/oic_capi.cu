@@ -125,7 +125,7 @@ struct oic_ctx {
   uint32_t              nReads = 0;
   std::vector<uint32_t> len, lib;
   std::vector<uint64_t> wordOff;
-  DevBuf dFwd, dRc, dNfwd, dNrc, dWordOff, dLen, dLib, dHasN;
+  DevBuf dFwd, dRc, dNfwd, dNrc, dPfwd, dPrc, dWordOff, dLen, dLib, dHasN;
   ReadsDev R{};
 
   // skip list
@@ -281,7 +281,7 @@ struct AlignConfig {
 AlignConfig align_normal(const oic_ctx *c) {
   AlignConfig a;
   a.bandW         = 512;
-  a.warps         = c->nSM * OIC_ALIGN_MIN_BLOCKS * align_warps_per_block(512);
+  a.warps         = c->nSM * OIC_ALIGN_MIN_BLOCKS * align_warps_per_block();
   a.caps.arenaCap = 1 << 20;
   a.caps.rowCap   = 1 << 14;
   a.caps.nodeCap  = 1 << 16;
@@ -674,7 +674,7 @@ int align_stage(oic_ctx *ctx, uint32_t nPairs, uint32_t nNodes, const oic_tuning
     an.caps.arenaCap = (int)tn.narrowArena;
     WarpScratch ws;
     if ((rc = ensure_align_scratch(ctx, an, false, ws))) return rc;
-    launch_align(an.bandW, ctx->R, ctx->T, ctx->dp, ctx->dEml.as<int>(), ctx->dPairs.as<PairRec>(),
+    launch_align(ctx->R, ctx->T, ctx->dp, ctx->dEml.as<int>(), ctx->dPairs.as<PairRec>(),
                  ctx->dWork.as<uint32_t>(), nNarrow, ctr32(ctx) + cWorkCounter, ctx->dNodes.as<int4>(), ws, an.caps,
                  an.warps, ao, ctx->st);
     CK(cudaMemcpyAsync(h, ctx->dCtr.p, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->st));
@@ -896,7 +896,7 @@ int align_stage_graph(oic_ctx *ctx, uint32_t nPairs, uint32_t nNodes, const oic_
       cudaMemsetAsync(ctx->dPairExt.p, 0, (size_t)cap * sizeof(int4), s);
     }
     cudaEventRecordWithFlags(ctx->gEv[0], s, cudaEventRecordExternal);   // recorded at every replay
-    launch_align(an.bandW, ctx->R, ctx->T, ctx->dp, ctx->dEml.as<int>(), ctx->dPairs.as<PairRec>(),
+    launch_align(ctx->R, ctx->T, ctx->dp, ctx->dEml.as<int>(), ctx->dPairs.as<PairRec>(),
                  ctx->dWork.as<uint32_t>(), 0, ctr32(ctx) + cWorkCounter, ctx->dNodes.as<int4>(), wsN, an.caps,
                  an.warps, aoN, s);
     cudaMemcpyAsync(ctr64(ctx) + kCellsSnap, ctr64(ctx) + kAlignStatBase + kStCells, sizeof(unsigned long long),
@@ -1231,7 +1231,7 @@ void oic_destroy(oic_ctx *ctx) {
                     &ctx->dStack2,   &ctx->dAlive2,     &ctx->dScanScratch, &ctx->dCtr,
                     &ctx->dWorkK,    &ctx->dWorkK2,     &ctx->dWorkV2,     &ctx->dWorkScratch, &ctx->dSegList,
                     &ctx->dRowsG,    &ctx->dRowsG2,     &ctx->dFilterPrm,  &ctx->dFeat,      &ctx->dLogit,
-                    &ctx->dPairCells, &ctx->dPairExt};
+                    &ctx->dPairCells, &ctx->dPairExt,    &ctx->dPfwd,       &ctx->dPrc};
   for (DevBuf *b : bufs) b->release();
   if (ctx->gExec) cudaGraphExecDestroy(ctx->gExec);
   for (cudaEvent_t e : ctx->gEv)
@@ -1279,10 +1279,14 @@ int oic_set_reads(oic_ctx *ctx, uint32_t nReads, const uint32_t *libID, const ui
   CK(ctx->dRc.ensure(nWords * 8));
   CK(ctx->dNfwd.ensure(nWords * 8));
   CK(ctx->dNrc.ensure(nWords * 8));
+  CK(ctx->dPfwd.ensure(nWords * 8));
+  CK(ctx->dPrc.ensure(nWords * 8));
   CK(cudaMemsetAsync(ctx->dFwd.p, 0, nWords * 8, ctx->st));
   CK(cudaMemsetAsync(ctx->dRc.p, 0, nWords * 8, ctx->st));
   CK(cudaMemsetAsync(ctx->dNfwd.p, 0, nWords * 8, ctx->st));
   CK(cudaMemsetAsync(ctx->dNrc.p, 0, nWords * 8, ctx->st));
+  CK(cudaMemsetAsync(ctx->dPfwd.p, 0, nWords * 8, ctx->st));
+  CK(cudaMemsetAsync(ctx->dPrc.p, 0, nWords * 8, ctx->st));
   CK(ctx->dWordOff.ensure((size_t)(nReads + 1) * 8));
   CK(ctx->dLen.ensure((size_t)(nReads + 1) * 4));
   CK(ctx->dLib.ensure((size_t)(nReads + 1) * 4));
@@ -1299,7 +1303,7 @@ int oic_set_reads(oic_ctx *ctx, uint32_t nReads, const uint32_t *libID, const ui
     CK(cudaMemsetAsync(ctr32(ctx) + cErr, 0, 4, ctx->st));
     launch_pack_reads(ascii.as<char>(), off.as<u64>(), ctx->dLen.as<uint32_t>(), ctx->dWordOff.as<u64>(),
                       nReads, ctx->dFwd.as<u64>(), ctx->dRc.as<u64>(), ctx->dNfwd.as<u64>(), ctx->dNrc.as<u64>(),
-                      ctx->dHasN.as<unsigned char>(), ctr32(ctx) + cErr, ctx->st);
+                      ctx->dPfwd.as<uint2>(), ctx->dPrc.as<uint2>(), ctx->dHasN.as<unsigned char>(), ctr32(ctx) + cErr, ctx->st);
     int rc = sync_check(ctx, "pack reads");
     uint32_t err = read_err(ctx);
     ascii.release();
@@ -1317,6 +1321,8 @@ int oic_set_reads(oic_ctx *ctx, uint32_t nReads, const uint32_t *libID, const ui
   R.rc      = ctx->dRc.as<u64>();
   R.nfwd    = ctx->dNfwd.as<u64>();
   R.nrc     = ctx->dNrc.as<u64>();
+  R.pfwd    = ctx->dPfwd.as<uint2>();
+  R.prc     = ctx->dPrc.as<uint2>();
   R.wordOff = ctx->dWordOff.as<u64>();
   R.len     = ctx->dLen.as<uint32_t>();
   R.lib     = ctx->dLib.as<uint32_t>();
@@ -1783,7 +1789,7 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
       ac.caps.arenaCap = (int)tn.narrowArena;
       WarpScratch ws;
       if ((rc = ensure_align_scratch(ctx, ac, false, ws))) break;
-      launch_extend_batch(ac.bandW, ctx->R, ctx->dp, ctx->dEml.as<int>(), dP.as<ExtendProblem>(), nAlign, ws,
+      launch_extend_batch(ctx->R, ctx->dp, ctx->dEml.as<int>(), dP.as<ExtendProblem>(), nAlign, ws,
                           ac.caps, ac.warps, dOut.as<int>(), dKind.as<int>(), dDl.as<int>(), dStatus.as<uint32_t>(),
                           ctr64(ctx) + kExtStatBase, ctx->st);
     } else {

@@ -3,9 +3,11 @@
 // Read layout in HBM: every read is packed 2 bits per base (A=0 C=1 G=2 T=3, base i
 // of a read at bits 2*(i%32) of 64-bit word i/32, the same order overlapInCore builds
 // its k-mer keys in, Build_Hash_Index.C:347-350) in two strand arrays -- forward and
-// reverse complement -- plus a parallel mask array with 0b11 at every N.  Reads start
-// on a word boundary and are separated by one zero guard word, so a 32-base window
-// that runs off either end of a read stays inside the arrays.
+// reverse complement -- plus a parallel mask array with 0b11 at every N.  The DP reads the
+// same bases as bit planes (word i: the low bits of bases 32i .. 32i+31, then their high
+// bits), in which a comparison of 32 bases is four funnel shifts and two logic
+// instructions.  Reads start on a word boundary and are separated by one zero guard word,
+// so a 32-base window that runs off either end of a read stays inside the arrays.
 #pragma once
 
 #include <cstdint>
@@ -25,7 +27,6 @@ constexpr int kMinIntersect   = 10;                              // overlapInCor
 constexpr int kShiftSlack     = 1;                               // overlapInCore.H:146
 constexpr int kEntriesPerBucket = 21;                            // overlapInCore.H:58
 constexpr u64 kEmptyKey       = ~0ull;
-constexpr u64 kPairMask       = 0x5555555555555555ull;
 
 // Device error flags (bitwise OR into ctx->dErr).  Kernels never trap: they record
 // the condition, skip the access and return.
@@ -50,6 +51,8 @@ struct ReadsDev {
   const u64 *rc;        // reverse-complement strand words
   const u64 *nfwd;      // N masks (0b11 per N) for the forward strand
   const u64 *nrc;
+  const uint2 *pfwd;    // bit planes of the forward strand (x low bits, y high bits)
+  const uint2 *prc;
   const u64 *wordOff;   // first word of read i (0-based index = ID-1)
   const u32 *len;
   const u32 *lib;
@@ -59,14 +62,14 @@ struct ReadsDev {
 
 // One read strand viewed as a base sequence: base i is base i of the read's first word.
 struct SeqView {
-  const u64 *w;    // the read's first word in its strand array
+  const uint2 *p;  // the read's first bit-plane word in its strand array
   const u64 *nm;   // its first N-mask word; nullptr when the read has no N
 };
 
 __device__ __forceinline__ SeqView make_view(const ReadsDev &R, u32 readIdx, int rev) {
   SeqView v;
   const u64 wo = R.wordOff[readIdx];
-  v.w  = (rev ? R.rc : R.fwd) + wo;
+  v.p  = (rev ? R.prc : R.pfwd) + wo;
   v.nm = R.hasN[readIdx] ? (rev ? R.nrc : R.nfwd) + wo : nullptr;
   return v;
 }
@@ -92,89 +95,55 @@ __device__ __forceinline__ u64 load_win32(const u64 *w, int g) {
   return (lo >> sh) | ((hi << 1) << (63 - sh));
 }
 
-// 32 bases g, g-1, ..., g-31 of one read (base g in bits 0-1; the two bits of each
-// base come out swapped, which equality tests do not see).
-__device__ __forceinline__ u64 load_win_rev(const u64 *w, int g) { return __brevll(load_win32(w, g - 31)); }
+// Bits 2j of x packed into bit j.
+__host__ __device__ __forceinline__ u32 even_bits(u64 x) {
+  u32 lo = (u32)x & 0x55555555u, hi = (u32)(x >> 32) & 0x55555555u;
+  lo = (lo | (lo >> 1)) & 0x33333333u;
+  hi = (hi | (hi >> 1)) & 0x33333333u;
+  lo = (lo | (lo >> 2)) & 0x0f0f0f0fu;
+  hi = (hi | (hi >> 2)) & 0x0f0f0f0fu;
+  lo = (lo | (lo >> 4)) & 0x00ff00ffu;
+  hi = (hi | (hi >> 4)) & 0x00ff00ffu;
+  lo = (lo | (lo >> 8)) & 0x0000ffffu;
+  hi = (hi | (hi >> 8)) & 0x0000ffffu;
+  return lo | (hi << 16);
+}
 
-// Number of leading bases (0..32) that agree between A (from a) and T (from t), with
-// N matching anything (prefixEditDistance-forward.C:164 / -reverse.C:186).
+// The low and the high bits of the 32 bases from base g of a read on (base g in bit 0).
+__device__ __forceinline__ uint2 load_planes(const uint2 *p, int g) {
+  const uint2 a = __ldg(p + (g >> 5)), b = __ldg(p + (g >> 5) + 1);
+  return make_uint2(__funnelshift_r(a.x, b.x, g), __funnelshift_r(a.y, b.y, g));
+}
+
+// m without the bits of bases that are N in A (from ga) or T (from gt).
+__device__ __forceinline__ u32 drop_n(u32 m, const u64 *An, int ga, const u64 *Tn, int gt) {
+  if (An) m &= ~even_bits(load_win32(An, ga));
+  if (Tn) m &= ~even_bits(load_win32(Tn, gt));
+  return m;
+}
+
+// Bit 31 - i of the result is set when the bases at distance i (0..31) from A[a] and T[t]
+// differ, in the direction of STEP; an N matches anything
+// (prefixEditDistance-forward.C:164 / -reverse.C:186).
 template <int STEP>
-__device__ __forceinline__ int match_run32(const SeqView &A, int a, const SeqView &T, int t) {
-  u64 wa, wt;
-  if (STEP > 0) {
-    wa = load_win32(A.w, a);
-    wt = load_win32(T.w, t);
-  } else {
-    wa = load_win_rev(A.w, a);
-    wt = load_win_rev(T.w, t);
-  }
-  u64 x  = wa ^ wt;
-  u64 mm = (x | (x >> 1)) & kPairMask;
-  if (mm && (A.nm || T.nm)) {
-    u64 n = 0;
-    if (A.nm) n |= (STEP > 0) ? load_win32(A.nm, a) : load_win_rev(A.nm, a);
-    if (T.nm) n |= (STEP > 0) ? load_win32(T.nm, t) : load_win_rev(T.nm, t);
-    mm &= ~n;
-  }
-  return mm ? (__ffsll((long long)mm) - 1) >> 1 : 32;
+__device__ __forceinline__ u32 mismatch32(const SeqView &A, int a, const SeqView &T, int t) {
+  const int   ga = STEP > 0 ? a : a - 31, gt = STEP > 0 ? t : t - 31;
+  const uint2 x = load_planes(A.p, ga), y = load_planes(T.p, gt);
+  u32         m = (x.x ^ y.x) | (x.y ^ y.y);
+  if (A.nm || T.nm) m = drop_n(m, A.nm, ga, T.nm, gt);
+  return STEP > 0 ? __brev(m) : m;
 }
 
-// 16 bases starting at base g of one read, from the strand viewed as 32-bit words (base
-// i in bits 2*(i%16) of word i/16 on a little-endian device): one funnel shift.  The
-// guard word before a read keeps g >= -32 in bounds.
-__device__ __forceinline__ u32 load_win16(const u64 *w, int g) {
-  const u32 *w32 = reinterpret_cast<const u32 *>(w);
-  const int  wi  = g >> 4;
-  return __funnelshift_r(__ldg(w32 + wi), __ldg(w32 + wi + 1), (g & 15) * 2);
-}
-
-// Number of leading bases (0..16) that agree between A (from a) and T (from t), N
-// matching anything: a cheaper first step for slides that are mostly short.
+// Bases that agree from A[step*row] / T[step*(row+d)] on, capped at `lim` (> 0).
 template <int STEP>
-__device__ __forceinline__ int match_run16(const SeqView &A, int a, const SeqView &T, int t) {
-  u32 wa, wt;
-  if (STEP > 0) {
-    wa = load_win16(A.w, a);
-    wt = load_win16(T.w, t);
-  } else {
-    wa = __brev(load_win16(A.w, a - 15));
-    wt = __brev(load_win16(T.w, t - 15));
-  }
-  const u32 x  = wa ^ wt;
-  u32       mm = (x | (x >> 1)) & 0x55555555u;
-  if (mm && (A.nm || T.nm)) {
-    u32 n = 0;
-    if (A.nm) n |= (STEP > 0) ? load_win16(A.nm, a) : __brev(load_win16(A.nm, a - 15));
-    if (T.nm) n |= (STEP > 0) ? load_win16(T.nm, t) : __brev(load_win16(T.nm, t - 15));
-    mm &= ~n;
-  }
-  return mm ? (__ffs((int)mm) - 1) >> 1 : 16;
-}
-
-// Whether the DP kernels start slides with the 16-base compare: above a 2 % error rate
-// most slides end within a few bases (measured: 11 % less one-warp DP time at 2 % read
-// error), while on low-error reads the slides along the alignment run ~100 bases and the
-// 32-base first step is cheaper (2 % more with the 16-base one at 0.5 % read error).
-__host__ __device__ inline bool slide_first16(double maxErate) { return maxErate > 0.02; }
-
-// Bases that agree from A[step*row] / T[step*(row+d)] on, capped at `lim` (> 0).  The
-// first step compares 32 bases, or 16 when FIRST16 (cheaper when most slides end
-// within a few bases, as at higher error rates); the rest go 32 at a time.
-template <int STEP, bool FIRST16 = false>
 __device__ __forceinline__ int slide(const SeqView &A, int a0, const SeqView &T, int t0, int row, int d, int lim,
                                      unsigned long long &slides) {
-  int  run  = 0;
-  bool more = true;
-  if (FIRST16) {
-    run  = match_run16<STEP>(A, a0 + STEP * row, T, t0 + STEP * (row + d));
-    more = run == 16;
+  int run = 0;
+  while (run < lim) {
+    const int r = __clz((int)mismatch32<STEP>(A, a0 + STEP * (row + run), T, t0 + STEP * (row + d + run)));
+    run += r;
+    if (r < 32) break;
   }
-  if (more)
-    while (run < lim) {
-      int r = match_run32<STEP>(A, a0 + STEP * (row + run), T, t0 + STEP * (row + d + run));
-      run += r;
-      if (r < 32) break;
-    }
   if (run > lim) run = lim;
   slides += (unsigned long long)run;
   return run;

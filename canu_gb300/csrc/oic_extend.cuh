@@ -30,7 +30,7 @@ static __device__ __forceinline__ void extend_loop(WarpDP &w, const ReadsDev &R,
     const int sLen = (int)R.len[pb.sRead], tLen = (int)R.len[pb.tRead];
     int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
     w.err = 0;
-    const int k = warp_extend<GROUP>(w, S, sLen, T, tLen, pb.mStart, pb.mOffset, pb.mLen, sLo, sHi, tLo, tHi, errors);
+    const int k = warp_extend<GROUP>(w, false, S, sLen, T, tLen, pb.mStart, pb.mOffset, pb.mLen, sLo, sHi, tLo, tHi, errors);
     if (lane == 0) {
       out[5 * i + 0] = sLo;
       out[5 * i + 1] = sHi;
@@ -48,19 +48,17 @@ static __device__ __forceinline__ void extend_loop(WarpDP &w, const ReadsDev &R,
 
 // CHECK: validate each problem on the device (for problems the host has not seen)
 // and OR capacity flags into stats[2].
-template <int BANDW, int WARPS, bool CHECK = false>
+template <int WARPS, bool CHECK = false>
 static __global__ void __launch_bounds__(WARPS * 32, (WARPS > 1 ? 3 : 1)) extend_batch_kernel(ReadsDev R, DevParams P, const int *eml,
                                                                   const ExtendProblem *probs, u32 n, WarpScratch scBase,
                                                                   AlignCaps cap, int *out, int *kind, int *deltaLen,
                                                                   u32 *status, unsigned long long *stats) {
-  extern __shared__ int smemRows[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const u64 gw   = (u64)blockIdx.x * WARPS + wib;
   const u64 nw   = (u64)gridDim.x * WARPS;
 
   WarpDP w;
-  int *smA = smemRows + (size_t)wib * 2 * BANDW;
-  warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, smA, smA + BANDW, eml, P);
+  warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, wib * kWarpSmemInts, eml, P);
   extend_loop<CHECK, false>(w, R, probs, n, gw, nw, out, kind, deltaLen, status, stats);
   const unsigned long long slidesWarp = warp_sum64(w.slides);
   if (lane == 0) {
@@ -78,7 +76,6 @@ static __global__ void __launch_bounds__(512, 1) extend_group_kernel(ReadsDev R,
                                                                       WarpScratch scBase, AlignCaps cap, int *out,
                                                                       int *kind, int *deltaLen, u32 *status,
                                                                       unsigned long long *stats, int U) {
-  extern __shared__ int smemRows[];
   __shared__ GroupShared gs;
   const WarpScratch sc = warp_scratch(scBase, cap, blockIdx.x);
   if (threadIdx.x >= 32) {
@@ -89,7 +86,7 @@ static __global__ void __launch_bounds__(512, 1) extend_group_kernel(ReadsDev R,
     return;
   }
   WarpDP w;
-  warp_dp_init(w, sc, cap, smemRows, smemRows + cap.bandW, eml, P);
+  warp_dp_init(w, sc, cap, 0, eml, P);
   w.gs       = &gs;
   w.gThreads = blockDim.x;
   w.gU       = U;

@@ -28,7 +28,8 @@ __device__ __forceinline__ int base_code(unsigned char c, bool &isN, bool &bad) 
 
 // Block per read, thread per 32-base word of both strands.
 __global__ void pack_reads_kernel(const char *ascii, const u64 *srcOff, const u32 *len, const u64 *wordOff, u32 nReads,
-                                  u64 *fwd, u64 *rc, u64 *nfwd, u64 *nrc, unsigned char *hasN, u32 *err) {
+                                  u64 *fwd, u64 *rc, u64 *nfwd, u64 *nrc, uint2 *pfwd, uint2 *prc, unsigned char *hasN,
+                                  u32 *err) {
   for (u32 r = blockIdx.x; r < nReads; r += gridDim.x) {
     const u32  L   = len[r];
     const u64  w0  = wordOff[r];
@@ -54,6 +55,8 @@ __global__ void pack_reads_kernel(const char *ascii, const u64 *srcOff, const u3
       nfwd[w0 + w] = fm;
       rc[w0 + w]   = b;
       nrc[w0 + w]  = bm;
+      pfwd[w0 + w] = make_uint2(even_bits(f), even_bits(f >> 1));
+      prc[w0 + w]  = make_uint2(even_bits(b), even_bits(b >> 1));
     }
     anyN   = __syncthreads_or(anyN);
     anyBad = __syncthreads_or(anyBad);
@@ -239,10 +242,11 @@ inline unsigned grid_for(u64 n, int threads) {
 }  // namespace
 
 void launch_pack_reads(const char *ascii, const u64 *srcOff, const u32 *len, const u64 *wordOff, u32 nReads, u64 *fwd,
-                       u64 *rc, u64 *nfwd, u64 *nrc, unsigned char *hasN, u32 *err, cudaStream_t st) {
+                       u64 *rc, u64 *nfwd, u64 *nrc, uint2 *pfwd, uint2 *prc, unsigned char *hasN, u32 *err,
+                       cudaStream_t st) {
   if (nReads == 0) return;
   unsigned g = nReads < 65535u * 4 ? nReads : 65535u * 4;
-  pack_reads_kernel<<<g, 128, 0, st>>>(ascii, srcOff, len, wordOff, nReads, fwd, rc, nfwd, nrc, hasN, err);
+  pack_reads_kernel<<<g, 128, 0, st>>>(ascii, srcOff, len, wordOff, nReads, fwd, rc, nfwd, nrc, pfwd, prc, hasN, err);
   g_launches++;
 }
 

@@ -19,7 +19,8 @@ namespace oic {
 // Pack ASCII reads into the 2-bit strand arrays (see oic_common.cuh).  err gets
 // kErrBadBase for a character outside ACGTN (either case).
 void launch_pack_reads(const char *ascii, const u64 *srcOff, const u32 *len, const u64 *wordOff, u32 nReads,
-                       u64 *fwd, u64 *rc, u64 *nfwd, u64 *nrc, unsigned char *hasN, u32 *err, cudaStream_t st);
+                       u64 *fwd, u64 *rc, u64 *nfwd, u64 *nrc, uint2 *pfwd, uint2 *prc, unsigned char *hasN, u32 *err,
+                       cudaStream_t st);
 
 // ---------------- hash block ----------------
 // K-mer keys of every block string; key = 1 << 2K for a window holding an N.
@@ -115,8 +116,8 @@ enum StatIdx {
   kStCells, kStSlides, kStExtensions, kStRows, kStCellsNoOlap, kStCount
 };
 
-// One pair per warp, 8 warps per CTA, 512-int shared-memory rows (bandW is ignored).
-void launch_align(int bandW, ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs,
+// One pair per warp, align_warps_per_block() warps per CTA.
+void launch_align(ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs,
                   const u32 *work, u32 nWork, u32 *workCounter, const int4 *nodes, WarpScratch sc, AlignCaps cap,
                   int nWarps, AlignOut out, cudaStream_t st);
 
@@ -128,8 +129,7 @@ void launch_align_group(int threads, int U, int bandW, int ctas, ReadsDev R, Tab
                         WarpScratch sc, AlignCaps cap, AlignOut out, cudaStream_t st);
 
 // Speculative CTA bin: one pair per CTA of align_spec_warps() warps, each warp running
-// whole extensions (one-warp DP, 512-int shared-memory rows, HBM rows up to
-// cap.rowsGW) of the pair's next alive match nodes, replayed in the reference's order.
+// whole extensions (one-warp DP, HBM rows up to cap.rowsGW) of the pair's next alive match nodes, replayed in the reference's order.
 // sc/cap describe ctas * align_spec_warps() warp scratches; a pair's alive flags use the
 // nodeCap bytes of all its CTA's warps.
 void launch_align_spec(int ctas, ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs,
@@ -146,7 +146,7 @@ struct ExtendProblem {
   u32 sRead, sRev, tRead;
   int mStart, mOffset, mLen;
 };
-void launch_extend_batch(int bandW, ReadsDev R, DevParams P, const int *eml, const ExtendProblem *probs, u32 n,
+void launch_extend_batch(ReadsDev R, DevParams P, const int *eml, const ExtendProblem *probs, u32 n,
                          WarpScratch sc, AlignCaps cap, int nWarps, int *out, int *kind, int *deltaLen, u32 *status,
                          unsigned long long *stats, cudaStream_t st);
 
@@ -191,7 +191,6 @@ void launch_run_compact(const u64 *keys, const u64 *runStart, u32 nRuns, u64 nVa
 // Compact per-pair record slots into a dense record array.
 void launch_compact_records(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst, cudaStream_t st);
 
-int align_warps_per_block(int bandW);
-size_t align_smem_bytes(int bandW);
+int align_warps_per_block();
 
 }  // namespace oic

@@ -37,7 +37,6 @@
 namespace oic {
 namespace {
 
-constexpr int    kNaBandW    = 512;
 constexpr int    kNaWarps    = 32;                // 4 blocks of 8 warps
 constexpr int    kNaArenaCap = 1 << 17;           // kept DP cells per warp
 constexpr int    kNaRowCap   = 8192;              // error rows per warp
@@ -96,14 +95,18 @@ extern "C" int oic_extend_batch_noalloc(oic_ctx *ctx, uint32_t nAlign, const oic
   cap.arenaCap = kNaArenaCap;
   cap.rowCap   = kNaRowCap;
   cap.nodeCap  = 0;
-  cap.bandW    = kNaBandW;
-  cap.rowsGW   = kNaBandW;
+  cap.bandW    = kRowW;
+  cap.rowsGW   = kRowW;
 
   // Counters in the context's preallocated block: [cells, slides, error flags].
   unsigned long long *stats = (unsigned long long *)v.ctr32 + kNoAllocStatBase;
   if (cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), v.st) != cudaSuccess) return OIC_ERR_CUDA;
   constexpr int wpb = 8;
-  extend_batch_kernel<kNaBandW, wpb, true><<<kNaWarps / wpb, wpb * 32, (size_t)wpb * 2 * kNaBandW * sizeof(int), v.st>>>(
+  constexpr size_t smem = (size_t)wpb * kWarpSmemInts * sizeof(int);
+  if (cudaFuncSetAttribute(extend_batch_kernel<wpb, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return OIC_ERR_CUDA;
+  extend_batch_kernel<wpb, true><<<kNaWarps / wpb, wpb * 32, smem, v.st>>>(
       v.R, v.dp, v.eml, (const ExtendProblem *)dProblems, nAlign, sc, cap, dOut, dKind, dDeltaLen, dStatus, stats);
   g_launches++;
   unsigned long long counters[3] = {0, 0, 0};

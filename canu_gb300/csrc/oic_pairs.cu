@@ -21,7 +21,7 @@ namespace oic {
 
 namespace {
 
-constexpr int kAlignWarpsSmall = 8;   // bandW 512
+constexpr int kAlignWarps = 8;
 
 struct Olap {
   int    s_lo, s_hi, t_lo, t_hi;
@@ -245,7 +245,7 @@ __device__ void output_partial(u32 *dst, u32 sID, u32 tID, int rev, const Olap &
 
 // Process_Matches for one pair.  Counts go to ps.pc, records (lane 0) to recOut.
 // Returns false on a capacity overflow: the caller then discards ps.pc and the records.
-template <bool GROUP, bool FIRST16 = false>
+template <bool GROUP>
 __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const TableDev &Tb, const PairRec &pr,
                              const int4 *nodesAll, u32 *recOut, u32 &nRec, int extLimit) {
   const int lane = threadIdx.x & 31;
@@ -345,7 +345,8 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     const int4 lm = nodes[li];
 
     int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
-    const int kind = warp_extend<GROUP, FIRST16>(w, S, sLen, T, tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi, errors);
+    const int kind = warp_extend<GROUP>(w, !P.partial, S, sLen, T, tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi,
+                                        errors);
     if (w.err) {
       w.cells  = cells0;
       w.slides = slides0;
@@ -420,7 +421,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
 }
 
 // The work loop of one warp: pairs from the shared work list until it is empty.
-template <bool GROUP, bool FIRST16 = false>
+template <bool GROUP>
 static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const ReadsDev &R, const TableDev &Tb,
                                                   const PairRec *pairs, const u32 *work, u32 nWork, u32 *workCounter,
                                                   const int4 *nodes, const AlignOut &out) {
@@ -444,7 +445,7 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
     const unsigned long long cellsBefore = w.cells;
     int extLimit = 0;   // 0: every match node may be extended (the reference's rule)
     if (out.tierLogit && out.tierLogit[pi] < out.tierThr) extLimit = out.tierBudget;
-    const bool ok = process_pair<GROUP, FIRST16>(w, ps, R, Tb, pr, nodes, out.rec + (u64)pi * 18, nRec, extLimit);
+    const bool ok = process_pair<GROUP>(w, ps, R, Tb, pr, nodes, out.rec + (u64)pi * 18, nRec, extLimit);
     if (lane == 0) {
       if (ok) {
         if (nRec == 0) ps.pc.v[kStCellsNoOlap] += w.cells - cellsBefore;
@@ -476,20 +477,16 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
   }
 }
 
-// One pair per warp, WARPS warps per CTA; FIRST16: slides start with a 16-base compare.
-template <int BANDW, int WARPS, bool FIRST16>
-__global__ void __launch_bounds__(WARPS * 32, (WARPS > 1 ? OIC_ALIGN_MIN_BLOCKS : 1)) align_kernel(ReadsDev R, TableDev Tb, DevParams P, const int *eml,
-                                                           const PairRec *pairs, const u32 *work, u32 nWork,
-                                                           u32 *workCounter, const int4 *nodes, WarpScratch scBase,
-                                                           AlignCaps cap, AlignOut out) {
-  extern __shared__ int smemRows[];
-  __shared__ PairSmem pairSmem[WARPS];
+// One pair per warp, kAlignWarps warps per CTA.
+__global__ void __launch_bounds__(kAlignWarps * 32, OIC_ALIGN_MIN_BLOCKS) align_kernel(
+    ReadsDev R, TableDev Tb, DevParams P, const int *eml, const PairRec *pairs, const u32 *work, u32 nWork,
+    u32 *workCounter, const int4 *nodes, WarpScratch scBase, AlignCaps cap, AlignOut out) {
+  __shared__ PairSmem pairSmem[kAlignWarps];
   const int wib = threadIdx.x >> 5;
-  const u64 gw  = (u64)blockIdx.x * WARPS + wib;
+  const u64 gw  = (u64)blockIdx.x * kAlignWarps + wib;
   WarpDP w;
-  int *smA = smemRows + (size_t)wib * 2 * BANDW;
-  warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, smA, smA + BANDW, eml, P);
-  align_loop<false, FIRST16>(w, pairSmem[wib], R, Tb, pairs, work, nWork, workCounter, nodes, out);
+  warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, wib * kWarpSmemInts, eml, P);
+  align_loop<false>(w, pairSmem[wib], R, Tb, pairs, work, nWork, workCounter, nodes, out);
 }
 
 // One pair per CTA (the wide bins): warp 0 runs the pair logic, and every error-row
@@ -500,7 +497,6 @@ __global__ void __launch_bounds__(512, 1) align_group_kernel(ReadsDev R, TableDe
                                                               const PairRec *pairs, const u32 *work, u32 nWork,
                                                               u32 *workCounter, const int4 *nodes, WarpScratch scBase,
                                                               AlignCaps cap, AlignOut out, int U) {
-  extern __shared__ int smemRows[];
   __shared__ PairSmem    pairSmem;
   __shared__ GroupShared gs;
   const WarpScratch sc = warp_scratch(scBase, cap, blockIdx.x);
@@ -512,7 +508,7 @@ __global__ void __launch_bounds__(512, 1) align_group_kernel(ReadsDev R, TableDe
     return;
   }
   WarpDP w;
-  warp_dp_init(w, sc, cap, smemRows, smemRows + cap.bandW, eml, P);
+  warp_dp_init(w, sc, cap, 0, eml, P);
   w.gs       = &gs;
   w.gThreads = blockDim.x;
   w.gU       = U;
@@ -563,7 +559,7 @@ static __device__ __forceinline__ void spec_work(WarpDP &w, SpecShared &ss, int 
   const unsigned long long c0 = w.cells, r0 = w.rows, s0 = w.slides;
   w.err = 0;
   int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
-  const int kind = warp_extend<false>(w, ss.S, ss.sLen, ss.T, ss.tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi, errors);
+  const int kind = warp_extend<false>(w, !w.P.partial, ss.S, ss.sLen, ss.T, ss.tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi, errors);
   const unsigned long long sl = warp_sum64(w.slides - s0);
   if (lane == 0) {
     SpecRes &r = ss.res[wib];
@@ -789,15 +785,13 @@ __device__ bool process_pair_spec(WarpDP &w, PairSmem &ps, SpecShared &ss, const
 __global__ void __launch_bounds__(kSpecWarps * 32, OIC_ALIGN_MIN_BLOCKS) align_spec_kernel(
     ReadsDev R, TableDev Tb, DevParams P, const int *eml, const PairRec *pairs, const u32 *work, u32 nWork,
     u32 *workCounter, const int4 *nodes, WarpScratch scBase, AlignCaps cap, AlignOut out) {
-  extern __shared__ int smemRows[];
   __shared__ PairSmem    ps;
   __shared__ SpecShared  ss;
   __shared__ WarpScratch wsc[kSpecWarps];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nThr = blockDim.x;
   const u64 gw = (u64)blockIdx.x * kSpecWarps + wib;
   WarpDP w;
-  int *smA = smemRows + (size_t)wib * 2 * 512;
-  warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, smA, smA + 512, eml, P);
+  warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, wib * kWarpSmemInts, eml, P);
   if (lane == 0) wsc[wib] = w.sc;
   w.cap.nodeCap = cap.nodeCap * kSpecWarps;   // warp 0's alive flags span the CTA's slots
   __syncthreads();
@@ -933,21 +927,18 @@ __global__ void compact_records_kernel(const u32 *rec, const u32 *cnt, const u32
 
 }  // namespace
 
-int align_warps_per_block(int) { return kAlignWarpsSmall; }
+int align_warps_per_block() { return kAlignWarps; }
 
-size_t align_smem_bytes(int) { return (size_t)kAlignWarpsSmall * 2 * 512 * sizeof(int); }
+static constexpr size_t kAlignSmem = (size_t)kAlignWarps * kWarpSmemInts * sizeof(int);
 
-void launch_align(int, ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs, const u32 *work,
+void launch_align(ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs, const u32 *work,
                   u32 nWork, u32 *workCounter, const int4 *nodes, WarpScratch sc, AlignCaps cap, int nWarps,
                   AlignOut out, cudaStream_t st) {
   if (nWork == 0 && !out.nWorkDev) return;
-  const int    blocks = (nWarps + kAlignWarpsSmall - 1) / kAlignWarpsSmall;
-  const size_t smem   = align_smem_bytes(512);
-  cap.bandW           = 512;
-  auto k = slide_first16(P.maxErate) ? align_kernel<512, kAlignWarpsSmall, true>
-                                     : align_kernel<512, kAlignWarpsSmall, false>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k<<<blocks, kAlignWarpsSmall * 32, smem, st>>>(R, T, P, eml, pairs, work, nWork, workCounter, nodes, sc, cap, out);
+  const int    blocks = (nWarps + kAlignWarps - 1) / kAlignWarps;
+  cudaFuncSetAttribute(align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmem);
+  align_kernel<<<blocks, kAlignWarps * 32, kAlignSmem, st>>>(R, T, P, eml, pairs, work, nWork, workCounter, nodes, sc,
+                                                             cap, out);
   g_launches++;
 }
 
@@ -967,9 +958,7 @@ void launch_align_spec(int ctas, ReadsDev R, TableDev T, DevParams P, const int 
                        const u32 *work, u32 nWork, u32 *workCounter, const int4 *nodes, WarpScratch sc, AlignCaps cap,
                        AlignOut out, cudaStream_t st) {
   if (nWork == 0 && !out.nWorkDev) return;
-  cap.bandW         = 512;
-  cap.rowsGW        = cap.rowsGW < 512 ? 512 : cap.rowsGW;
-  const size_t smem = (size_t)kSpecWarps * 2 * 512 * sizeof(int);
+  const size_t smem = (size_t)kSpecWarps * kWarpSmemInts * sizeof(int);
   cudaFuncSetAttribute(align_spec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   align_spec_kernel<<<ctas, kSpecWarps * 32, smem, st>>>(R, T, P, eml, pairs, work, nWork, workCounter, nodes, sc, cap,
                                                         out);
@@ -978,16 +967,14 @@ void launch_align_spec(int ctas, ReadsDev R, TableDev T, DevParams P, const int 
 
 int align_spec_warps() { return kSpecWarps; }
 
-void launch_extend_batch(int, ReadsDev R, DevParams P, const int *eml, const ExtendProblem *probs, u32 n,
+void launch_extend_batch(ReadsDev R, DevParams P, const int *eml, const ExtendProblem *probs, u32 n,
                          WarpScratch sc, AlignCaps cap, int nWarps, int *out, int *kind, int *deltaLen, u32 *status,
                          unsigned long long *stats, cudaStream_t st) {
   if (n == 0) return;
-  const int    blocks = (nWarps + kAlignWarpsSmall - 1) / kAlignWarpsSmall;
-  const size_t smem   = align_smem_bytes(512);
-  cap.bandW           = 512;
-  auto k = extend_batch_kernel<512, kAlignWarpsSmall>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k<<<blocks, kAlignWarpsSmall * 32, smem, st>>>(R, P, eml, probs, n, sc, cap, out, kind, deltaLen, status, stats);
+  const int    blocks = (nWarps + kAlignWarps - 1) / kAlignWarps;
+  auto k = extend_batch_kernel<kAlignWarps>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmem);
+  k<<<blocks, kAlignWarps * 32, kAlignSmem, st>>>(R, P, eml, probs, n, sc, cap, out, kind, deltaLen, status, stats);
   g_launches++;
 }
 

@@ -119,7 +119,9 @@ __global__ void __launch_bounds__(kSeedThreads) seed_kernel(ReadsDev R, TableDev
 
     const u32 sRead = segReads[seg >> 1];
     const int dir   = seg & 1;
-    const SeqView S = make_view(R, sRead, dir);
+    const u64 wo    = R.wordOff[sRead];
+    const u64 *Sw   = (dir ? R.rc : R.fwd) + wo;
+    const u64 *Sn   = R.hasN[sRead] ? (dir ? R.nrc : R.nfwd) + wo : nullptr;
     const int sLen  = (int)R.len[sRead];
     const int nK    = sLen - K + 1;
     const i64 thr   = (i64)(sRead + 1) - (i64)T.firstID;   // T qualifies iff tStr > thr
@@ -136,8 +138,8 @@ __global__ void __launch_bounds__(kSeedThreads) seed_kernel(ReadsDev R, TableDev
       const int i = i0 + lane;
       u32 n = 0, qEnd = 0;
       if (i < nK) {
-        u64 key = load_win32(S.w, i) & kmask;
-        bool ok = !(S.nm && (load_win32(S.nm, i) & kmask));
+        u64 key = load_win32(Sw, i) & kmask;
+        bool ok = !(Sn && (load_win32(Sn, i) & kmask));
         u64 val;
         if (ok && table_find(T, key, val)) {
           if (val >> 63) {

@@ -1,0 +1,80 @@
+"""The one-warp DP where it can go wrong, against the oracle: slides that end around the 32-
+and 1024-base steps, bands around the 32- and 64-diagonal chunks and past the shared-memory
+rows, reads with N, both directions."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import canu_gb300 as oic
+from test_gpu_edges import mutate, rand_seq
+from test_gpu_extend import port_aligner
+
+pytestmark = pytest.mark.gpu
+
+K = 22
+COMP = bytes.maketrans(b"acgtn", b"tgcan")
+
+
+def slides(r):
+    """Reads that agree over runs of given lengths, each ended by one error, on both sides of
+    an exact seed in the middle."""
+    pairs = []
+    for run in (1, 31, 32, 33, 63, 64, 65, 96, 1023, 1024, 1025, 1055, 1056, 1057, 2048, 2081):
+        for kind in "sid":
+            left, seed, right = rand_seq(r, 2 * run + 40), rand_seq(r, K), rand_seq(r, 2 * run + 40)
+            other = []
+            for side, at in ((left, len(left) - 1 - run), (right, run)):
+                c = side[at]
+                new = {"s": "ACGT"[("ACGT".index(c) + 1) % 4], "i": c + "ACGT"[("ACGT".index(c) + 2) % 4], "d": ""}[kind]
+                other.append(side[:at] + new + side[at + 1:])
+            pairs.append((left + seed + right, other[0] + seed + other[1], len(left), len(other[0])))
+    return pairs
+
+
+def noisy(r, n, length, err, with_n=False):
+    pairs = []
+    for i in range(n):
+        left, seed, right = rand_seq(r, length), rand_seq(r, K), rand_seq(r, length // 2 + 37 * i)
+        a, b = mutate(r, left, err / 2), mutate(r, right, err / 2)
+        c, d = mutate(r, left, err / 2), mutate(r, right, err / 2)
+        if with_n:
+            a = "".join("N" if r.random() < 0.01 else x for x in a)
+            d = "".join("N" if r.random() < 0.01 else x for x in d)
+        pairs.append((a + seed + b, c + seed + d, len(a), len(c)))
+    return pairs
+
+
+def unrelated(r):
+    return [(rand_seq(r, 900), rand_seq(r, 1100), 400 + i, 500 - i) for i in range(8)]
+
+
+@pytest.mark.parametrize("name,erate,partial", [("slides", 0.06, 0), ("slides", 0.01, 1), ("narrow", 0.02, 0),
+                                                ("mid", 0.06, 0), ("wide", 0.12, 0), ("wide", 0.12, 1), ("n", 0.06, 0),
+                                                ("unrelated", 0.12, 0)])
+def test_row_loop_edges_match_oracle(name, erate, partial, built, oracle):
+    r = np.random.default_rng(11)
+    pairs = {"slides": lambda: slides(r), "narrow": lambda: noisy(r, 6, 3000, 0.012), "mid": lambda: noisy(r, 6, 2500, 0.03),
+             # 2 % error under a 12 % limit: the band passes 508 diagonals after some 400 rows
+             "wide": lambda: noisy(r, 2, 26000, 0.02), "n": lambda: noisy(r, 6, 2000, 0.03, True),
+             "unrelated": lambda: unrelated(r)}[name]()
+    seqs, prob = [], []
+    for i, (s, t, ms, mt) in enumerate(pairs):
+        rev = i % 2
+        stored = s.encode().lower()
+        seqs += [stored[::-1].translate(COMP) if rev else stored, t.encode().lower()]
+        prob.append((2 * i + 1, rev, 2 * i + 2, ms, mt, K))
+    off = np.cumsum([0] + [len(x) for x in seqs])
+    erate = float(np.float32(erate))
+    with oic.Overlapper(oic.default_params(kmerLen=K, maxErate=erate, partial=partial)) as ov:
+        ov.set_reads(np.ones(len(seqs)), [len(x) for x in seqs], off[:-1], np.frombuffer(b"".join(seqs), np.uint8))
+        a = np.array(prob)
+        out, kind, dl = ov.extend_batch(*[a[:, j] for j in range(6)])
+    plib = ctypes.CDLL(oracle["lib"])
+    al = port_aligner(plib, erate, 1.0, partial)
+    for i, (s, t, ms, mt) in enumerate(pairs):
+        o, n = np.zeros(5, dtype=np.int32), ctypes.c_int32()
+        k = plib.oic_port_extend(al, s.encode().lower(), len(s), t.encode().lower(), len(t), ms, mt, K, o.ctypes.data, None,
+                                 ctypes.byref(n), None, None)
+        assert k == kind[i] and (o == out[i]).all() and n.value == dl[i], (i, k, o, n.value, kind[i], out[i], dl[i])
+    plib.oic_port_aligner_free(al)
