@@ -281,7 +281,7 @@ struct AlignConfig {
 AlignConfig align_normal(const oic_ctx *c) {
   AlignConfig a;
   a.bandW         = 512;
-  a.warps         = c->nSM * OIC_ALIGN_MIN_BLOCKS * align_warps_per_block();
+  a.warps         = c->nSM * align_warps_per_block();
   a.caps.arenaCap = 1 << 20;
   a.caps.rowCap   = 1 << 14;
   a.caps.nodeCap  = 1 << 16;

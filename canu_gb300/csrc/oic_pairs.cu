@@ -21,7 +21,8 @@ namespace oic {
 
 namespace {
 
-constexpr int kAlignWarps = 8;
+constexpr int kExtendWarps = 8;    // warps per CTA of the batched extensions
+constexpr int kAlignWarps  = 24;   // warps per CTA of the one-warp DP: a team, one CTA per SM
 
 struct Olap {
   int    s_lo, s_hi, t_lo, t_hi;
@@ -174,6 +175,13 @@ __device__ __forceinline__ void put_record(u32 *dst, u32 a, u32 b, u32 ahg5, u32
   dst[5] = (u32)d1;
 }
 
+// The outcome of one extension: Extend_Alignment's outputs and the work it took.
+struct ExtRes {
+  int sLo, sHi, tLo, tHi, errors, kind, leftLen;
+  u32 err;
+  unsigned long long cells, slides, rows;
+};
+
 struct PairCounts {
   unsigned long long v[kStCount];
 };
@@ -185,6 +193,7 @@ struct PairSmem {
   int                nExt;       // extensions run for the pair in flight
   int                firstHit;   // index of its first extension that added an overlap, -1 none
   unsigned long long cellsFirst; // DP cells of its first extension
+  ExtRes             res;        // its latest extension
   PairCounts         pc;    // counts of the pair in flight
   PairCounts         acc;   // committed counts of the warp
 };
@@ -243,11 +252,219 @@ __device__ void output_partial(u32 *dst, u32 sID, u32 tID, int rev, const Olap &
 }
 
 
+// Extends node lm of (S, T) into res; the deltas stay in the warp's scratch.  The work is
+// reported in res only.
+__device__ __forceinline__ void extend_node(WarpDP &w, const SeqView &S, int sLen, const SeqView &T, int tLen,
+                                            const int4 &lm, ExtRes &res) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long c0 = w.cells, r0 = w.rows, s0 = w.slides;
+  w.err = 0;
+  int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
+  const int kind = warp_extend<false>(w, !w.P.partial, S, sLen, T, tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi, errors);
+  const unsigned long long sl = warp_sum64(w.slides - s0);
+  if (lane == 0) {
+    res.sLo = sLo; res.sHi = sHi; res.tLo = tLo; res.tHi = tHi; res.errors = errors; res.kind = kind;
+    res.leftLen = w.leftLen;
+    res.err     = w.err;
+    res.cells   = w.cells - c0;
+    res.rows    = w.rows - r0;
+    res.slides  = sl;
+  }
+  w.cells  = c0;
+  w.rows   = r0;
+  w.slides = s0;
+  w.err    = 0;
+  __syncwarp();
+}
+
+// ---------------------------------------------------------------------------------
+// The team of a one-warp DP CTA.  Each warp takes pairs of its own; a warp that finds the
+// work list empty helps the others of its CTA.  Process_Matches extends, one after
+// another, the longest alive match node (first in list order on ties) and then removes the
+// nodes that lie on its alignment (Process_String_Overlaps.C:420-491).  An extension
+// depends only on its own node, and removal only ever takes nodes away, so the nodes are
+// extended in the order (length descending, list index ascending), skipping removed ones.
+// A helper claims the next unclaimed alive node of an open pair, extends it, and holds the
+// result until the pair's owner either reaches that node, and commits it exactly as if it
+// had run the extension itself, or removes it.  Only committed extensions count as work.
+//
+// A pair takes 20 to 1,000 extensions one after another, so without helpers a batch lasts
+// as long as its longest chain.  DP times without and with the team: 59 reads 17.1 -> 5.8
+// ms, 20 Mbp of 2 % reads 321 -> 193 ms, 4 Mbp of noisy reads 504 -> 135 ms.  Teams of 16,
+// 20, 24 and 28 warps measured 222 / 203 / 194 / 194 ms on the 2 % reads and 541 / 499 /
+// 477 / 478 ms on 150 Mbp of 0.5 % reads, where no chain is long (three CTAs of 8 warps
+// without helpers: 426 ms).
+//
+// Every wait is bounded: an owner that waits too long for a result extends the node
+// itself, a helper that waits too long for its result to be taken leaves (its scratch
+// stays readable).
+enum { kSlotFree = 0, kSlotRunning = 1, kSlotDone = 2, kSlotCancelled = 3 };
+constexpr unsigned char kNodeDead = 0, kNodeOpen = 1, kNodeOwner = 2, kNodeHelper = 3;   // kNodeHelper + h: helper h
+
+struct TeamPair {            // a pair open to helpers
+  int            lock;
+  int            open;       // nodes that can be claimed (kNodeOpen); 0: none, or no open pair
+  SeqView        S, T;
+  int            sLen, tLen, cnt;
+  const int4    *nodes;
+  unsigned char *alive;      // kNode* of each match node, written under the lock
+};
+struct TeamSlot {            // a helper's claim
+  int            state;      // kSlot*
+  int            owner;
+  const int     *deltaL;
+  ExtRes         res;
+};
+struct Team {
+  int      owners;           // warps that still take pairs from the work list
+  TeamPair pair[kAlignWarps];
+  TeamSlot slot[kAlignWarps];
+};
+
+constexpr int kLockTries = 1 << 22, kWaitTries = 1 << 24;
+
+// Lock of a pair, taken by a warp (bounded: false when it could not be had).
+__device__ __forceinline__ bool team_lock(TeamPair &p) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) {
+    int tries = 0;
+    while (atomicCAS(&p.lock, 0, 1) != 0) {
+      if (++tries > kLockTries) { ok = 0; break; }
+      __nanosleep(64);
+    }
+    __threadfence_block();
+  }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+__device__ __forceinline__ void team_unlock(TeamPair &p) {
+  __threadfence_block();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) atomicExch(&p.lock, 0);
+  __syncwarp();
+}
+__device__ __forceinline__ int team_read(const int &v) { return *(const volatile int *)&v; }
+
+// The best node (length descending, index ascending) whose state lies in [lo, hi]; -1: none.
+__device__ __forceinline__ int best_node(const int4 *nodes, const volatile unsigned char *alive, int cnt, int lo, int hi) {
+  int myLen = -1, myIdx = INT_MAX;
+  for (int i = threadIdx.x & 31; i < cnt; i += 32) {
+    const int a = alive[i];
+    if (a >= lo && a <= hi) {
+      const int len = nodes[i].y;
+      if (len > myLen) {
+        myLen = len;
+        myIdx = i;
+      }
+    }
+  }
+  const int maxLen = __reduce_max_sync(0xffffffffu, myLen);
+  if (maxLen < 0) return -1;
+  return __reduce_min_sync(0xffffffffu, myLen == maxLen ? myIdx : INT_MAX);
+}
+
+// Frees or cancels helper h's claim (by the owner, under its pair's lock, one lane).
+__device__ __forceinline__ void team_drop(Team &tm, int h) {
+  TeamSlot &s = tm.slot[h];
+  if (atomicCAS(&s.state, kSlotRunning, kSlotCancelled) == kSlotDone) atomicExch(&s.state, kSlotFree);
+}
+
+// Closes warp `me`'s pair: no new claims, outstanding ones dropped.  False when the lock
+// could not be had (the pair is closed all the same; its helpers give up by themselves).
+__device__ __forceinline__ bool team_close(Team &tm, int me) {
+  TeamPair &p   = tm.pair[me];
+  const int lane = threadIdx.x & 31;
+  const bool ok  = team_lock(p);
+  if (lane == 0) atomicExch(&p.open, 0);
+  if (ok) {
+    if (lane < kAlignWarps) {
+      const int st = team_read(tm.slot[lane].state);
+      if ((st == kSlotRunning || st == kSlotDone) && team_read(tm.slot[lane].owner) == me) team_drop(tm, lane);
+    }
+    team_unlock(p);
+  }
+  return ok;
+}
+
+// A warp without pairs of its own: extend nodes of the team's open pairs until every
+// owner is done.
+static __device__ __noinline__ void team_help(WarpDP &w, Team &tm, int me) {
+  const int lane = threadIdx.x & 31;
+  TeamSlot &slot = tm.slot[me];
+  for (int idle = 0; idle < kWaitTries;) {
+    if (__shfl_sync(0xffffffffu, team_read(tm.owners), 0) == 0) return;
+    const unsigned open = __ballot_sync(0xffffffffu, lane < kAlignWarps && team_read(tm.pair[lane].open) > 0);
+    int  node = -1;
+    SeqView S, T;
+    int  sLen = 0, tLen = 0;
+    int4 lm = make_int4(0, 0, 0, 0);
+    if (open) {
+      // The first open pair after this warp, so that the helpers spread over the pairs.
+      const unsigned above = open & ~((2u << me) - 1);
+      const int      o     = __ffs((int)(above ? above : open)) - 1;
+      TeamPair      &p     = tm.pair[o];
+      if (team_lock(p)) {
+        if (__shfl_sync(0xffffffffu, team_read(p.open), 0) > 0)
+          node = best_node(p.nodes, p.alive, p.cnt, kNodeOpen, kNodeOpen);
+        if (node >= 0) {
+          S    = p.S;
+          T    = p.T;
+          sLen = p.sLen;
+          tLen = p.tLen;
+          lm   = p.nodes[node];
+          __syncwarp();
+          if (lane == 0) {
+            ((volatile unsigned char *)p.alive)[node] = (unsigned char)(kNodeHelper + me);
+            *(volatile int *)&slot.owner              = o;
+            p.open--;
+            atomicExch(&slot.state, kSlotRunning);
+          }
+        }
+        team_unlock(p);
+      }
+    }
+    if (node < 0) {
+      __nanosleep(500);
+      idle++;
+      continue;
+    }
+    idle = 0;
+    extend_node(w, S, sLen, T, tLen, lm, slot.res);
+    __threadfence_block();
+    __syncwarp();
+    if (lane == 0 && atomicCAS(&slot.state, kSlotRunning, kSlotDone) == kSlotCancelled)
+      atomicExch(&slot.state, kSlotFree);
+    __syncwarp();
+    // Hold the result until it is taken or dropped.
+    for (int tries = 0; __shfl_sync(0xffffffffu, team_read(slot.state), 0) == kSlotDone; tries++) {
+      if (tries > kWaitTries) return;
+      __nanosleep(200);
+    }
+  }
+}
+
+// The owner waits for helper h's result; false when it did not come in time (the claim is
+// then dropped).
+__device__ __forceinline__ bool team_wait(Team &tm, int h) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0) {
+    int tries = 0;
+    while (team_read(tm.slot[h].state) != kSlotDone) {
+      if (++tries > kWaitTries) { ok = 0; break; }
+      __nanosleep(100);
+    }
+    if (!ok) team_drop(tm, h);
+    __threadfence_block();
+  }
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
 // Process_Matches for one pair.  Counts go to ps.pc, records (lane 0) to recOut.
 // Returns false on a capacity overflow: the caller then discards ps.pc and the records.
+// tm (one-warp DP only): the CTA's team, of which this is warp `me`.
 template <bool GROUP>
 __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const TableDev &Tb, const PairRec &pr,
-                             const int4 *nodesAll, u32 *recOut, u32 &nRec, int extLimit) {
+                             const int4 *nodesAll, u32 *recOut, u32 &nRec, int extLimit, Team *tm, int me) {
   const int lane = threadIdx.x & 31;
   const DevParams &P = w.P;
   if (lane == 0) {
@@ -321,47 +538,83 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     w.err |= kErrNodesPerPair;
     return false;
   }
-  for (int i = lane; i < cnt; i += 32) w.sc.alive[i] = 1;
+  volatile unsigned char *const alive = w.sc.alive;
+  for (int i = lane; i < cnt; i += 32) alive[i] = kNodeOpen;
   __syncwarp();
 
   const SeqView S = make_view(R, sRead, rev);
   const SeqView T = make_view(R, tRead, 0);
   const unsigned long long cells0 = w.cells, slides0 = w.slides, rows0 = w.rows;
 
+  // Pairs that run one extension, or stop after a few without an overlap, are not opened.
+  const bool open = !GROUP && cnt > 1 && !cons && extLimit == 0;
+  if (open) {
+    TeamPair &p = tm->pair[me];
+    if (lane == 0) {
+      p.S     = S;
+      p.T     = T;
+      p.sLen  = sLen;
+      p.tLen  = tLen;
+      p.cnt   = cnt;
+      p.nodes = nodes;
+      p.alive = w.sc.alive;
+      __threadfence_block();
+      atomicExch(&p.open, cnt);
+    }
+    __syncwarp();
+  }
+
   while (true) {
     // Longest remaining match, first in list order on ties (:424-431).
-    int myLen = -1, myIdx = INT_MAX;
-    for (int i = lane; i < cnt; i += 32)
-      if (w.sc.alive[i]) {
-        const int len = nodes[i].y;
-        if (len > myLen) {
-          myLen = len;
-          myIdx = i;
+    if (open && !team_lock(tm->pair[me])) { w.err |= kErrInternal; break; }
+    const int li = best_node(nodes, alive, cnt, kNodeOpen, 255);
+    int h = -1;
+    if (open) {
+      if (li >= 0) {
+        h = (int)alive[li] - kNodeHelper;
+        __syncwarp();
+        if (h < 0 && lane == 0) {
+          alive[li] = kNodeOwner;
+          tm->pair[me].open--;
         }
       }
-    const int maxLen = __reduce_max_sync(0xffffffffu, myLen);
-    if (maxLen < 0) break;
-    const int li = __reduce_min_sync(0xffffffffu, myLen == maxLen ? myIdx : INT_MAX);
-    const int4 lm = nodes[li];
-
-    int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
-    const int kind = warp_extend<GROUP>(w, !P.partial, S, sLen, T, tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi,
-                                        errors);
-    if (w.err) {
-      w.cells  = cells0;
-      w.slides = slides0;
-      w.rows   = rows0;
-      return false;
+      team_unlock(tm->pair[me]);
     }
-    const bool dov = (kind == kDovetail) || P.partial;
+    if (li < 0) break;
+
+    ExtRes    &res = ps.res;
+    const int *dl  = w.sc.deltaL;
+    if (!GROUP && h >= 0 && team_wait(*tm, h)) {
+      if (lane == 0) res = tm->slot[h].res;
+      dl = tm->slot[h].deltaL;
+      __syncwarp();
+      w.cells += res.cells;
+      w.rows += res.rows;
+      if (lane == 0) w.slides += res.slides;
+    } else {
+      h = -1;
+      const int4 lm = nodes[li];
+      int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
+      const int kind = warp_extend<GROUP>(w, !P.partial, S, sLen, T, tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi, errors);
+      if (lane == 0) {
+        res.sLo = sLo; res.sHi = sHi; res.tLo = tLo; res.tHi = tHi; res.errors = errors; res.kind = kind;
+        res.leftLen = w.leftLen;
+        res.err     = 0;
+      }
+      __syncwarp();
+    }
+    w.err |= res.err;
+    if (w.err) break;
+    const int  sLo = res.sLo, sHi = res.sHi, tLo = res.tLo, tHi = res.tHi, leftLen = res.leftLen;
+    const bool dov = (res.kind == kDovetail) || P.partial;
     if (lane == 0) {
       ps.pc.v[kStExtensions]++;
       bool added = false;
       if (dov && 1 + sHi - sLo >= P.minOlapLen && 1 + tHi - tLo >= P.minOlapLen) {
         const int    olapLen = 1 + min(sHi - sLo, tHi - tLo);
-        const double quality = __ddiv_rn((double)errors, (double)olapLen);
-        if (errors <= error_bound(olapLen, P.maxErate)) {
-          add_overlap(P.partial, sLo, sHi, tLo, tHi, quality, w.leftLen, ps.olap, ps.nOlap);
+        const double quality = __ddiv_rn((double)res.errors, (double)olapLen);
+        if (res.errors <= error_bound(olapLen, P.maxErate)) {
+          add_overlap(P.partial, sLo, sHi, tLo, tHi, quality, leftLen, ps.olap, ps.nOlap);
           added = true;
         }
       }
@@ -378,16 +631,41 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     }
 
     // Drop the longest match and every match that lies on the alignment (:476-490).
-    for (int i = lane; i < cnt; i += 32) {
-      if (!w.sc.alive[i]) continue;
-      const int4 q = nodes[i];
-      bool rm = (i == li);
-      if (!rm && dov && sLo - kShiftSlack <= q.z && q.z + q.y <= (sHi + 1) + kShiftSlack - 1 &&
-          lies_on_alignment(w.sc.deltaL, w.leftLen, q.z, q.x, sLo, tLo))
-        rm = true;
-      if (rm) w.sc.alive[i] = 0;
+    for (int i0 = 0; i0 < cnt; i0 += 32) {
+      const int i = i0 + lane;
+      bool rm = false;
+      if (i < cnt && alive[i] != kNodeDead) {
+        rm = i == li;
+        if (!rm && dov) {
+          const int4 q = nodes[i];
+          rm = sLo - kShiftSlack <= q.z && q.z + q.y <= (sHi + 1) + kShiftSlack - 1 &&
+               lies_on_alignment(dl, leftLen, q.z, q.x, sLo, tLo);
+        }
+      }
+      if (!open) {
+        if (rm) alive[i] = kNodeDead;
+      } else if (__any_sync(0xffffffffu, rm)) {
+        if (!team_lock(tm->pair[me])) { w.err |= kErrInternal; break; }
+        const int st = rm ? (int)alive[i] : (int)kNodeDead;
+        if (rm) {
+          alive[i] = kNodeDead;
+          if (st >= kNodeHelper && i != li) team_drop(*tm, st - kNodeHelper);
+        }
+        const unsigned was = __ballot_sync(0xffffffffu, st == kNodeOpen);
+        if (lane == 0) tm->pair[me].open -= __popc(was);
+        team_unlock(tm->pair[me]);
+      }
     }
+    if (w.err) break;
+    if (h >= 0 && lane == 0) atomicExch(&tm->slot[h].state, kSlotFree);   // the deltas have been read
     __syncwarp();
+  }
+  if (open && !team_close(*tm, me)) w.err |= kErrInternal;
+  if (w.err) {
+    w.cells  = cells0;
+    w.slides = slides0;
+    w.rows   = rows0;
+    return false;
   }
 
   if (lane == 0) {
@@ -424,7 +702,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
 template <bool GROUP>
 static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const ReadsDev &R, const TableDev &Tb,
                                                   const PairRec *pairs, const u32 *work, u32 nWork, u32 *workCounter,
-                                                  const int4 *nodes, const AlignOut &out) {
+                                                  const int4 *nodes, const AlignOut &out, Team *tm = nullptr, int me = 0) {
   const int lane = threadIdx.x & 31;
   // Inside a captured graph the list's length and start are known only on the device.
   if (out.nWorkDev) nWork = *out.nWorkDev;
@@ -433,11 +711,11 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
     for (int i = 0; i < kStCount; i++) ps.acc.v[i] = 0;
   __syncwarp();
 
-  while (true) {
-    u32 k = 0;
-    if (lane == 0) k = atomicAdd(workCounter, 1u);
-    k = __shfl_sync(0xffffffffu, k, 0);
-    if (k >= nWork) break;
+  // The list starts with the longest chains of extensions: the first pairs are dealt one
+  // to an SM, then a second one, ..., so that no SM gets several of them while the helpers
+  // of the others have nothing to do; the rest are taken as warps become free.
+  const u32 owners = GROUP ? gridDim.x : gridDim.x * kAlignWarps;
+  for (u32 k = GROUP ? blockIdx.x : (u32)me * gridDim.x + blockIdx.x; k < nWork;) {
     const u32 pi = work[k];
     const PairRec pr = pairs[pi];
     u32 nRec = 0;
@@ -445,7 +723,8 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
     const unsigned long long cellsBefore = w.cells;
     int extLimit = 0;   // 0: every match node may be extended (the reference's rule)
     if (out.tierLogit && out.tierLogit[pi] < out.tierThr) extLimit = out.tierBudget;
-    const bool ok = process_pair<GROUP>(w, ps, R, Tb, pr, nodes, out.rec + (u64)pi * 18, nRec, extLimit);
+    const bool ok = process_pair<GROUP>(w, ps, R, Tb, pr, nodes, out.rec + (u64)pi * 18, nRec, extLimit, tm,
+                                        me);
     if (lane == 0) {
       if (ok) {
         if (nRec == 0) ps.pc.v[kStCellsNoOlap] += w.cells - cellsBefore;
@@ -463,8 +742,14 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
         out.overflow[slot] = pi;
         atomicOr(out.err, w.err);
       }
+      k = owners + atomicAdd(workCounter, 1u);
     }
+    k = __shfl_sync(0xffffffffu, k, 0);
+  }
+  if (!GROUP) {
+    if (lane == 0) atomicSub(&tm->owners, 1);
     __syncwarp();
+    team_help(w, *tm, me);
   }
   // Cells and rows are warp-uniform; slides are counted per lane.
   const unsigned long long slidesWarp = warp_sum64(w.slides);
@@ -477,16 +762,26 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
   }
 }
 
-// One pair per warp, kAlignWarps warps per CTA.
-__global__ void __launch_bounds__(kAlignWarps * 32, OIC_ALIGN_MIN_BLOCKS) align_kernel(
+// One pair per warp, kAlignWarps warps per CTA, one CTA per SM.
+__global__ void __launch_bounds__(kAlignWarps * 32, 1) align_kernel(
     ReadsDev R, TableDev Tb, DevParams P, const int *eml, const PairRec *pairs, const u32 *work, u32 nWork,
     u32 *workCounter, const int4 *nodes, WarpScratch scBase, AlignCaps cap, AlignOut out) {
   __shared__ PairSmem pairSmem[kAlignWarps];
+  __shared__ Team     team;
   const int wib = threadIdx.x >> 5;
   const u64 gw  = (u64)blockIdx.x * kAlignWarps + wib;
   WarpDP w;
   warp_dp_init(w, warp_scratch(scBase, cap, gw), cap, wib * kWarpSmemInts, eml, P);
-  align_loop<false>(w, pairSmem[wib], R, Tb, pairs, work, nWork, workCounter, nodes, out);
+  if ((threadIdx.x & 31) == 0) {
+    team.pair[wib].lock   = 0;
+    team.pair[wib].open   = 0;
+    team.slot[wib].state  = kSlotFree;
+    team.slot[wib].owner  = -1;
+    team.slot[wib].deltaL = w.sc.deltaL;
+    if (wib == 0) team.owners = kAlignWarps;
+  }
+  __syncthreads();
+  align_loop<false>(w, pairSmem[wib], R, Tb, pairs, work, nWork, workCounter, nodes, out, &team, wib);
 }
 
 // One pair per CTA (the wide bins): warp 0 runs the pair logic, and every error-row
@@ -534,12 +829,6 @@ __global__ void __launch_bounds__(512, 1) align_group_kernel(ReadsDev R, TableDe
 constexpr int kSpecWarps = 8;
 enum { kSpecExtend = 1, kSpecExit = 2 };
 
-struct SpecRes {
-  int sLo, sHi, tLo, tHi, errors, kind, leftLen;
-  u32 err;
-  unsigned long long cells, slides, rows;
-};
-
 struct SpecShared {
   int         cmd;
   int         nCand;
@@ -547,30 +836,14 @@ struct SpecShared {
   SeqView     S, T;
   int         sLen, tLen;
   const int4 *nodes;
-  SpecRes     res[kSpecWarps];
+  ExtRes      res[kSpecWarps];
 };
 
 // Warp `wib` extends node cand[wib] of the posted pair into res[wib]; its deltas stay
 // in its scratch (sc.deltaL) until the next round.
 static __device__ __forceinline__ void spec_work(WarpDP &w, SpecShared &ss, int wib) {
-  const int lane = threadIdx.x & 31;
   if (wib >= ss.nCand) return;
-  const int4 lm = ss.nodes[ss.cand[wib]];
-  const unsigned long long c0 = w.cells, r0 = w.rows, s0 = w.slides;
-  w.err = 0;
-  int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
-  const int kind = warp_extend<false>(w, !w.P.partial, ss.S, ss.sLen, ss.T, ss.tLen, lm.z, lm.x, lm.y, sLo, sHi, tLo, tHi, errors);
-  const unsigned long long sl = warp_sum64(w.slides - s0);
-  if (lane == 0) {
-    SpecRes &r = ss.res[wib];
-    r.sLo = sLo; r.sHi = sHi; r.tLo = tLo; r.tHi = tHi; r.errors = errors; r.kind = kind;
-    r.leftLen = w.leftLen;
-    r.err     = w.err;
-    r.cells   = w.cells - c0;
-    r.rows    = w.rows - r0;
-    r.slides  = sl;
-  }
-  __syncwarp();
+  extend_node(w, ss.S, ss.sLen, ss.T, ss.tLen, ss.nodes[ss.cand[wib]], ss.res[wib]);
 }
 
 // Process_Matches for one pair on warp 0 of a speculative CTA (same rules and outputs as
@@ -702,7 +975,7 @@ __device__ bool process_pair_spec(WarpDP &w, PairSmem &ps, SpecShared &ss, const
     for (int j = 0; j < nC; j++) {
       const int li = ss.cand[j];
       if (alive[li] != 2) continue;            // removed by an earlier extension of the round
-      const SpecRes &r = ss.res[j];
+      const ExtRes &r = ss.res[j];
       if (r.err) {
         w.err |= r.err;
         failed = true;
@@ -782,7 +1055,7 @@ __device__ bool process_pair_spec(WarpDP &w, PairSmem &ps, SpecShared &ss, const
 // their pair logic; all kSpecWarps warps run the extensions of each round.  Warp j's
 // scratch is scBase's warp blockIdx.x * kSpecWarps + j; the pair's alive flags are in
 // the nodeCap * kSpecWarps bytes that start at warp 0's.
-__global__ void __launch_bounds__(kSpecWarps * 32, OIC_ALIGN_MIN_BLOCKS) align_spec_kernel(
+__global__ void __launch_bounds__(kSpecWarps * 32, 3) align_spec_kernel(
     ReadsDev R, TableDev Tb, DevParams P, const int *eml, const PairRec *pairs, const u32 *work, u32 nWork,
     u32 *workCounter, const int4 *nodes, WarpScratch scBase, AlignCaps cap, AlignOut out) {
   __shared__ PairSmem    ps;
@@ -929,7 +1202,8 @@ __global__ void compact_records_kernel(const u32 *rec, const u32 *cnt, const u32
 
 int align_warps_per_block() { return kAlignWarps; }
 
-static constexpr size_t kAlignSmem = (size_t)kAlignWarps * kWarpSmemInts * sizeof(int);
+static constexpr size_t kAlignSmem  = (size_t)kAlignWarps * kWarpSmemInts * sizeof(int);
+static constexpr size_t kExtendSmem = (size_t)kExtendWarps * kWarpSmemInts * sizeof(int);
 
 void launch_align(ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs, const u32 *work,
                   u32 nWork, u32 *workCounter, const int4 *nodes, WarpScratch sc, AlignCaps cap, int nWarps,
@@ -971,10 +1245,10 @@ void launch_extend_batch(ReadsDev R, DevParams P, const int *eml, const ExtendPr
                          WarpScratch sc, AlignCaps cap, int nWarps, int *out, int *kind, int *deltaLen, u32 *status,
                          unsigned long long *stats, cudaStream_t st) {
   if (n == 0) return;
-  const int    blocks = (nWarps + kAlignWarps - 1) / kAlignWarps;
-  auto k = extend_batch_kernel<kAlignWarps>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmem);
-  k<<<blocks, kAlignWarps * 32, kAlignSmem, st>>>(R, P, eml, probs, n, sc, cap, out, kind, deltaLen, status, stats);
+  const int blocks = (nWarps + kExtendWarps - 1) / kExtendWarps;
+  auto k = extend_batch_kernel<kExtendWarps>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExtendSmem);
+  k<<<blocks, kExtendWarps * 32, kExtendSmem, st>>>(R, P, eml, probs, n, sc, cap, out, kind, deltaLen, status, stats);
   g_launches++;
 }
 

@@ -1,13 +1,13 @@
 """The one-warp DP where it can go wrong, against the oracle: slides that end around the 32-
 and 1024-base steps, bands around the 32- and 64-diagonal chunks and past the shared-memory
-rows, reads with N, both directions."""
+rows, reads with N, both directions; and a pair whose match nodes keep helper warps busy."""
 import ctypes
 
 import numpy as np
 import pytest
 
 import canu_gb300 as oic
-from test_gpu_edges import mutate, rand_seq
+from test_gpu_edges import mutate, rand_seq, run_both
 from test_gpu_extend import port_aligner
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +78,15 @@ def test_row_loop_edges_match_oracle(name, erate, partial, built, oracle):
                                  ctypes.byref(n), None, None)
         assert k == kind[i] and (o == out[i]).all() and n.value == dl[i], (i, k, o, n.value, kind[i], out[i], dl[i])
     plib.oic_port_aligner_free(al)
+
+
+@pytest.mark.parametrize("extra", [[], ["-m"], ["-partial"]])
+def test_few_pairs_with_many_nodes(extra, built, oracle, tmp_path):
+    """Three reads, hundreds of match nodes a pair: every other warp of the owners' CTAs
+    helps, and the records and counts are those of one extension after another."""
+    r = np.random.default_rng(12)
+    g = rand_seq(r, 16000)
+    seqs = [mutate(r, g, 0.015), mutate(r, g[2000:], 0.015), mutate(r, g[:13000], 0.015)]
+    rec = run_both(built, oracle, tmp_path, seqs, ["-t", "2", "-k", "22", "--hashbits", "16", "--maxerate", "0.06",
+                                                   "--minlength", "500"] + extra)
+    assert len(rec) >= 3
