@@ -579,6 +579,103 @@ static __device__ __noinline__ void warp_rows(WarpDP &w, RowsOut &o, int step, c
   __syncwarp();
 }
 
+// ---------------------------------------------------------------------------------
+// True when no alignment of S and T with at most E errors runs from the start of S or T to
+// the end of S or T and, on the way, through a point on a diagonal (T offset - S offset) of
+// [dlo, dhi] that it reaches within those errors: then no match node on those diagonals
+// whose error limit is at most E extends to both ends.  (False says nothing.)
+//
+// One wavefront over all of them: row e holds, for each diagonal, the furthest S position
+// that e errors reach from any start on the boundary.  Every alignment of the statement is
+// followed: with e errors used it is at most E - e diagonals beside [dlo, dhi] if the point
+// is still ahead, and at most e if it lies behind, so row e needs only the diagonals within
+// max(E - e, e).  Nothing else is pruned, so reaching an end row is the only way out.  Cells
+// that no alignment has reached hold a large negative value.
+//
+// The row is updated in place in the warp's row buffers (nDiag <= kProofDiags), 64 diagonals
+// per step: a step's loads, the old value to its left among them, come before its stores.
+constexpr int kProofDiags = 2 * kRowStride - 4;
+static __device__ __noinline__ bool no_path_within(WarpDP &w, const SeqView &Sref, int sLen, const SeqView &Tref,
+                                                   int tLen, int dlo, int dhi, int E) {
+  const SeqView S = Sref, T = Tref;
+  const int lane  = threadIdx.x & 31;
+  constexpr int kFar = -(1 << 28);
+  const int lo = max(dlo - E, 1 - sLen), hi = min(dhi + E, tLen - 1);
+  int *const v = smemRows + w.smOff + 1 - lo;   // v[d], d in [lo - 1, hi + 1]
+  for (int d = lo - 1 + lane; d <= hi + 1; d += 32) v[d] = kFar;
+  __syncwarp();
+  u32 cells = 0;
+  bool end  = false;
+  int  e    = 0;
+  for (; e <= E && !end; e++) {
+    const int W  = max(E - e, e);
+    const int dL = max(lo, dlo - W), dR = min(hi, dhi + W);
+    int left = v[dL - 1];                       // old value left of the step
+#pragma unroll 1
+    for (int c = dL; c <= dR; c += 64) {
+      const int  da = min(c + lane, dR), db = min(c + 32 + lane, dR);
+      const bool ina = c + lane <= dR, inb = c + 32 + lane <= dR;
+      const int  a0 = v[da], a1 = v[da + 1], b0 = v[db], b1 = v[db + 1];
+      int am = __shfl_up_sync(0xffffffffu, a0, 1), bm = __shfl_up_sync(0xffffffffu, b0, 1);
+      const int a31 = __shfl_sync(0xffffffffu, a0, 31);
+      if (lane == 0) {
+        am = left;
+        bm = a31;
+      }
+      left = __shfl_sync(0xffffffffu, b0, 31);
+      int ra = e ? max(max(a0, a1) + 1, am) : max(0, -da);
+      int rb = e ? max(max(b0, b1) + 1, bm) : max(0, -db);
+      const bool oka = ina && ra >= 0, okb = inb && rb >= 0;
+      const int  ka = min(sLen - ra, tLen - da - ra), kb = min(sLen - rb, tLen - db - rb);
+      int sa = 0, sb = 0;
+      if (oka) sa = __clz((int)mismatch32<+1>(S, ra, T, ra + da));
+      if (okb) sb = __clz((int)mismatch32<+1>(S, rb, T, rb + db));
+      unsigned moreA = __ballot_sync(0xffffffffu, oka && sa == 32 && ka > 32);
+      unsigned moreB = __ballot_sync(0xffffffffu, okb && sb == 32 && kb > 32);
+      while (moreA | moreB) {                   // a long slide, 1024 bases per step (as in row_loop)
+        const bool second = moreA == 0;
+        const unsigned m = second ? moreB : moreA;
+        const int  q  = __ffs((int)m) - 1;
+        const int  r0 = __shfl_sync(0xffffffffu, second ? rb : ra, q);
+        const int  rq = __shfl_sync(0xffffffffu, second ? kb : ka, q);
+        const int  dq = c + q + (second ? 32 : 0);
+        if (second) moreB = m & (m - 1);
+        else moreA = m & (m - 1);
+        for (int run = 32;; run += 1024) {
+          const int at = run + 32 * lane;
+          int len = 0;
+          if (at < rq) len = __clz((int)mismatch32<+1>(S, r0 + at, T, r0 + at + dq));
+          const unsigned stop = __ballot_sync(0xffffffffu, len < 32);
+          if (stop) {
+            const int f   = __ffs((int)stop) - 1;
+            const int all = run + 32 * f + __shfl_sync(0xffffffffu, len, f);
+            if (lane == q) {
+              if (second) sb = all;
+              else sa = all;
+            }
+            break;
+          }
+        }
+      }
+      __syncwarp();
+      if (ina) v[da] = oka ? ra + min(sa, ka) : kFar;
+      if (inb) v[db] = okb ? rb + min(sb, kb) : kFar;
+      end |= __any_sync(0xffffffffu, (oka && sa >= ka) || (okb && sb >= kb));
+    }
+    cells += (u32)(dR - dL + 1);
+    __syncwarp();
+    // The cells beside the row are not part of it (they hold row e - 1's edge cells).
+    if (lane == 0) {
+      v[dL - 1] = kFar;
+      v[dR + 1] = kFar;
+    }
+    __syncwarp();
+  }
+  w.cells += cells;
+  w.rows += (u32)e;
+  return !end;
+}
+
 // The row loop by every thread of the CTA (nThr threads, tid = threadIdx.x).  Thread t
 // takes U consecutive diagonals per pass, d0 = Lc + U*t + U*nThr*k, so the U+2
 // neighbour values of row e-1 are read once for U cells and U slides are in flight.

@@ -62,8 +62,10 @@ typedef struct oic_stats {
   uint64_t kmerHitsWithoutOlap, kmerHitsWithOlap, kmerHitsSkipped, multiOverlap;
   uint64_t totalOverlaps, containedOverlaps, dovetailOverlaps;
   uint64_t badShortWindow, badLongWindow;
-  uint64_t dpCells, slideBases, extensions, seeds, candidatePairs, nodes, dpRows;   /* work done: outside
-                                                      -partial, an extension whose right side fails has no left */
+  uint64_t dpCells, slideBases, extensions, seeds, candidatePairs, nodes, dpRows;   /* work done, which may be
+                                                      less than the reference's: outside -partial, an extension
+                                                      whose right side fails has no left side, and match nodes
+                                                      shown to have no overlap together are not extended */
   uint32_t nHashBlocks, reserved;
   double   msHash, msSeed, msAlign, msTotal;       /* device time (CUDA events) of oic_run work */
   double   msReads;                                /* device time of the last oic_set_reads */

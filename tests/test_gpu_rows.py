@@ -90,3 +90,37 @@ def test_few_pairs_with_many_nodes(extra, built, oracle, tmp_path):
     rec = run_both(built, oracle, tmp_path, seqs, ["-t", "2", "-k", "22", "--hashbits", "16", "--maxerate", "0.06",
                                                    "--minlength", "500"] + extra)
     assert len(rec) >= 3
+
+
+@pytest.mark.parametrize("err,erate,with_n", [(0.0055, 0.01, False), (0.0055, 0.01, True), (0.011, 0.02, False),
+                                              (0.024, 0.045, False), (0.004, 0.06, False)])
+def test_hopeless_groups_keep_records(err, erate, with_n, built):
+    """Read pairs just above and below the error limit, and pairs that share a repeat only:
+    the one-warp DP, which drops groups of match nodes it shows to have no overlap, against
+    the CTA DP, which extends each of them."""
+    r = np.random.default_rng(13)
+    rep = rand_seq(r, 3000)
+    g = rand_seq(r, 9000) + rep + rand_seq(r, 12000) + mutate(r, rep, 0.01) + rand_seq(r, 9000) + mutate(r, rep, 0.02)
+    seqs = []
+    for _ in range(45):
+        n = int(r.integers(2500, 9000))
+        p = int(r.integers(0, len(g) - n))
+        s = mutate(r, g[p:p + n], err)
+        if with_n:
+            s = "".join("N" if r.random() < 0.0005 else c for c in s)
+        seqs.append((s if r.random() < 0.5 else s[::-1].translate(str.maketrans("ACGT", "TGCA"))).encode())
+    off = np.cumsum([0] + [len(x) for x in seqs])
+    got = []
+    for wide in (0, 1):
+        with oic.Overlapper(oic.default_params(kmerLen=K, hashBits=18, maxErate=erate, minOlapLen=500)) as ov:
+            ov.set_reads(np.ones(len(seqs)), [len(x) for x in seqs], off[:-1], np.frombuffer(b"".join(seqs), np.uint8))
+            ov.set_tuning(forceWide=wide)
+            ov.run()
+            got.append((oic.sort_records(ov.overlaps()), ov.stats()))
+    (a, sa), (b, sb) = got
+    assert a.shape == b.shape and (a == b).all()
+    for k in ("kmerHitsWithoutOlap", "kmerHitsWithOlap", "kmerHitsSkipped", "multiOverlap", "totalOverlaps",
+              "containedOverlaps", "dovetailOverlaps", "seeds", "candidatePairs", "nodes"):
+        assert sa[k] == sb[k], k
+    if erate <= 0.02:
+        assert sa["extensions"] < sb["extensions"]   # groups were dropped
