@@ -14,6 +14,9 @@
 
 namespace oic {
 
+// The DP's rows, in dynamic shared memory (each warp its slice from WarpDP::smOff on).
+extern __shared__ __align__(16) int smemRows[];
+
 // Per-warp global scratch.
 struct WarpScratch {
   int  *arena;       // kept DP rows, band-compacted
@@ -62,14 +65,13 @@ static __device__ __forceinline__ WarpScratch warp_scratch(const WarpScratch &ba
 }
 
 // Row-0 exact slide shared by the warp: each lane tests one 32-base window per step.
-template <int STEP>
 __device__ __forceinline__ int warp_slide0(const SeqView &A, int a0, const SeqView &T, int t0, int m,
                                            unsigned long long &slides) {
   const int lane = threadIdx.x & 31;
   int       run  = m;
   for (int base = 0; base < m; base += 32 * 32) {
     const int off = base + lane * 32;
-    const int r   = off < m ? __clz((int)mismatch32<STEP>(A, a0 + STEP * off, T, t0 + STEP * off)) : 32;
+    const int r   = off < m ? match_run32(A, a0 + off, T, t0 + off) : 32;
     const unsigned stop = __ballot_sync(0xffffffffu, r < 32);
     if (stop) {
       const int f = __ffs((int)stop) - 1;
@@ -89,14 +91,15 @@ __device__ __forceinline__ int warp_slide0(const SeqView &A, int a0, const SeqVi
 //
 // A step needs the row above at d - 1, d and d + 1 and moves d by at most one, so the
 // values that the next kTraceRows rows can need lie within a window of 32 diagonals: the
-// warp loads those windows together (one coalesced load per row, all in flight) and walks
-// them with shuffles.  One lane walking the arena by itself waited for an L2 round trip
-// per row.
-constexpr int kTraceRows = 8;
+// warp loads those windows into its (now unused) shared-memory rows together, one coalesced
+// load per row, all in flight, and walks them there.  One lane walking the arena by itself
+// waited for an L2 round trip per row.
+constexpr int kTraceRows = 12;
 static __device__ __noinline__ int trace_rows(const WarpDP &w, int e, int d, int last, int *out, int &nOut) {
   static_assert(kTraceRows + 1 <= 15, "the window holds d - kTraceRows - 1 .. d + kTraceRows + 1");
   const int4 *const rowHdr = w.sc.rowHdr;
   const int *const  arena  = w.sc.arena;
+  int *const        tile   = smemRows + w.smOff;
   const int         lane   = threadIdx.x & 31;
   const int4        none   = make_int4(0, 1, 0, 0);   // an empty band
   int  n = 0;
@@ -107,30 +110,29 @@ static __device__ __noinline__ int trace_rows(const WarpDP &w, int e, int d, int
     const int  kn = k - kTraceRows - 1 - lane;
     hNext         = lane < kTraceRows && kn >= 0 ? rowHdr[kn] : none;
     const int d0  = d - 16, dd = d0 + lane;
-    int v[kTraceRows];
-#pragma unroll
+#pragma unroll 6
     for (int j = 0; j < kTraceRows; j++) {
       const int off = __shfl_sync(0xffffffffu, h.x, j), L = __shfl_sync(0xffffffffu, h.y, j),
                 R   = __shfl_sync(0xffffffffu, h.z, j);
-      v[j] = (dd >= L && dd <= R) ? arena[off + dd - L] : -2;
+      tile[32 * j + lane] = (dd >= L && dd <= R) ? arena[off + dd - L] : -2;
     }
-#pragma unroll
-    for (int j = 0; j < kTraceRows; j++) {
-      if (j < k) {
-        const int g0 = __shfl_sync(0xffffffffu, v[j], d - d0);
-        const int gm = __shfl_sync(0xffffffffu, v[j], d - 1 - d0);
-        const int gp = __shfl_sync(0xffffffffu, v[j], d + 1 - d0);
-        int from = 0, mx = 1 + g0;
-        if (gm > mx) { from = -1; mx = gm; }
-        if (1 + gp > mx) { from = 1; mx = 1 + gp; }
-        if (from) {
-          if (lane == 0) out[n] = from < 0 ? mx - last - 1 : last - (mx - 1);
-          last = from < 0 ? gm : gp;
-          d += from;
-          n++;
-        }
+    __syncwarp();
+    const int rows = min(k, kTraceRows);
+#pragma unroll 1
+    for (int j = 0; j < rows; j++) {
+      const int *g = tile + 32 * j + (d - d0);
+      const int g0 = g[0], gm = g[-1], gp = g[1];
+      int from = 0, mx = 1 + g0;
+      if (gm > mx) { from = -1; mx = gm; }
+      if (1 + gp > mx) { from = 1; mx = 1 + gp; }
+      if (from) {
+        if (lane == 0) out[n] = from < 0 ? mx - last - 1 : last - (mx - 1);
+        last = from < 0 ? gm : gp;
+        d += from;
+        n++;
       }
     }
+    __syncwarp();
   }
   nOut = n;
   return last;
@@ -268,7 +270,7 @@ struct RowsOut {
 struct GroupJob {
   SeqView A, T;
   int     a0, t0;
-  int     m, n, errorLimit, step, u;
+  int     m, n, errorLimit, u;
   int    *rowA, *rowB;       // row buffers (rowA holds row 0)
 };
 struct GroupShared {
@@ -296,7 +298,7 @@ struct RowJob {
   int       *arena;
   int4      *rowHdr;
   const int *eml;
-  int        a0, t0, step;
+  int        a0, t0;
   int        arenaCap, bufW;
   int        e, L, R, off, base;   // the row to compute; kept band, place and buffer origin of the row before it
   int        dEnd, Rc, rowEnd, ppEnd;
@@ -307,17 +309,13 @@ constexpr int kJobInts      = (sizeof(RowJob) + 15) / 16 * 4;
 constexpr int kWarpSmemInts = 2 * kRowStride + kJobInts;
 static_assert(2 * kRowStride % 4 == 0, "RowJob starts on 16 bytes");
 
-extern __shared__ __align__(16) int smemRows[];
-
-// Mismatch mask of 32 bases of A from base ga and T from base gt on in read order (the
-// caller passes the window's low ends); bit 31 is the first base in the direction of the
-// extension.  fwd: forward extension.
+// match_run32 of the job's sequences, their planes in registers.
 template <bool HASN>
-__device__ __forceinline__ int match_len(const RowJob &job, const uint2 *Ap, int ga, const uint2 *Tp, int gt, bool fwd) {
+__device__ __forceinline__ int match_len(const RowJob &job, const uint2 *Ap, int ga, const uint2 *Tp, int gt) {
   const uint2 x = load_planes(Ap, ga), y = load_planes(Tp, gt);
   u32 m = (x.x ^ y.x) | (x.y ^ y.y);
   if (HASN) m = drop_n(m, job.A.nm, ga, job.T.nm, gt);
-  return __clz((int)(fwd ? __brev(m) : m));
+  return __clz((int)m);
 }
 
 // Rows e, e + 1, ... by one warp, from the kept band [L, R] of row e - 1 in the buffer
@@ -328,16 +326,23 @@ __device__ __forceinline__ int match_len(const RowJob &job, const uint2 *Ap, int
 // kept band set to -2 as the reference does (forward.C:150-153), so the neighbour reads
 // need no bounds tests.
 //
-// What bounds it: instruction issue (64 % of the slots) and the latency of a row.  A row of
-// the 0.5 % reads is 33 diagonals and issues 350 warp instructions, of which the leading
-// diagonal's long slide is a third; with the interleaved 2-bit words, a window of 32 bases
-// cost 60 instructions, the row 520, and the longest slide ran alone, 32 bases per step
-// (150 Mbp of those reads: DP 648 -> 426 ms; 20 Mbp of 2 % reads 346 -> 321 ms).
-// Both directions run the same instructions, and 64 diagonals at a time share one copy of
-// the code for long slides: with a copy per direction and chunk the loop missed the
-// instruction cache (6.9 stall cycles per issue; DP 601 ms).  Keeping each diagonal's
-// mismatch mask from row to row does not pay: inside the band every diagonal moves as fast
-// as the alignment does, so a mask of 32 bases is used up in a row or two (519 ms).
+// What bounds it: instruction issue (63 % of the slots) and the latency of a row.  A row of
+// the 2 % reads is 104 diagonals and issues 487 warp instructions, a fifth of them moves of
+// the address descriptors that every load of a called function needs.  Measured on the way
+// here (DP of 150 Mbp of 0.5 % reads; 20 Mbp of 2 % reads; 4 Mbp of noisy reads):
+//   interleaved 2-bit words, the longest slide alone, 32 bases per step, on teams' SMs
+//     shared by three CTAs: 648 / 346 / 523 ms;
+//   bit planes, long slides by the warp: 426 / 321 / 504 ms; as a team (oic_pairs.cu) and
+//     with hopeless groups settled together: 120 / 189 / 127 ms;
+//   lanes past the band repeating its last diagonal instead of being masked, one vote for
+//     everything rare, the band's edges by two warp reductions per row: 126 / 159 / 54 ms;
+//   both directions on forward windows (to the left on the reverse complements), planes
+//     with the first base topmost: 107 / 149 / 49 ms.
+// A copy of the loop per direction and chunk missed the instruction cache (601 / 377 / 754
+// ms before teams).  32 diagonals per step issue as many instructions and wait longer (111 /
+// 169 / 56 ms).  Keeping each diagonal's mismatch mask from row to row does not pay: inside
+// the band every diagonal moves as fast as the alignment does, so a mask of 32 bases is
+// used up in a row or two.
 enum { kRowsWiden = 3 };
 template <bool HASN, bool WIDE>
 static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *rowsG, const int m, const int n,
@@ -345,13 +350,16 @@ static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *r
   const int lane = threadIdx.x & 31;
   int *prev = WIDE ? rowsG : smemRows + smOff, *cur = WIDE ? rowsG + job.bufW : prev + kRowStride;
   const uint2 *const Ap = job.A.p, *const Tp = job.T.p;
-  int *const arena = job.arena;
-  const int  sgn = job.step;
-  const bool fwd = sgn > 0;
-  const int  a0 = job.a0 - (fwd ? 0 : 31), t0 = job.t0 - (fwd ? 0 : 31);
+  int4 *const rowHdr = job.rowHdr;
+  const int *const eml = job.eml;
+  const int  a0 = job.a0, t0 = job.t0;
   const int  bufW = job.bufW, arenaCap = job.arenaCap;
+  int *const arena = job.arena;
+  __builtin_assume(__isGlobal(rowHdr));
+  __builtin_assume(__isGlobal(arena));
+  __builtin_assume(__isGlobal(eml));
   int e = job.e, L = job.L, R = job.R, off = job.off, base = job.base;
-  int lim = e <= errorLimit ? job.eml[e] : 0;
+  int lim = e <= errorLimit ? eml[e] : 0;
   u32 cells = 0, slides = 0;
   int status = kRowsDone;
   for (; e <= errorLimit; e++) {
@@ -359,103 +367,93 @@ static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *r
     const int Lc = max(L - 1, -e), Rc = min(R + 1, e);
     const int width = Rc - Lc + 1;
     if (width + 4 > bufW) { status = kRowsWiden; break; }
-    const int limNext = e < errorLimit ? job.eml[e + 1] : 0;
+    const int limNext = e < errorLimit ? eml[e + 1] : 0;
     const int *pv = prev + (2 - base);        // pv[d] = row e-1 at diagonal d
     int       *cv = cur + (2 - Lc);           // cv[d] = row e at diagonal d
     int       *av = arena + (off - L);        // av[d]: row e-1's place in the arena
-    int L2 = INT_MAX, R2 = INT_MIN, prevMax = -1, dEnd = INT_MAX;
+    int myL = INT_MAX, myR = INT_MIN, prevMax = -1, dEnd = INT_MAX;
 #pragma unroll 1
     for (int c = Lc; c <= Rc; c += 64) {
-      const bool two = c + 32 <= Rc;
-      const int  da = min(c + lane, Rc), db = min(c + 32 + lane, Rc);
-      const bool ina = c + lane <= Rc, inb = c + 32 + lane <= Rc;
-      int pa = pv[da + 1], pb = 0, ra, rb = 0, ka, kb = 0;   // row e-1 at d + 1; value; room to the nearer end
-      {
-        const int p0 = pv[da];
-        ra = max(max(p0, pa) + 1, pv[da - 1]);
-        if (ina && da >= L && da <= R) {      // keep row e-1 for the traceback
-          av[da]  = p0;
-          prevMax = max(prevMax, p0);
-        }
-        ka = min(m - ra, n - da - ra);        // >= 0: no cell of row e-1 is at an end
-      }
-      if (two) {
-        const int p0 = pv[db];
+      // Lanes past the band repeat its last diagonal: what they compute and store is what
+      // that diagonal's lane computes and stores.
+      const int da = min(c + lane, Rc);
+      const int pa = pv[da + 1], qa = pv[da];
+      int ra = max(max(qa, pa) + 1, pv[da - 1]);
+      if (da >= L && da <= R) av[da] = qa;    // keep row e-1 for the traceback
+      prevMax = max(prevMax, qa);
+      const int za = min(m, n - da);          // where the nearer end is: ra <= za, as no cell of row e-1 is at one
+      int sa = ra + match_len<HASN>(job, Ap, a0 + ra, Tp, t0 + da + ra);
+      int db = 0, pb = 0, rb = -(1 << 28), zb = INT_MAX, sb = rb;
+      if (c + 32 <= Rc) {
+        db = min(c + 32 + lane, Rc);
+        const int qb = pv[db];
         pb = pv[db + 1];
-        rb = max(max(p0, pb) + 1, pv[db - 1]);
-        if (inb && db <= R) {                 // db > Lc + 31 >= L
-          av[db]  = p0;
-          prevMax = max(prevMax, p0);
-        }
-        kb = min(m - rb, n - db - rb);
+        rb = max(max(qb, pb) + 1, pv[db - 1]);
+        if (db <= R) av[db] = qb;             // db > Lc + 31 >= L
+        prevMax = max(prevMax, qb);
+        zb = min(m, n - db);
+        sb = rb + match_len<HASN>(job, Ap, a0 + rb, Tp, t0 + db + rb);
       }
-      int sa = match_len<HASN>(job, Ap, a0 + sgn * ra, Tp, t0 + sgn * (ra + da), fwd), sb = 0;
-      if (two) sb = match_len<HASN>(job, Ap, a0 + sgn * rb, Tp, t0 + sgn * (rb + db), fwd);
-      unsigned moreA = __ballot_sync(0xffffffffu, ina && sa == 32 && ka > 32);
-      unsigned moreB = __ballot_sync(0xffffffffu, inb && sb == 32 && kb > 32);
-      while (moreA | moreB) {
-        // One lane's slide goes on: the warp looks at 32 windows of 32 bases per step.
-        const bool second = moreA == 0;
-        const unsigned w = second ? moreB : moreA;
-        const int  q  = __ffs((int)w) - 1;
-        const int  r0 = __shfl_sync(0xffffffffu, second ? rb : ra, q);
-        const int  rq = __shfl_sync(0xffffffffu, second ? kb : ka, q);
-        const int  dq = c + q + (second ? 32 : 0);
-        if (second) moreB = w & (w - 1);
-        else moreA = w & (w - 1);
-        for (int run = 32;; run += 1024) {
-          const int at = run + 32 * lane;
-          int len = 0;
-          if (at < rq) len = match_len<HASN>(job, Ap, a0 + sgn * (r0 + at), Tp, t0 + sgn * (r0 + at + dq), fwd);
-          const unsigned stop = __ballot_sync(0xffffffffu, len < 32);
-          if (stop) {
-            const int f   = __ffs((int)stop) - 1;
-            const int all = run + 32 * f + __shfl_sync(0xffffffffu, len, f);
-            if (lane == q) {
-              if (second) sb = all;
-              else sa = all;
+      if (__any_sync(0xffffffffu, sa >= min(za, ra + 32) || sb >= min(zb, rb + 32))) {
+        // A slide through its whole window, or up to an end.
+        unsigned moreA = __ballot_sync(0xffffffffu, c + lane <= Rc && sa == ra + 32 && sa < za);
+        unsigned moreB = __ballot_sync(0xffffffffu, c + 32 + lane <= Rc && sb == rb + 32 && sb < zb);
+        while (moreA | moreB) {
+          // One lane's slide goes on: the warp looks at 32 windows of 32 bases per step.
+          const bool second = moreA == 0;
+          const unsigned w = second ? moreB : moreA;
+          const int  q  = __ffs((int)w) - 1;
+          const int  zq = __shfl_sync(0xffffffffu, second ? zb : za, q);
+          const int  dq = c + q + (second ? 32 : 0);
+          if (second) moreB = w & (w - 1);
+          else moreA = w & (w - 1);
+          for (int r = __shfl_sync(0xffffffffu, second ? sb : sa, q);; r += 1024) {
+            const int at = r + 32 * lane;
+            int len = 0;
+            if (at < zq) len = match_len<HASN>(job, Ap, a0 + at, Tp, t0 + dq + at);
+            const unsigned stop = __ballot_sync(0xffffffffu, len < 32);
+            if (stop) {
+              const int f  = __ffs((int)stop) - 1;
+              const int to = __shfl_sync(0xffffffffu, at + len, f);
+              if (dq == (second ? db : da)) {   // the lane, and those that repeat it
+                if (second) sb = to;
+                else sa = to;
+              }
+              break;
             }
-            break;
+          }
+        }
+        if (dEnd == INT_MAX) {
+          const unsigned endA = __ballot_sync(0xffffffffu, sa >= za), endB = __ballot_sync(0xffffffffu, sb >= zb);
+          if (endA | endB) {
+            const int f = __ffs((int)(endA ? endA : endB)) - 1;
+            dEnd = c + f + (endA ? 0 : 32);
+            if (lane == f) {
+              job.rowEnd = endA ? za : zb;
+              job.ppEnd  = endA ? pa : pb;
+            }
           }
         }
       }
-      sa = min(sa, ka);
-      ra += sa;
-      unsigned keepB = 0, endB = 0;
+      sa = min(sa, za);
+      sb = min(sb, zb);
+      cv[da] = sa;
+      if (c + 32 <= Rc) cv[db] = sb;
+      if (c + lane <= Rc) slides += (u32)(sa - ra);
+      if (c + 32 + lane <= Rc) slides += (u32)(sb - rb);
       // pruneAlign (prefixEditDistance.H:249-258): extra = max(d, 0) on both band edges
-      const unsigned keepA = __ballot_sync(0xffffffffu, ina && ra + max(da, 0) >= lim);
-      const unsigned endA  = __ballot_sync(0xffffffffu, ina && sa == ka);   // at the end of A or T
-      if (ina) {
-        cv[da] = ra;
-        slides += (u32)sa;
+      if (sa + max(da, 0) >= lim) {
+        myL = min(myL, da);
+        myR = da;
       }
-      if (two) {
-        sb = min(sb, kb);
-        rb += sb;
-        keepB = __ballot_sync(0xffffffffu, inb && rb + max(db, 0) >= lim);
-        endB  = __ballot_sync(0xffffffffu, inb && sb == kb);
-        if (inb) {
-          cv[db] = rb;
-          slides += (u32)sb;
-        }
-      }
-      if ((endA | endB) && dEnd == INT_MAX) {
-        const int f = __ffs((int)(endA ? endA : endB)) - 1;
-        dEnd = c + f + (endA ? 0 : 32);
-        if (lane == f) {
-          job.rowEnd = endA ? ra : rb;
-          job.ppEnd  = endA ? pa : pb;
-        }
-      }
-      const u64 keep = (u64)keepA | ((u64)keepB << 32);
-      if (keep) {
-        if (L2 == INT_MAX) L2 = c + __ffsll((long long)keep) - 1;
-        R2 = c + 63 - __clzll((long long)keep);
+      if (sb + max(db, 0) >= lim) {
+        myL = min(myL, db);
+        myR = db;
       }
     }
     // Row e-1's header, with its largest value (forward.C:284-289) for max_score_rows.
     prevMax = __reduce_max_sync(0xffffffffu, prevMax);
-    if (lane == 0) job.rowHdr[e - 1] = make_int4(off, L, R, prevMax);
+    if (lane == 0) rowHdr[e - 1] = make_int4(off, L, R, prevMax);
     if (dEnd != INT_MAX) {
       cells += (u32)(dEnd - Lc + 1);
       status = kRowsEnd;
@@ -467,6 +465,7 @@ static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *r
     }
     cells += (u32)width;
     // The kept band is [first, last] unpruned diagonal (forward.C:245-280).
+    const int L2 = __reduce_min_sync(0xffffffffu, myL), R2 = __reduce_max_sync(0xffffffffu, myR);
     if (L2 == INT_MAX) break;
     __syncwarp();
     if (lane < 4) cv[lane < 2 ? L2 - 2 + lane : R2 - 1 + lane] = -2;
@@ -492,7 +491,7 @@ static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *r
         prevMax            = max(prevMax, v);
       }
       prevMax = __reduce_max_sync(0xffffffffu, prevMax);
-      if (lane == 0) job.rowHdr[errorLimit] = make_int4(off, L, R, prevMax);
+      if (lane == 0) rowHdr[errorLimit] = make_int4(off, L, R, prevMax);
     }
   }
   __syncwarp();
@@ -511,8 +510,8 @@ static __device__ __noinline__ int row_loop(RowJob &job, const int smOff, int *r
 
 // The row loop by one warp: rows in shared memory, and in the warp's HBM rows from the row
 // on whose band has outgrown them.  r0: row 0's value.
-static __device__ __noinline__ void warp_rows(WarpDP &w, RowsOut &o, int step, const SeqView &A, int a0, int m,
-                                              const SeqView &T, int t0, int n, int errorLimit, int r0) {
+static __device__ __noinline__ void warp_rows(WarpDP &w, RowsOut &o, const SeqView &A, int a0, int m, const SeqView &T,
+                                              int t0, int n, int errorLimit, int r0) {
   const int  lane = threadIdx.x & 31;
   int *const bufA = smemRows + w.smOff, *const bufB = bufA + kRowStride;
   RowJob    &job  = *(RowJob *)(bufB + kRowStride);
@@ -528,7 +527,6 @@ static __device__ __noinline__ void warp_rows(WarpDP &w, RowsOut &o, int step, c
     job.eml      = w.eml;
     job.a0       = a0;
     job.t0       = t0;
-    job.step     = step;
     job.arenaCap = w.cap.arenaCap;
     job.bufW     = kRowW;
     job.e        = 1;
@@ -595,9 +593,9 @@ static __device__ __noinline__ void warp_rows(WarpDP &w, RowsOut &o, int step, c
 // The row is updated in place in the warp's row buffers (nDiag <= kProofDiags), 64 diagonals
 // per step: a step's loads, the old value to its left among them, come before its stores.
 constexpr int kProofDiags = 2 * kRowStride - 4;
-static __device__ __noinline__ bool no_path_within(WarpDP &w, const SeqView &Sref, int sLen, const SeqView &Tref,
+static __device__ __noinline__ bool no_path_within(WarpDP &w, const ReadView &Sref, int sLen, const ReadView &Tref,
                                                    int tLen, int dlo, int dhi, int E) {
-  const SeqView S = Sref, T = Tref;
+  const SeqView S = Sref.f, T = Tref.f;
   const int lane  = threadIdx.x & 31;
   constexpr int kFar = -(1 << 28);
   const int lo = max(dlo - E, 1 - sLen), hi = min(dhi + E, tLen - 1);
@@ -628,32 +626,20 @@ static __device__ __noinline__ bool no_path_within(WarpDP &w, const SeqView &Sre
       const bool oka = ina && ra >= 0, okb = inb && rb >= 0;
       const int  ka = min(sLen - ra, tLen - da - ra), kb = min(sLen - rb, tLen - db - rb);
       int sa = 0, sb = 0;
-      if (oka) sa = __clz((int)mismatch32<+1>(S, ra, T, ra + da));
-      if (okb) sb = __clz((int)mismatch32<+1>(S, rb, T, rb + db));
-      unsigned moreA = __ballot_sync(0xffffffffu, oka && sa == 32 && ka > 32);
-      unsigned moreB = __ballot_sync(0xffffffffu, okb && sb == 32 && kb > 32);
-      while (moreA | moreB) {                   // a long slide, 1024 bases per step (as in row_loop)
-        const bool second = moreA == 0;
-        const unsigned m = second ? moreB : moreA;
-        const int  q  = __ffs((int)m) - 1;
-        const int  r0 = __shfl_sync(0xffffffffu, second ? rb : ra, q);
-        const int  rq = __shfl_sync(0xffffffffu, second ? kb : ka, q);
-        const int  dq = c + q + (second ? 32 : 0);
-        if (second) moreB = m & (m - 1);
-        else moreA = m & (m - 1);
-        for (int run = 32;; run += 1024) {
-          const int at = run + 32 * lane;
-          int len = 0;
-          if (at < rq) len = __clz((int)mismatch32<+1>(S, r0 + at, T, r0 + at + dq));
-          const unsigned stop = __ballot_sync(0xffffffffu, len < 32);
-          if (stop) {
-            const int f   = __ffs((int)stop) - 1;
-            const int all = run + 32 * f + __shfl_sync(0xffffffffu, len, f);
-            if (lane == q) {
-              if (second) sb = all;
-              else sa = all;
-            }
-            break;
+      if (oka) sa = match_run32(S, ra, T, ra + da);
+      if (okb) sb = match_run32(S, rb, T, rb + db);
+      // Slides past a window go on 32 bases per step (the first half's, then the second's).
+      bool fa = oka && sa == 32 && ka > 32, fb = okb && sb == 32 && kb > 32;
+      while (__any_sync(0xffffffffu, fa || fb)) {
+        if (fa || fb) {
+          const int r   = fa ? ra + sa : rb + sb;
+          const int len = match_run32(S, r, T, r + (fa ? da : db));
+          if (fa) {
+            sa += len;
+            fa = len == 32 && sa < ka;
+          } else {
+            sb += len;
+            fb = len == 32 && sb < kb;
           }
         }
       }
@@ -681,7 +667,7 @@ static __device__ __noinline__ bool no_path_within(WarpDP &w, const SeqView &Sre
 // neighbour values of row e-1 are read once for U cells and U slides are in flight.
 // Every decision is made on CTA-reduced values, so all threads take the same path and
 // meet the same barriers.
-template <int STEP, int U>
+template <int U>
 static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpScratch &sc, const AlignCaps &cap,
                                                   const int *eml, int tid, int nThr, int (*red)[4],
                                                   unsigned long long &slides) {
@@ -730,7 +716,7 @@ static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpS
           if (q[k] > row) row = q[k];
           if (1 + q[k + 2] > row) row = 1 + q[k + 2];
           const int room = min(m - row, n - row - d);
-          if (room > 0) row += slide<STEP>(A, a0, T, t0, row, d, room, slides);
+          if (room > 0) row += slide(A, a0, T, t0, row, d, room, slides);
           cv[d] = row;
           if ((row == m || row + d == n) && d < myEnd) myEnd = d;
           if (!(row + max(d, 0) < lim)) {
@@ -801,18 +787,13 @@ static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpS
   return o;
 }
 
-// The job a GroupJob names, with its compile-time step and tile.
+// The job a GroupJob names, with its compile-time tile.
 static __device__ __forceinline__ RowsOut group_rows_any(const GroupJob &j, const WarpScratch &sc,
                                                          const AlignCaps &cap, const int *eml, int tid, int nThr,
                                                          int (*red)[4], unsigned long long &slides) {
-  if (j.step > 0) {
-    if (j.u == 4) return group_rows<+1, 4>(j, sc, cap, eml, tid, nThr, red, slides);
-    if (j.u == 2) return group_rows<+1, 2>(j, sc, cap, eml, tid, nThr, red, slides);
-    return group_rows<+1, 1>(j, sc, cap, eml, tid, nThr, red, slides);
-  }
-  if (j.u == 4) return group_rows<-1, 4>(j, sc, cap, eml, tid, nThr, red, slides);
-  if (j.u == 2) return group_rows<-1, 2>(j, sc, cap, eml, tid, nThr, red, slides);
-  return group_rows<-1, 1>(j, sc, cap, eml, tid, nThr, red, slides);
+  if (j.u == 4) return group_rows<4>(j, sc, cap, eml, tid, nThr, red, slides);
+  if (j.u == 2) return group_rows<2>(j, sc, cap, eml, tid, nThr, red, slides);
+  return group_rows<1>(j, sc, cap, eml, tid, nThr, red, slides);
 }
 
 // Worker warps of a group CTA: run the row loops warp 0 posts until it posts exit.
@@ -827,26 +808,26 @@ static __device__ __noinline__ void group_worker(GroupShared &gs, const WarpScra
   }
 }
 
-// forward() (prefixEditDistance-forward.C:94-314) for STEP = +1 and reverse()
-// (prefixEditDistance-reverse.C:114-330) for STEP = -1.  A[STEP*i] is base a0+STEP*i of
-// view A, T likewise.  The row loop runs on this warp, or on the whole CTA when w.gs is
+// forward() (prefixEditDistance-forward.C:94-314) for step = +1 and reverse()
+// (prefixEditDistance-reverse.C:114-330) for step = -1.  A[i] is base a0+i of view A,
+// T likewise (for step = -1 the reads' reverse complements).  The row loop runs on this warp, or on the whole CTA when w.gs is
 // set (warp 0 of a group CTA); the rest runs on this warp.  Returns the error count;
 // the outputs are warp-uniform.  On a capacity overflow sets w.err and returns 0.
 // endOnly: the caller uses the outputs only when the end is reached (toEnd); otherwise
 // they are not computed.
-template <int STEP, bool GROUP>
-static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, int a0, int m, const SeqView &T, int t0, int n,
+template <bool GROUP>
+static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const int step, const SeqView &A, int a0, int m, const SeqView &T, int t0, int n,
                               int errorLimit, bool endOnly, int &aEnd, int &tEnd, int &leftover, bool &toEnd) {
   const int lane = threadIdx.x & 31;
   const double BMV = w.P.branchMatchValue;
 
-  if (STEP > 0) w.rightLen = 0;
+  if (step > 0) w.rightLen = 0;
   else w.leftLen = 0;
 
-  const int r0 = warp_slide0<STEP>(A, a0, T, t0, m, w.slides);
+  const int r0 = warp_slide0(A, a0, T, t0, m, w.slides);
   if (r0 == m) {
-    aEnd = tEnd = STEP * m;
-    if (STEP < 0) leftover = m;
+    aEnd = tEnd = step * m;
+    if (step < 0) leftover = m;
     toEnd = true;
     return 0;
   }
@@ -865,7 +846,6 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
       j.m          = m;
       j.n          = n;
       j.errorLimit = errorLimit;
-      j.step       = STEP;
       j.u          = w.gU;
       j.rowA       = w.smA;
       j.rowB       = w.smB;
@@ -876,7 +856,7 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
     const GroupJob j = w.gs->job;
     o = group_rows_any(j, w.sc, w.cap, w.eml, lane, w.gThreads, w.gs->red, w.slides);
   } else {
-    warp_rows(w, o, STEP, A, a0, m, T, t0, n, errorLimit, r0);
+    warp_rows(w, o, A, a0, m, T, t0, n, errorLimit, r0);
   }
   w.cells += o.cells;
   w.rows += o.rows;
@@ -909,7 +889,7 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
     abort_ = __shfl_sync(0xffffffffu, abort_, 0);
     if (!abort_) {
       int d = o.dEnd;
-      if (STEP > 0) {
+      if (step > 0) {
         // Force the last error to be a mismatch (forward.C:215-221).
         if (row == m && 1 + o.ppEnd == row && d < o.Rc) d++;
         aEnd = row;
@@ -931,10 +911,10 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const SeqView &A, i
 
   // Branch point, errors exhausted, or every diagonal pruned (forward.C:197-212,
   // 306-313): the alignment ends at the Max_Score row.
-  aEnd = STEP * msLen;
-  tEnd = STEP * (msLen + msD);
+  aEnd = step * msLen;
+  tEnd = step * (msLen + msD);
   const int last = arena_get(w, msE, msD);
-  if (STEP > 0) set_right_delta(w, msE, msD, last);
+  if (step > 0) set_right_delta(w, msE, msD, last);
   else set_left_delta(w, msE, msD, last, leftover, tEnd, n);
   toEnd = false;
   return msE;
@@ -968,7 +948,7 @@ enum { kNone = 0, kLeftBranch = 1, kRightBranch = 2, kDovetail = 3 };
 // traced: pairs that share only a repeat fail on one side in nearly every extension, and
 // on repeat-rich low-error reads they are nine tenths of the cells.
 template <bool GROUP>
-static __device__ __noinline__ int warp_extend(WarpDP &w, bool dovetailOnly, const SeqView &S, int sLen, const SeqView &T, int tLen, int mStart,
+static __device__ __noinline__ int warp_extend(WarpDP &w, bool dovetailOnly, const ReadView &S, int sLen, const ReadView &T, int tLen, int mStart,
                            int mOffset, int mLen, int &sLo, int &sHi, int &tLo, int &tHi, int &errors) {
   const int lane = threadIdx.x & 31;
   int  rightErrors = 0, leftErrors = 0, leftover = 0;
@@ -986,12 +966,12 @@ static __device__ __noinline__ int warp_extend(WarpDP &w, bool dovetailOnly, con
     sHi = tHi = 0;
     rToEnd    = true;
   } else if (sRightLen <= tRightLen) {
-    rightErrors = warp_prefix_dp<+1, GROUP>(w, S, sRightBegin, sRightLen, T, tRightBegin, tRightLen, errorLimit,
+    rightErrors = warp_prefix_dp<GROUP>(w, +1, S.f, sRightBegin, sRightLen, T.f, tRightBegin, tRightLen, errorLimit,
                                      dovetailOnly, sHi, tHi, leftover, rToEnd);
     if (w.err) return kNone;
     for (int i = lane; i < w.rightLen; i += 32) w.sc.deltaR[i] = -w.sc.deltaR[i];
   } else {
-    rightErrors = warp_prefix_dp<+1, GROUP>(w, T, tRightBegin, tRightLen, S, sRightBegin, sRightLen, errorLimit,
+    rightErrors = warp_prefix_dp<GROUP>(w, +1, T.f, tRightBegin, tRightLen, S.f, sRightBegin, sRightLen, errorLimit,
                                      dovetailOnly, tHi, sHi, leftover, rToEnd);
     if (w.err) return kNone;
   }
@@ -1005,11 +985,11 @@ static __device__ __noinline__ int warp_extend(WarpDP &w, bool dovetailOnly, con
     sLo = tLo = 0;
     lToEnd    = true;
   } else if (sRightBegin <= tRightBegin) {
-    leftErrors = warp_prefix_dp<-1, GROUP>(w, S, sLeftBegin, sLeftBegin + 1, T, tLeftBegin, tLeftBegin + 1,
+    leftErrors = warp_prefix_dp<GROUP>(w, -1, S.c, sLen - mStart, sLeftBegin + 1, T.c, tLen - mOffset, tLeftBegin + 1,
                                     errorLimit - rightErrors, dovetailOnly, sLo, tLo, leftover, lToEnd);
     if (w.err) return kNone;
   } else {
-    leftErrors = warp_prefix_dp<-1, GROUP>(w, T, tLeftBegin, tLeftBegin + 1, S, sLeftBegin, sLeftBegin + 1,
+    leftErrors = warp_prefix_dp<GROUP>(w, -1, T.c, tLen - mOffset, tLeftBegin + 1, S.c, sLen - mStart, sLeftBegin + 1,
                                     errorLimit - rightErrors, dovetailOnly, tLo, sLo, leftover, lToEnd);
     if (w.err) return kNone;
     for (int i = lane; i < w.leftLen; i += 32) w.sc.deltaL[i] = -w.sc.deltaL[i];

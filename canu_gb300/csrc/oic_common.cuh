@@ -5,8 +5,8 @@
 // its k-mer keys in, Build_Hash_Index.C:347-350) in two strand arrays -- forward and
 // reverse complement -- plus a parallel mask array with 0b11 at every N.  The DP reads the
 // same bases as bit planes (word i: the low bits of bases 32i .. 32i+31, then their high
-// bits), in which a comparison of 32 bases is four funnel shifts and two logic
-// instructions.  Reads start on a word boundary and are separated by one zero guard word,
+// bits, base 32i topmost), in which a comparison of 32 bases is four funnel shifts and two
+// logic instructions, and the first difference a count of leading zeros.  Reads start on a word boundary and are separated by one zero guard word,
 // so a 32-base window that runs off either end of a read stays inside the arrays.
 #pragma once
 
@@ -66,11 +66,18 @@ struct SeqView {
   const u64 *nm;   // its first N-mask word; nullptr when the read has no N
 };
 
-__device__ __forceinline__ SeqView make_view(const ReadsDev &R, u32 readIdx, int rev) {
-  SeqView v;
-  const u64 wo = R.wordOff[readIdx];
-  v.p  = (rev ? R.prc : R.pfwd) + wo;
-  v.nm = R.hasN[readIdx] ? (rev ? R.nrc : R.nfwd) + wo : nullptr;
+// A read strand and its reverse complement.
+struct ReadView {
+  SeqView f, c;
+};
+
+__device__ __forceinline__ ReadView make_view(const ReadsDev &R, u32 readIdx, int rev) {
+  ReadView v;
+  const u64  wo = R.wordOff[readIdx];
+  const bool hn = R.hasN[readIdx] != 0;
+  const SeqView a = {R.pfwd + wo, hn ? R.nfwd + wo : nullptr}, b = {R.prc + wo, hn ? R.nrc + wo : nullptr};
+  v.f = rev ? b : a;
+  v.c = rev ? a : b;
   return v;
 }
 
@@ -109,38 +116,35 @@ __host__ __device__ __forceinline__ u32 even_bits(u64 x) {
   return lo | (hi << 16);
 }
 
-// The low and the high bits of the 32 bases from base g of a read on (base g in bit 0).
+// The low and the high bits of the 32 bases from base g of a read on (base g topmost).
 __device__ __forceinline__ uint2 load_planes(const uint2 *p, int g) {
   const uint2 a = __ldg(p + (g >> 5)), b = __ldg(p + (g >> 5) + 1);
-  return make_uint2(__funnelshift_r(a.x, b.x, g), __funnelshift_r(a.y, b.y, g));
+  return make_uint2(__funnelshift_l(b.x, a.x, g), __funnelshift_l(b.y, a.y, g));
 }
 
 // m without the bits of bases that are N in A (from ga) or T (from gt).
 __device__ __forceinline__ u32 drop_n(u32 m, const u64 *An, int ga, const u64 *Tn, int gt) {
-  if (An) m &= ~even_bits(load_win32(An, ga));
-  if (Tn) m &= ~even_bits(load_win32(Tn, gt));
+  if (An) m &= ~__brev(even_bits(load_win32(An, ga)));
+  if (Tn) m &= ~__brev(even_bits(load_win32(Tn, gt)));
   return m;
 }
 
-// Bit 31 - i of the result is set when the bases at distance i (0..31) from A[a] and T[t]
-// differ, in the direction of STEP; an N matches anything
-// (prefixEditDistance-forward.C:164 / -reverse.C:186).
-template <int STEP>
-__device__ __forceinline__ u32 mismatch32(const SeqView &A, int a, const SeqView &T, int t) {
-  const int   ga = STEP > 0 ? a : a - 31, gt = STEP > 0 ? t : t - 31;
-  const uint2 x = load_planes(A.p, ga), y = load_planes(T.p, gt);
+// Number of leading bases (0..32) that agree between A (from a) and T (from t), an N
+// matching anything (prefixEditDistance-forward.C:164).  An extension to the left
+// (-reverse.C:186) compares the reads' reverse complements.
+__device__ __forceinline__ int match_run32(const SeqView &A, int a, const SeqView &T, int t) {
+  const uint2 x = load_planes(A.p, a), y = load_planes(T.p, t);
   u32         m = (x.x ^ y.x) | (x.y ^ y.y);
-  if (A.nm || T.nm) m = drop_n(m, A.nm, ga, T.nm, gt);
-  return STEP > 0 ? __brev(m) : m;
+  if (A.nm || T.nm) m = drop_n(m, A.nm, a, T.nm, t);
+  return __clz((int)m);
 }
 
-// Bases that agree from A[step*row] / T[step*(row+d)] on, capped at `lim` (> 0).
-template <int STEP>
+// Bases that agree from A[row] / T[row+d] on, capped at `lim` (> 0).
 __device__ __forceinline__ int slide(const SeqView &A, int a0, const SeqView &T, int t0, int row, int d, int lim,
                                      unsigned long long &slides) {
   int run = 0;
   while (run < lim) {
-    const int r = __clz((int)mismatch32<STEP>(A, a0 + STEP * (row + run), T, t0 + STEP * (row + d + run)));
+    const int r = match_run32(A, a0 + row + run, T, t0 + row + d + run);
     run += r;
     if (r < 32) break;
   }

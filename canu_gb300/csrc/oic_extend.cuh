@@ -25,8 +25,8 @@ static __device__ __forceinline__ void extend_loop(WarpDP &w, const ReadsDev &R,
       }
       continue;
     }
-    const SeqView S = make_view(R, pb.sRead, pb.sRev ? 1 : 0);
-    const SeqView T = make_view(R, pb.tRead, 0);
+    const ReadView S = make_view(R, pb.sRead, pb.sRev ? 1 : 0);
+    const ReadView T = make_view(R, pb.tRead, 0);
     const int sLen = (int)R.len[pb.sRead], tLen = (int)R.len[pb.tRead];
     int sLo = 0, sHi = 0, tLo = 0, tHi = 0, errors = 0;
     w.err = 0;

@@ -55,8 +55,8 @@ __global__ void pack_reads_kernel(const char *ascii, const u64 *srcOff, const u3
       nfwd[w0 + w] = fm;
       rc[w0 + w]   = b;
       nrc[w0 + w]  = bm;
-      pfwd[w0 + w] = make_uint2(even_bits(f), even_bits(f >> 1));
-      prc[w0 + w]  = make_uint2(even_bits(b), even_bits(b >> 1));
+      pfwd[w0 + w] = make_uint2(__brev(even_bits(f)), __brev(even_bits(f >> 1)));
+      prc[w0 + w]  = make_uint2(__brev(even_bits(b)), __brev(even_bits(b >> 1)));
     }
     anyN   = __syncthreads_or(anyN);
     anyBad = __syncthreads_or(anyBad);

@@ -254,7 +254,7 @@ __device__ void output_partial(u32 *dst, u32 sID, u32 tID, int rev, const Olap &
 
 // Extends node lm of (S, T) into res; the deltas stay in the warp's scratch.  The work is
 // reported in res only.
-__device__ __forceinline__ void extend_node(WarpDP &w, const SeqView &S, int sLen, const SeqView &T, int tLen,
+__device__ __forceinline__ void extend_node(WarpDP &w, const ReadView &S, int sLen, const ReadView &T, int tLen,
                                             const int4 &lm, ExtRes &res) {
   const int lane = threadIdx.x & 31;
   const unsigned long long c0 = w.cells, r0 = w.rows, s0 = w.slides;
@@ -304,7 +304,7 @@ constexpr unsigned char kNodeDead = 0, kNodeOpen = 1, kNodeOwner = 2, kNodeHelpe
 struct TeamPair {            // a pair open to helpers
   int            lock;
   int            open;       // nodes that can be claimed (kNodeOpen); 0: none, or no open pair
-  SeqView        S, T;
+  ReadView       S, T;
   int            sLen, tLen, cnt;
   const int4    *nodes;
   unsigned char *alive;      // kNode* of each match node, written under the lock
@@ -395,7 +395,7 @@ static __device__ __noinline__ void team_help(WarpDP &w, Team &tm, int me) {
     if (__shfl_sync(0xffffffffu, team_read(tm.owners), 0) == 0) return;
     const unsigned open = __ballot_sync(0xffffffffu, lane < kAlignWarps && team_read(tm.pair[lane].open) > 0);
     int  node = -1;
-    SeqView S, T;
+    ReadView S, T;
     int  sLen = 0, tLen = 0;
     int4 lm = make_int4(0, 0, 0, 0);
     if (open) {
@@ -471,7 +471,7 @@ __device__ __forceinline__ bool team_wait(Team &tm, int h) {
 // It is tried when its cells are estimated at less than half the work of extending the
 // group, from the last extension's cells and rows and the measured instructions of each.
 constexpr int kProofSpan = 64;
-static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, const SeqView &S, int sLen, const SeqView &T, int tLen,
+static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, const ReadView &S, int sLen, const ReadView &T, int tLen,
                                                         const int4 *nodes, int cnt, volatile unsigned char *alive,
                                                         float extCells, float extRows, Team *tm, int me, bool open) {
   const int lane = threadIdx.x & 31;
@@ -605,8 +605,8 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
   for (int i = lane; i < cnt; i += 32) alive[i] = kNodeOpen;
   __syncwarp();
 
-  const SeqView S = make_view(R, sRead, rev);
-  const SeqView T = make_view(R, tRead, 0);
+  const ReadView S = make_view(R, sRead, rev);
+  const ReadView T = make_view(R, tRead, 0);
   const unsigned long long cells0 = w.cells, slides0 = w.slides, rows0 = w.rows;
 
   // Pairs that run one extension, or stop after a few without an overlap, are not opened.
@@ -904,7 +904,7 @@ struct SpecShared {
   int         cmd;
   int         nCand;
   int         cand[kSpecWarps];
-  SeqView     S, T;
+  ReadView    S, T;
   int         sLen, tLen;
   const int4 *nodes;
   ExtRes      res[kSpecWarps];
