@@ -232,15 +232,15 @@ uint32_t read_err(oic_ctx *ctx) {
 }
 
 struct SeedConfig {
-  int warps;
+  int ctas;
   SeedCaps caps;
 };
 
-// Seed configurations, tried in this order for a ref strand: pair table and node
-// pool in HBM scratch on four warps per SM slot; in large HBM scratch on one warp per SM.
+// Seed configurations, tried in this order for a ref strand: pair table and node pool in
+// HBM scratch on seed_ctas_per_sm() CTAs per SM; in large HBM scratch on one CTA per SM.
 SeedConfig seed_normal(const oic_ctx *c) {
   SeedConfig s;
-  s.warps           = c->nSM * 8 * 4;
+  s.ctas         = c->nSM * seed_ctas_per_sm();
   s.caps.slotCap = 4096;
   s.caps.pairCap = 2048;
   s.caps.nodeCap = 32768;
@@ -248,7 +248,7 @@ SeedConfig seed_normal(const oic_ctx *c) {
 }
 SeedConfig seed_wide(const oic_ctx *c) {
   SeedConfig s;
-  s.warps        = c->nSM;
+  s.ctas         = c->nSM;
   s.caps.slotCap = 1 << 17;
   s.caps.pairCap = 1 << 16;
   s.caps.nodeCap = 1 << 22;
@@ -260,7 +260,7 @@ int ensure_seed_scratch(oic_ctx *ctx, const SeedConfig &sc, bool wide, SeedScrat
   DevBuf &v = wide ? ctx->dSeedSlotV2 : ctx->dSeedSlotV;
   DevBuf &p = wide ? ctx->dSeedPairs2 : ctx->dSeedPairs;
   DevBuf &n = wide ? ctx->dSeedNodes2 : ctx->dSeedNodes;
-  const size_t W = (size_t)((sc.warps + 3) / 4 * 4);
+  const size_t W = (size_t)sc.ctas;
   CK(k.ensure(W * sc.caps.slotCap * sizeof(int)));
   CK(v.ensure(W * sc.caps.slotCap * sizeof(int)));
   CK(p.ensure(W * sc.caps.pairCap * sizeof(PairAcc)));
@@ -549,7 +549,7 @@ int seed_stage(oic_ctx *ctx, const uint32_t *refs, uint32_t nRefs, cudaEvent_t e
       CK(cudaMemsetAsync(ctr32(ctx) + cSegOvf, 0, sizeof(uint32_t), ctx->st));
     }
     launch_seed(ctx->R, ctx->T, ctx->dp, ctx->dSegReads.as<uint32_t>(), t ? ctx->dSegList.as<uint32_t>() : nullptr,
-                nTodo, ctr32(ctx) + cSegCounter, ss, tiers[t].caps, tiers[t].warps, so, ctx->st);
+                nTodo, ctr32(ctx) + cSegCounter, ss, tiers[t].caps, tiers[t].ctas, so, ctx->st);
     CK(cudaMemcpyAsync(h, ctx->dCtr.p, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->st));
     if ((rc = sync_check(ctx, "seed kernel"))) return rc;
     if (h[cErr] & (kErrOutNodes | kErrOutPairs)) {

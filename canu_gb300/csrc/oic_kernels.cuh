@@ -49,7 +49,7 @@ struct PairRec {
   u32 flags;      // bit0 reverse strand, bit1 consistent, bit2 S left-end screened, bit3 S right-end screened
 };
 
-struct PairAcc {   // seed-replay state of one pair (per-warp scratch)
+struct PairAcc {   // seed-replay state of one pair
   u32 T;
   int head;
   int diagCt, diagBgn, diagEnd;
@@ -59,10 +59,10 @@ struct PairAcc {   // seed-replay state of one pair (per-warp scratch)
 };
 
 struct SeedScratch {
-  int     *slotKey;    // per warp: slotCap ints
+  int     *slotKey;    // per CTA: slotCap ints
   int     *slotVal;
-  PairAcc *pairs;      // per warp: pairCap
-  int4    *nodes;      // per warp: nodeCap (offset, len, start, next)
+  PairAcc *pairs;      // per CTA: pairCap
+  int4    *nodes;      // per CTA: nodeCap (offset, len, start, next)
 };
 
 struct SeedCaps {
@@ -86,7 +86,9 @@ struct SeedOut {
 
 // Segment k is (ref index << 1 | strand) = segList[k], or k when segList is null.
 void launch_seed(ReadsDev R, TableDev T, DevParams P, const u32 *segReads, const u32 *segList, u32 nSeg,
-                 u32 *segCounter, SeedScratch sc, SeedCaps cap, int nWarps, SeedOut out, cudaStream_t st);
+                 u32 *segCounter, SeedScratch sc, SeedCaps cap, int ctas, SeedOut out, cudaStream_t st);
+
+int seed_ctas_per_sm();
 
 // ---------------- pairs / DP ----------------
 struct AlignOut {
