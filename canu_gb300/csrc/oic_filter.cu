@@ -398,44 +398,46 @@ __global__ void __launch_bounds__(kBwdWarps * 32) mlp_bwd_hidden_kernel(const __
 }
 
 // grad W[m][c] += sum_s G[s][m] * H[s][c]   (M = 128, N = NC columns of H)
-// grad b[m]    += sum_s G[s][m]
-// Each block takes a contiguous range of samples in steps of 32.
+// grad b[m]    += sum_s G[s][m]             (as the product with a column of ones)
+// for both layers in one launch: blocks of y 0 take layer 2 (G2, H1), of y 1 layer 1 (G1, X).
+// Each block takes a contiguous range of samples in steps of 64.
+//
+// What bounds it is the latency of a step and the FP32 atomics of a block's 128 x NC sums.
+// One launch per layer in blocks of at least 1,024 samples put 32 blocks on 152 SMs (87 + 81
+// us at 32,768 samples; now 25 us for both), and a serial sum over the rows for the bias was
+// half of a step.
 constexpr int kWgWarps = 8;
-constexpr int kWgRows  = 32;
+constexpr int kWgRows  = 64;
+constexpr u32 kWgMin   = 256;
 
-template <int NC>
 struct WgSmem {
   __half g[kWgRows * kHS];
   __half h[kWgRows * kHS];
-  float  bsum[kHid];
 };
 
 template <int NC>
-__global__ void __launch_bounds__(kWgWarps * 32) mlp_wgrad_kernel(const __half *G, const __half *H, u32 n,
-                                                                 u32 perBlock, float *gradW, float *gradB) {
-  __shared__ __align__(16) WgSmem<NC> s;
+__device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __half *H, u32 n, u32 perBlock,
+                                            float *gradW, float *gradB) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  constexpr int NT = NC / 8;
-  float acc[NT][4];
+  constexpr int NT   = NC / 8;
+  constexpr u32 kOne = 0x3c003c00u;   // two FP16 ones
+  float acc[NT][4], bsum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int i = 0; i < NT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-  float bs = 0.0f;
   const u64 s0 = (u64)blockIdx.x * perBlock;
   const u64 s1 = s0 + perBlock < n ? s0 + perBlock : n;
   const int m0 = wib * 16;
   for (u64 r = s0; r < s1; r += kWgRows) {
     __syncthreads();
-    const u64 lim = s1;
-    stage_rows(s.g, kHS, G, kHid, r, kWgRows, lim, threadIdx.x, blockDim.x);
-    stage_rows(s.h, kHS, H, NC, r, kWgRows, lim, threadIdx.x, blockDim.x);
+    stage_rows(s.g, kHS, G, kHid, r, kWgRows, s1, threadIdx.x, blockDim.x);
+    stage_rows(s.h, kHS, H, NC, r, kWgRows, s1, threadIdx.x, blockDim.x);
     __syncthreads();
-    if (threadIdx.x < kHid)
-      for (int q = 0; q < kWgRows; q++) bs += __half2float(s.g[q * kHS + threadIdx.x]);
 #pragma unroll
     for (int ks = 0; ks < kWgRows / 16; ks++) {
       // A[m][k] = G[k][m]: stored [k][m], transposed ldmatrix.
       u32 a[4];
       ldsm_x4_t(a, s.g + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * kHS + m0 + ((lane >> 3) & 1) * 8);
+      mma16816(bsum, a, kOne, kOne);
 #pragma unroll
       for (int np = 0; np < NT / 2; np++) {
         u32 b[4];
@@ -454,7 +456,17 @@ __global__ void __launch_bounds__(kWgWarps * 32) mlp_wgrad_kernel(const __half *
     atomicAdd(&gradW[(m0 + g + 8) * NC + c], acc[nt][2]);
     atomicAdd(&gradW[(m0 + g + 8) * NC + c + 1], acc[nt][3]);
   }
-  if (threadIdx.x < kHid) atomicAdd(&gradB[threadIdx.x], bs);
+  if (t == 0) {   // every column of the product with ones is the sum
+    atomicAdd(&gradB[m0 + g], bsum[0]);
+    atomicAdd(&gradB[m0 + g + 8], bsum[2]);
+  }
+}
+
+__global__ void __launch_bounds__(kWgWarps * 32) mlp_wgrad_kernel(const __half *G2, const __half *H1, const __half *G1,
+                                                                 const __half *X, u32 n, u32 perBlock, float *grad) {
+  __shared__ __align__(16) WgSmem s;
+  if (blockIdx.y == 0) wgrad_block<kHid>(s, G2, H1, n, perBlock, grad + kOffW2, grad + kOffB2);
+  else wgrad_block<kIn>(s, G1, X, n, perBlock, grad + kOffW1, grad + kOffB1);
 }
 
 // Adam on FP32 master weights; writes the FP16 copy and clears the gradient.
@@ -508,7 +520,9 @@ cudaError_t launch_mlp_forward(const void *prm, const void *X, u32 n, float *log
   const size_t smem = sizeof(FwdSmem);
   cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int blocks = blocks_for(((u64)n + 15) / 16, kFwdWarps * 4, num_sms() * 2);
+  // One tile per warp until the SMs are full (four per warp left half of them idle at
+  // 32,768 samples: 33 us, now 18).
+  const int blocks = blocks_for(((u64)n + 15) / 16, kFwdWarps, num_sms() * 2);
   mlp_forward_kernel<<<blocks, kFwdWarps * 32, smem, st>>>((const __half *)prm, (const __half *)X, n, logit,
                                                            (__half *)H1, (__half *)H2);
   g_launches++;
@@ -522,20 +536,19 @@ cudaError_t launch_mlp_backward(const void *prm, const void *X, const void *H1, 
   const size_t smem = sizeof(BwdSmem);
   cudaError_t e = cudaFuncSetAttribute(mlp_bwd_hidden_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int blocks = blocks_for(((u64)n + 15) / 16, kBwdWarps * 4, num_sms() * 2);
+  const int blocks = blocks_for(((u64)n + 15) / 16, kBwdWarps, num_sms() * 2);
   mlp_bwd_hidden_kernel<<<blocks, kBwdWarps * 32, smem, st>>>((const __half *)prm, (const __half *)H1,
                                                               (const __half *)H2, logit, label, weight, n,
                                                               (__half *)G2, (__half *)G1, grad, loss);
   g_launches++;
-  // Weight gradients: blocks of at least 1024 samples keep the FP32 atomics few.
-  u32 per = 1024;
+  // Weight gradients: about two blocks per SM and layer, but at least kWgMin samples each,
+  // so that the FP32 atomics of a block's sums stay a small part (a step of 32,768 samples
+  // with at least 128 / 256 / 512: 98 / 90 / 89 us; 256 keeps smaller batches spread).
+  u32 per = kWgMin;
   while ((u64)per * num_sms() * 2 < n) per *= 2;
-  const int wb = (int)(((u64)n + per - 1) / per);
-  mlp_wgrad_kernel<kHid><<<wb, kWgWarps * 32, 0, st>>>((const __half *)G2, (const __half *)H1, n, per,
-                                                       grad + kOffW2, grad + kOffB2);
-  g_launches++;
-  mlp_wgrad_kernel<kIn><<<wb, kWgWarps * 32, 0, st>>>((const __half *)G1, (const __half *)X, n, per, grad + kOffW1,
-                                                      grad + kOffB1);
+  const dim3 wb((unsigned)(((u64)n + per - 1) / per), 2);
+  mlp_wgrad_kernel<<<wb, kWgWarps * 32, 0, st>>>((const __half *)G2, (const __half *)H1, (const __half *)G1,
+                                                 (const __half *)X, n, per, grad);
   g_launches++;
   return cudaGetLastError();
 }
