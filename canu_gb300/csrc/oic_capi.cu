@@ -197,6 +197,7 @@ constexpr int kSeedStatBase  = 16;   // u64 index: [seeds, segments]
 constexpr int kAlignStatBase = 20;   // u64 index: kStCount entries
 constexpr int kExtStatBase   = 40;
 constexpr int kCellsSnap     = 60;   // u64 index: DP cells after the one-warp bin of a captured batch
+constexpr int kHashBase      = 62;   // u64 index: [valid k-mers, distinct k-mers] of a hash block
 static_assert(kNoAllocStatBase >= kExtStatBase + 3 && kNoAllocStatBase + 3 <= kCellsSnap,
               "the no-allocation entry point's counters overlap another slot");
 
@@ -1401,6 +1402,9 @@ int oic_load_hash_block(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t *
   CK(cudaMemcpyAsync(ctx->dStrKmers.p, strKmers.data(), nCand * 4, cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemcpyAsync(ctx->dFlat.p, flat.data(), (size_t)(nCand + 1) * 8, cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemsetAsync(ctx->dNewKeys.p, 0, (size_t)nCand * 4 + 4, ctx->st));
+  // With no more k-mers than the entry limit no read can meet it: the block is every
+  // candidate string, and the strings' new k-mers need not be known one by one.
+  const bool whole = nFlat <= entryLim;
   if (nCand) launch_chunk_str(ctx->dFlat.as<u64>(), nCand, nFlat, ctx->dChunkStr.as<uint32_t>(), ctx->st);
 
   const size_t n = (size_t)nFlat;
@@ -1408,43 +1412,59 @@ int oic_load_hash_block(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t *
   CK(ctx->dSortV.ensure(n * 4 + 4));
   CK(ctx->dSortK2.ensure(n * 8 + 8));
   CK(ctx->dSortV2.ensure(n * 4 + 4));
-  CK(ctx->dFlags.ensure(n * 4 + 4));
-  CK(ctx->dPos.ensure(n * 4 + 4));
+  if (!whole) {
+    CK(ctx->dFlags.ensure(n * 4 + 4));
+    CK(ctx->dPos.ensure(n * 4 + 4));
+  }
   CK(ctx->dSortScratch.ensure(std::max(radix_sort_scratch(n), scan_u32_scratch(n)) + 256));
 
   launch_kmer_emit(ctx->R, ctx->dStrRead.as<uint32_t>(), ctx->dStrKmers.as<uint32_t>(), ctx->dFlat.as<u64>(), nCand,
                    (int)K, ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), ctx->st);
   CK(radix_sort_u64_u32(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), ctx->dSortK2.as<u64>(),
                         ctx->dSortV2.as<uint32_t>(), n, 2 * (int)K + 1, ctx->dSortScratch.p, ctx->st));
-  launch_first_occ(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), n, ctx->dFlat.as<u64>(),
-                   ctx->dChunkStr.as<uint32_t>(), (int)K,
-                   ctx->dNewKeys.as<uint32_t>(), ctx->st);
-  std::vector<uint32_t> newKeys(nCand);
-  CK(cudaMemcpyAsync(newKeys.data(), ctx->dNewKeys.p, (size_t)nCand * 4, cudaMemcpyDeviceToHost, ctx->st));
-  int rc = sync_check(ctx, "hash k-mer sort");
-  if (rc) return rc;
+  int      rc  = OIC_OK;
+  uint32_t cut = nCand, nOcc = 0;
+  uint64_t distinct = 0;
+  const u64      *occKeys = ctx->dSortK.as<u64>();
+  const uint32_t *occVals = ctx->dSortV.as<uint32_t>();
+  if (whole) {
+    // The occurrences are the valid keys, which sort before the windows with an N.
+    unsigned long long hc[2];
+    CK(cudaMemsetAsync(ctr64(ctx) + kHashBase, 0, sizeof(hc), ctx->st));
+    launch_count_runs(occKeys, n, (int)K, ctr64(ctx) + kHashBase, ctr64(ctx) + kHashBase + 1, ctx->st);
+    CK(cudaMemcpyAsync(hc, ctr64(ctx) + kHashBase, sizeof(hc), cudaMemcpyDeviceToHost, ctx->st));
+    if ((rc = sync_check(ctx, "hash k-mer sort"))) return rc;
+    nOcc     = (uint32_t)hc[0];
+    distinct = hc[1];
+  } else {
+    launch_first_occ(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), n, ctx->dFlat.as<u64>(),
+                     ctx->dChunkStr.as<uint32_t>(), (int)K, ctx->dNewKeys.as<uint32_t>(), ctx->st);
+    std::vector<uint32_t> newKeys(nCand);
+    CK(cudaMemcpyAsync(newKeys.data(), ctx->dNewKeys.p, (size_t)nCand * 4, cudaMemcpyDeviceToHost, ctx->st));
+    if ((rc = sync_check(ctx, "hash k-mer sort"))) return rc;
 
-  // The load loop stops before a read once the data length or the distinct-k-mer
-  // count reached its limit (Build_Hash_Index.C:504-506).
-  uint32_t cut = 0;
-  uint64_t len = 0, distinct = 0;
-  for (; cut < nCand; cut++) {
-    if (!(len < maxData && distinct < entryLim)) break;
-    if (eligible[cut]) len += (uint64_t)strLen[cut] + 1;
-    distinct += newKeys[cut];
+    // The load loop stops before a read once the data length or the distinct-k-mer
+    // count reached its limit (Build_Hash_Index.C:504-506).
+    uint64_t len = 0;
+    for (cut = 0; cut < nCand; cut++) {
+      if (!(len < maxData && distinct < entryLim)) break;
+      if (eligible[cut]) len += (uint64_t)strLen[cut] + 1;
+      distinct += newKeys[cut];
+    }
+
+    // Keep the occurrences of the loaded strings (and drop windows with an N).
+    launch_keep_flags(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), n, (int)K, (uint32_t)flat[cut],
+                      ctx->dFlags.as<uint32_t>(), ctx->st);
+    CK(scan_u32(ctx->dFlags.as<uint32_t>(), ctx->dPos.as<uint32_t>(), n, ctr32(ctx) + cRecTotal, ctx->dSortScratch.p,
+                ctx->st));
+    launch_compact_kv(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), ctx->dFlags.as<uint32_t>(),
+                      ctx->dPos.as<uint32_t>(), n, ctx->dSortK2.as<u64>(), ctx->dSortV2.as<uint32_t>(), ctx->st);
+    CK(cudaMemcpyAsync(&nOcc, ctr32(ctx) + cRecTotal, 4, cudaMemcpyDeviceToHost, ctx->st));
+    if ((rc = sync_check(ctx, "hash compaction"))) return rc;
+    occKeys = ctx->dSortK2.as<u64>();
+    occVals = ctx->dSortV2.as<uint32_t>();
   }
   const uint32_t nStr = cut;
-
-  // Keep the occurrences of the loaded strings (and drop windows with an N).
-  launch_keep_flags(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), n, (int)K, (uint32_t)flat[nStr],
-                    ctx->dFlags.as<uint32_t>(), ctx->st);
-  CK(scan_u32(ctx->dFlags.as<uint32_t>(), ctx->dPos.as<uint32_t>(), n, ctr32(ctx) + cRecTotal, ctx->dSortScratch.p,
-              ctx->st));
-  launch_compact_kv(ctx->dSortK.as<u64>(), ctx->dSortV.as<uint32_t>(), ctx->dFlags.as<uint32_t>(),
-                    ctx->dPos.as<uint32_t>(), n, ctx->dSortK2.as<u64>(), ctx->dSortV2.as<uint32_t>(), ctx->st);
-  uint32_t nOcc = 0;
-  CK(cudaMemcpyAsync(&nOcc, ctr32(ctx) + cRecTotal, 4, cudaMemcpyDeviceToHost, ctx->st));
-  if ((rc = sync_check(ctx, "hash compaction"))) return rc;
 
   uint64_t cap = 1024;
   while (cap < 2 * (distinct + ctx->skipKeys.size() + 1)) cap <<= 1;
@@ -1453,8 +1473,8 @@ int oic_load_hash_block(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t *
   CK(ctx->dOcc.ensure((size_t)nOcc * 8 + 8));
   launch_table_init(ctx->dTable.as<u64>(), cap, ctx->st);
   CK(cudaMemsetAsync(ctr32(ctx) + cErr, 0, 4, ctx->st));
-  launch_table_build(ctx->dSortK2.as<u64>(), nOcc, ctx->dTable.as<u64>(), cap - 1, ctr32(ctx) + cErr, ctx->st);
-  launch_occ_convert(ctx->dSortV2.as<uint32_t>(), nOcc, ctx->dFlat.as<u64>(), ctx->dChunkStr.as<uint32_t>(),
+  launch_table_build(occKeys, nOcc, ctx->dTable.as<u64>(), cap - 1, ctr32(ctx) + cErr, ctx->st);
+  launch_occ_convert(occVals, nOcc, ctx->dFlat.as<u64>(), ctx->dChunkStr.as<uint32_t>(),
                      ctx->dOcc.as<u64>(), ctx->st);
 
   // String_Info (Build_Hash_Index.C:511-536): loaded strings unscreened, skipped ones screened.

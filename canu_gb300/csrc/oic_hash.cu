@@ -133,53 +133,70 @@ __global__ void compact_kv_kernel(const u64 *keys, const u32 *vals, const u32 *f
     }
 }
 
-__device__ __forceinline__ bool table_slot(const u64 *tKV, u64 mask, u64 key, u64 &slot) {
-  u64 s = mix64(key) & mask;
-  for (u64 probe = 0; probe <= mask; probe++) {
-    u64 k = tKV[2 * s];
-    if (k == key) { slot = s; return true; }
-    if (k == kEmptyKey) return false;
-    s = (s + 1) & mask;
-  }
-  return false;
-}
-
 // Every slot empty: key all ones, value 0 (one 16-byte store per slot).
 __global__ void table_init_kernel(u64 *tKV, u64 cap) {
   for (u64 s = (u64)blockIdx.x * blockDim.x + threadIdx.x; s < cap; s += (u64)gridDim.x * blockDim.x)
     ((ulonglong2 *)tKV)[s] = make_ulonglong2(kEmptyKey, 0ull);
 }
 
-// Run starts claim a slot; the occurrence run begins at p.
-__global__ void table_starts_kernel(const u64 *keys, u64 n, u64 *tKV, u64 mask, u32 *err) {
+// Valid keys (they sort before the invalid one) and distinct keys among them.
+__global__ void __launch_bounds__(256) count_runs_kernel(const u64 *keys, u64 n, int K, unsigned long long *valid,
+                                                         unsigned long long *distinct) {
+  const u64 invalid = 1ull << (2 * K);
+  u32 nv = 0, nd = 0;
   for (u64 p = (u64)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (u64)gridDim.x * blockDim.x) {
-    u64 k = keys[p];
+    const u64 k = keys[p];
+    if (k >= invalid) continue;
+    nv++;
+    nd += p == 0 || keys[p - 1] != k;
+  }
+  nv = __reduce_add_sync(0xffffffffu, nv);
+  nd = __reduce_add_sync(0xffffffffu, nd);
+  __shared__ u32 s[2];
+  if (threadIdx.x < 2) s[threadIdx.x] = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&s[0], nv);
+    atomicAdd(&s[1], nd);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicAdd(valid, (unsigned long long)s[0]);
+    atomicAdd(distinct, (unsigned long long)s[1]);
+  }
+}
+
+// The first key of each run claims a slot and finds the run's end: doubling steps, then a
+// binary search (most runs hold one key, and a repeat's thousands).  One access to the
+// table per distinct key; a second kernel that looked the run ends up again took as long.
+__global__ void table_runs_kernel(const u64 *keys, u64 n, u64 *tKV, u64 mask, u32 *err) {
+  for (u64 p = (u64)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (u64)gridDim.x * blockDim.x) {
+    const u64 k = keys[p];
     if (p > 0 && keys[p - 1] == k) continue;
+    u64 last = p, next = p + 1, step = 1;   // keys[last] == k
+    while (next < n && keys[next] == k) {
+      last = next;
+      step <<= 1;
+      next = last + step;
+    }
+    next = next < n ? next : n;             // past the run
+    while (next - last > 1) {
+      const u64 mid = (last + next) >> 1;
+      if (keys[mid] == k) last = mid;
+      else next = mid;
+    }
     u64  s    = mix64(k) & mask;
     bool done = false;
     for (u64 probe = 0; probe <= mask; probe++) {
       u64 old = atomicCAS(&tKV[2 * s], kEmptyKey, k);
       if (old == kEmptyKey || old == k) {
-        tKV[2 * s + 1] = p;
-        done     = true;
+        tKV[2 * s + 1] = p | ((next - p) << 32);
+        done           = true;
         break;
       }
       s = (s + 1) & mask;
     }
     if (!done) atomicOr(err, kErrTableFull);
-  }
-}
-
-// Run ends fill in the count.
-__global__ void table_counts_kernel(const u64 *keys, u64 n, u64 *tKV, u64 mask) {
-  for (u64 p = (u64)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (u64)gridDim.x * blockDim.x) {
-    u64 k = keys[p];
-    if (p + 1 < n && keys[p + 1] == k) continue;
-    u64 s;
-    if (table_slot(tKV, mask, k, s)) {
-      u64 start      = tKV[2 * s + 1] & 0xffffffffull;
-      tKV[2 * s + 1] = start | ((p + 1 - start) << 32);
-    }
   }
 }
 
@@ -195,40 +212,50 @@ __global__ void occ_convert_kernel(const u32 *vals, u64 n, const u64 *flatStart,
 // screen the read ends near its occurrences (Mark_Screened_Ends_Chain, :96-121); with
 // the hopeless check on, an absent k-mer gets an empty entry of its own
 // (Add_Extra_Hash_String, :26-86) so that probes still see it as screened.
+//
+// A warp per k-mer: lane 0 finds it, all lanes go through its occurrences (a thread each
+// walked runs of thousands alone: 2.1 ms for 150 Mbp of reads).
 __global__ void skip_mark_kernel(const u64 *skipKeys, u64 nSkip, TableDev T, u64 *tKV,
                                  unsigned char *lscr, unsigned char *rscr, int K, int hopeless, u32 *err) {
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < nSkip; i += (u64)gridDim.x * blockDim.x) {
-    const u64 key = skipKeys[i];
-    u64       s   = mix64(key) & T.mask;
-    bool      done = false;
-    for (u64 probe = 0; probe <= T.mask && !done; probe++) {
-      u64 k = tKV[2 * s];
-      if (k == kEmptyKey) {
-        if (!hopeless) { done = true; break; }
-        k = atomicCAS(&tKV[2 * s], kEmptyKey, key);
+  const int lane = threadIdx.x & 31;
+  const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
+  for (u64 i = (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < nSkip; i += warps) {
+    u32 start = 0, cnt = 0;
+    if (lane == 0) {
+      const u64 key = skipKeys[i];
+      u64       s   = mix64(key) & T.mask;
+      bool      done = false;
+      for (u64 probe = 0; probe <= T.mask && !done; probe++) {
+        u64 k = tKV[2 * s];
         if (k == kEmptyKey) {
-          atomicOr(&tKV[2 * s + 1], 1ull << 63);   // count 0, screened
-          done = true;
+          if (!hopeless) { done = true; break; }
+          k = atomicCAS(&tKV[2 * s], kEmptyKey, key);
+          if (k == kEmptyKey) {
+            atomicOr(&tKV[2 * s + 1], 1ull << 63);   // count 0, screened
+            done = true;
+            break;
+          }
+        }
+        if (k == key) {
+          u64 v = atomicOr(&tKV[2 * s + 1], 1ull << 63);
+          start = (u32)(v & 0xffffffffull);
+          cnt   = (u32)((v >> 32) & 0x7fffffffull);
+          done  = true;
           break;
         }
+        s = (s + 1) & T.mask;
       }
-      if (k == key) {
-        u64 v = atomicOr(&tKV[2 * s + 1], 1ull << 63);
-        u32 start = (u32)(v & 0xffffffffull);
-        u32 cnt   = (u32)((v >> 32) & 0x7fffffffull);
-        for (u32 j = 0; j < cnt; j++) {
-          u64 o   = T.occ[start + j];
-          u32 str = (u32)(o >> 32);
-          u64 off = (u32)o;
-          if (off < (u64)kHopelessMatch) lscr[str] = 1;
-          if ((u64)T.slen[str] - off - (u64)K + 1 < (u64)kHopelessMatch) rscr[str] = 1;
-        }
-        done = true;
-        break;
-      }
-      s = (s + 1) & T.mask;
+      if (!done) atomicOr(err, kErrTableFull);
     }
-    if (!done) atomicOr(err, kErrTableFull);
+    start = __shfl_sync(0xffffffffu, start, 0);
+    cnt   = __shfl_sync(0xffffffffu, cnt, 0);
+    for (u32 j = lane; j < cnt; j += 32) {
+      u64 o   = T.occ[start + j];
+      u32 str = (u32)(o >> 32);
+      u64 off = (u32)o;
+      if (off < (u64)kHopelessMatch) lscr[str] = 1;
+      if ((u64)T.slen[str] - off - (u64)K + 1 < (u64)kHopelessMatch) rscr[str] = 1;
+    }
   }
 }
 
@@ -278,6 +305,14 @@ void launch_first_occ(const u64 *keys, const u32 *vals, u64 n, const u64 *flatSt
   g_launches++;
 }
 
+void launch_count_runs(const u64 *keys, u64 n, int K, unsigned long long *valid, unsigned long long *distinct,
+                       cudaStream_t st) {
+  if (n == 0) return;
+  const unsigned g = grid_for(n, 256 * 16);
+  count_runs_kernel<<<g, 256, 0, st>>>(keys, n, K, valid, distinct);
+  g_launches++;
+}
+
 void launch_keep_flags(const u64 *keys, const u32 *vals, u64 n, int K, u32 flatLimit, u32 *flags, cudaStream_t st) {
   if (n == 0) return;
   keep_flags_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, vals, n, K, flatLimit, flags);
@@ -298,9 +333,7 @@ void launch_table_init(u64 *tKV, u64 cap, cudaStream_t st) {
 
 void launch_table_build(const u64 *keys, u64 n, u64 *tKV, u64 mask, u32 *err, cudaStream_t st) {
   if (n == 0) return;
-  table_starts_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, n, tKV, mask, err);
-  g_launches++;
-  table_counts_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, n, tKV, mask);
+  table_runs_kernel<<<grid_for(n, 256), 256, 0, st>>>(keys, n, tKV, mask, err);
   g_launches++;
 }
 
@@ -313,7 +346,7 @@ void launch_occ_convert(const u32 *vals, u64 n, const u64 *flatStart, const u32 
 void launch_skip_mark(const u64 *skipKeys, u64 nSkip, TableDev T, u64 *tKVMut, unsigned char *lscr,
                       unsigned char *rscr, int K, int hopeless, u32 *err, cudaStream_t st) {
   if (nSkip == 0) return;
-  skip_mark_kernel<<<grid_for(nSkip, 128), 128, 0, st>>>(skipKeys, nSkip, T, tKVMut, lscr, rscr, K, hopeless, err);
+  skip_mark_kernel<<<grid_for(nSkip, 8), 256, 0, st>>>(skipKeys, nSkip, T, tKVMut, lscr, rscr, K, hopeless, err);
   g_launches++;
 }
 

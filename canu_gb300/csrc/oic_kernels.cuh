@@ -27,12 +27,16 @@ void launch_kmer_emit(ReadsDev R, const u32 *strRead, const u32 *strKmers, const
 void launch_chunk_str(const u64 *flatStart, u32 nStr, u64 nFlat, u32 *chunkStr, cudaStream_t st);
 void launch_first_occ(const u64 *keys, const u32 *vals, u64 n, const u64 *flatStart, const u32 *chunkStr, int K,
                       u32 *newKeys, cudaStream_t st);
+// *valid += valid keys of the sorted keys[0 .. n), *distinct += distinct ones among them.
+void launch_count_runs(const u64 *keys, u64 n, int K, unsigned long long *valid, unsigned long long *distinct,
+                       cudaStream_t st);
 // flags[p] = 1 when keys[p] is a valid k-mer and vals[p] < flatLimit.
 void launch_keep_flags(const u64 *keys, const u32 *vals, u64 n, int K, u32 flatLimit, u32 *flags, cudaStream_t st);
 void launch_compact_kv(const u64 *keys, const u32 *vals, const u32 *flags, const u32 *pos, u64 n, u64 *keysOut,
                        u32 *valsOut, cudaStream_t st);
 // Open-addressing table of 16-byte slots (key, value) at tKV, capacity mask + 1;
-// launch_table_init empties every slot.
+// launch_table_init empties every slot; launch_table_build enters the runs of the sorted
+// keys.
 void launch_table_init(u64 *tKV, u64 cap, cudaStream_t st);
 void launch_table_build(const u64 *keys, u64 n, u64 *tKV, u64 mask, u32 *err, cudaStream_t st);
 void launch_occ_convert(const u32 *vals, u64 n, const u64 *flatStart, const u32 *chunkStr, u64 *occ, cudaStream_t st);

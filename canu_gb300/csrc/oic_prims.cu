@@ -3,8 +3,8 @@
 // Scan: three-phase (per-tile reduce, recursive scan of tile sums, per-tile scan).
 // Sort: 8-bit digits; per pass an upsweep histogram per 4096-key tile (digit-major,
 // so one exclusive scan gives every (digit, tile) its output base), then a downsweep
-// that ranks keys stably inside the tile with warp match_any, groups the tile by digit
-// in shared memory and writes each digit's run out with coalesced stores.
+// that ranks keys stably inside the tile, groups the tile by digit in shared memory and
+// writes each digit's run out with coalesced stores.
 #include "oic_prims.cuh"
 
 namespace oic {
@@ -122,39 +122,51 @@ cudaError_t scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *to
 
 namespace {
 
-constexpr int kSortThreads = 256;
+constexpr int kUpThreads   = 256;                         // upsweep
+constexpr int kUpItems     = 16;
+constexpr int kSortThreads = 512;                         // downsweep
 constexpr int kSortWarps   = kSortThreads / 32;
-constexpr int kSortItems   = 16;
+constexpr int kSortItems   = 8;
 constexpr int kSortTile    = kSortThreads * kSortItems;   // 4096
 constexpr int kDigits      = 256;
+static_assert(kUpThreads * kUpItems == kSortTile && kUpThreads == kDigits, "one histogram per downsweep tile");
 
-__global__ void __launch_bounds__(kSortThreads) radix_upsweep_kernel(const unsigned long long *keys, uint64_t n, int shift,
+__global__ void __launch_bounds__(kUpThreads) radix_upsweep_kernel(const unsigned long long *keys, uint64_t n, int shift,
                                                                      uint32_t *hist, uint32_t nTiles,
                                                                      const uint32_t *nDev) {
-  __shared__ uint32_t h[kSortWarps][kDigits];
+  __shared__ uint32_t h[(kUpThreads / 32)][kDigits];
   if (nDev && *nDev < n) n = *nDev;
   const int wid = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kSortWarps * kDigits; i += kSortThreads) (&h[0][0])[i] = 0;
-  __syncthreads();
   const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
+  if (base >= n) {   // a tile past the end (launches sized for a capacity)
+    hist[(uint64_t)threadIdx.x * nTiles + blockIdx.x] = 0;
+    return;
+  }
+  for (int i = threadIdx.x; i < (kUpThreads / 32) * kDigits; i += kUpThreads) (&h[0][0])[i] = 0;
+  __syncthreads();
 #pragma unroll 4
-  for (int k = 0; k < kSortItems; k++) {
-    uint64_t i = base + (uint64_t)k * kSortThreads + threadIdx.x;
+  for (int k = 0; k < kUpItems; k++) {
+    uint64_t i = base + (uint64_t)k * kUpThreads + threadIdx.x;
     if (i < n) atomicAdd(&h[wid][(keys[i] >> shift) & 0xff], 1u);
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < kDigits; d += kSortThreads) {
+  for (int d = threadIdx.x; d < kDigits; d += kUpThreads) {
     uint32_t s = 0;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; w++) s += h[w][d];
+    for (int w = 0; w < (kUpThreads / 32); w++) s += h[w][d];
     hist[(uint64_t)d * nTiles + blockIdx.x] = s;
   }
 }
 
 // Downsweep of one 4096-key tile: rank every key inside the tile (stable: warp order,
-// then item order, then lane order) with warp match_any, place the tile in shared
-// memory grouped by digit, then write each digit's run to its output range -- the
-// writes of consecutive threads go to consecutive addresses.
+// then item order, then lane order), place the tile in shared memory grouped by digit, then
+// write each digit's run to its output range -- the writes of consecutive threads go to
+// consecutive addresses.  VALS false: keys only.
+//
+// The lanes with the same digit are found with eight ballots: match_any walks a warp's
+// distinct digits one by one, and 8 warps x 16 keys of them waited for it two thirds of the
+// time (97 G keys/s).
+template <bool VALS>
 __global__ void __launch_bounds__(kSortThreads) radix_downsweep_kernel(const unsigned long long *keysIn, const uint32_t *valsIn,
                                                                        unsigned long long *keysOut, uint32_t *valsOut, uint64_t n,
                                                                        int shift, const uint32_t *offsets,
@@ -162,83 +174,91 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep_kernel(const uns
   extern __shared__ __align__(16) unsigned char sortDyn[];
   unsigned long long *sk = (unsigned long long *)sortDyn;           // kSortTile keys
   uint32_t           *sv = (uint32_t *)(sk + kSortTile);             // kSortTile values
-  __shared__ uint32_t cnt[kSortWarps][kDigits];
-  __shared__ uint32_t tileBase[kDigits];     // output position of the tile's first key of each digit
-  __shared__ uint32_t localStart[kDigits];   // position of that key inside the tile
+  __shared__ uint16_t cnt[kSortWarps][kDigits];
+  __shared__ uint32_t tileBase[kDigits];     // output position of the tile's first key of each digit ...
+  __shared__ uint32_t warpSums[kDigits / 32];
   if (nDev && *nDev < n) n = *nDev;
+  const uint64_t tile0 = (uint64_t)blockIdx.x * kSortTile;
+  if (tile0 >= n) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kSortWarps * kDigits; i += kSortThreads) (&cnt[0][0])[i] = 0;
-  for (int d = threadIdx.x; d < kDigits; d += kSortThreads) tileBase[d] = offsets[(uint64_t)d * nTiles + blockIdx.x];
+  for (int i = threadIdx.x; i < kSortWarps * kDigits / 2; i += kSortThreads) ((uint32_t *)&cnt[0][0])[i] = 0;
   __syncthreads();
 
-  const uint64_t base = (uint64_t)blockIdx.x * kSortTile + (uint64_t)wid * (32 * kSortItems);
+  const uint64_t base = tile0 + (uint64_t)wid * (32 * kSortItems);
   const unsigned ltMask = (1u << lane) - 1;
   unsigned long long k[kSortItems];
   uint32_t v[kSortItems];
   uint32_t rank[kSortItems];
-  int      dig[kSortItems];
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
     uint64_t i = base + (uint64_t)it * 32 + lane;
     bool     ok = i < n;
     k[it]       = ok ? keysIn[i] : 0;
-    v[it]       = ok ? valsIn[i] : 0;
+    if (VALS) v[it] = ok ? valsIn[i] : 0;
   }
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
     const bool ok = base + (uint64_t)it * 32 + lane < n;
-    int d       = ok ? (int)((k[it] >> shift) & 0xff) : kDigits;
-    dig[it]     = d;
-    unsigned peers  = __match_any_sync(0xffffffffu, d);
-    int      leader = __ffs(peers) - 1;
-    uint32_t b      = 0;
-    if (lane == leader && ok) b = cnt[wid][d];
-    b         = __shfl_sync(0xffffffffu, b, leader);
-    rank[it]  = b + __popc(peers & ltMask);
+    const uint32_t d = (uint32_t)(k[it] >> shift) & 0xff;
+    unsigned peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+      const unsigned m = __ballot_sync(0xffffffffu, (d >> b) & 1);
+      peers &= (d >> b) & 1 ? m : ~m;
+    }
+    const uint32_t c = cnt[wid][d];
+    rank[it]  = c + __popc(peers & ltMask);
     __syncwarp();
-    if (lane == leader && ok) cnt[wid][d] = b + __popc(peers);
+    if (ok && (peers & ltMask) == 0) cnt[wid][d] = (uint16_t)(c + __popc(peers));
     __syncwarp();
   }
   __syncthreads();
   // Per digit: the warps' exclusive prefix, then the digit's start inside the tile.
-  uint32_t tot = 0;
-  {
-    const int d = threadIdx.x;   // kSortThreads == kDigits
-    uint32_t s = 0;
+  uint32_t s = 0, incl = 0;
+  const int d0 = threadIdx.x;
+  if (d0 < kDigits) {
 #pragma unroll
     for (int w = 0; w < kSortWarps; w++) {
-      uint32_t c = cnt[w][d];
-      cnt[w][d]  = s;
+      const uint32_t c = cnt[w][d0];
+      cnt[w][d0]       = (uint16_t)s;
       s += c;
     }
-    uint32_t all;
-    const uint32_t start = block_excl_scan(s, all);
-    localStart[d] = start;
+    incl = warp_incl_scan(s);
+    if (lane == 31) warpSums[wid] = incl;
+  }
+  __syncthreads();
+  if (d0 < kDigits) {
+    uint32_t start = incl - s;
+    for (int w = 0; w < wid; w++) start += warpSums[w];
 #pragma unroll
-    for (int w = 0; w < kSortWarps; w++) cnt[w][d] += start;
-    tot = all;
+    for (int w = 0; w < kSortWarps; w++) cnt[w][d0] = (uint16_t)(cnt[w][d0] + start);
+    tileBase[d0] = offsets[(uint64_t)d0 * nTiles + blockIdx.x] - start;   // ... minus its place in the tile
   }
   __syncthreads();
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
-    if (dig[it] < kDigits) {
-      const uint32_t p = cnt[wid][dig[it]] + rank[it];
+    if (base + (uint64_t)it * 32 + lane < n) {
+      const uint32_t p = cnt[wid][(uint32_t)(k[it] >> shift) & 0xff] + rank[it];
       sk[p] = k[it];
-      sv[p] = v[it];
+      if (VALS) sv[p] = v[it];
     }
   }
   __syncthreads();
-  for (uint32_t p = threadIdx.x; p < tot; p += kSortThreads) {
-    const unsigned long long key = sk[p];
-    const int d = (int)((key >> shift) & 0xff);
-    const uint64_t pos = (uint64_t)tileBase[d] + (p - localStart[d]);
-    keysOut[pos] = key;
-    valsOut[pos] = sv[p];
+  const uint32_t tot = (uint32_t)(n - tile0 < kSortTile ? n - tile0 : kSortTile);
+#pragma unroll
+  for (int it = 0; it < kSortItems; it++) {
+    const uint32_t p = it * kSortThreads + threadIdx.x;
+    if (p < tot) {
+      const unsigned long long key = sk[p];
+      const uint64_t pos = (uint64_t)(uint32_t)(tileBase[(uint32_t)(key >> shift) & 0xff] + p);
+      keysOut[pos] = key;
+      if (VALS) valsOut[pos] = sv[p];
+    }
   }
 }
 
-constexpr size_t kDownsweepDyn = (size_t)kSortTile * (sizeof(unsigned long long) + sizeof(uint32_t));
-static_assert(kSortThreads == kDigits && kSortThreads == kScanThreads, "one digit per thread in the downsweep");
+constexpr size_t kDownsweepKeys = (size_t)kSortTile * sizeof(unsigned long long);
+constexpr size_t kDownsweepDyn  = kDownsweepKeys + (size_t)kSortTile * sizeof(uint32_t);
 
 }  // namespace
 
@@ -259,27 +279,23 @@ cudaError_t radix_sort_u64_u32(unsigned long long *keys, uint32_t *vals, unsigne
   unsigned long long *ks = keys, *kd = keysAlt;
   uint32_t *vs = vals, *vd = valsAlt;
   int       passes = 0;
-  static bool attrSet = false;   // opt in to the downsweep's 48 KB of dynamic shared memory (per process)
-  if (!attrSet) {
-    cudaError_t e = cudaFuncSetAttribute(radix_downsweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kDownsweepDyn);
-    if (e != cudaSuccess) return e;
-    attrSet = true;
-  }
+  const size_t dyn = vals ? kDownsweepDyn : kDownsweepKeys;
+  auto down        = vals ? radix_downsweep_kernel<true> : radix_downsweep_kernel<false>;
+  cudaError_t e    = cudaFuncSetAttribute(down, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  if (e != cudaSuccess) return e;
   for (int shift = 0; shift < bits; shift += 8, passes++) {
-    radix_upsweep_kernel<<<(unsigned)nTiles, kSortThreads, 0, st>>>(ks, n, shift, hist, (uint32_t)nTiles, nDev);
+    radix_upsweep_kernel<<<(unsigned)nTiles, kUpThreads, 0, st>>>(ks, n, shift, hist, (uint32_t)nTiles, nDev);
     g_launches++;
-    cudaError_t e = scan_u32(hist, hist, nh, nullptr, scanSc, st);
+    e = scan_u32(hist, hist, nh, nullptr, scanSc, st);
     if (e != cudaSuccess) return e;
-    radix_downsweep_kernel<<<(unsigned)nTiles, kSortThreads, kDownsweepDyn, st>>>(ks, vs, kd, vd, n, shift, hist,
-                                                                                   (uint32_t)nTiles, nDev);
+    down<<<(unsigned)nTiles, kSortThreads, dyn, st>>>(ks, vs, kd, vd, n, shift, hist, (uint32_t)nTiles, nDev);
     g_launches++;
     unsigned long long *tk = ks; ks = kd; kd = tk;
     uint32_t *tv = vs; vs = vd; vd = tv;
   }
   if (ks != keys) {
     cudaMemcpyAsync(keys, ks, n * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(vals, vs, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
+    if (vals) cudaMemcpyAsync(vals, vs, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
   }
   return cudaGetLastError();
 }
