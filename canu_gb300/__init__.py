@@ -365,15 +365,17 @@ class Overlapper:
         """Canonical k-mers of reads [bgn, end] seen at least min_count times:
         (list of k-mer strings, uint32 counts), ascending canonical 2-bit key."""
         n = ctypes.c_uint64()
-        rc = self._lib.oic_count_kmers(self._ctx, bgn, end, min_count, None, None, 0, ctypes.byref(n))
-        if rc not in (OIC_OK, OIC_ERR_OVERFLOW):
-            self._check(rc)
         k = self.params.kmerLen
-        buf = np.zeros(n.value * k, dtype=np.uint8)
-        cnt = np.zeros(n.value, dtype=np.uint32)
-        if n.value:
-            self._check(self._lib.oic_count_kmers(self._ctx, bgn, end, min_count, _ptr(buf), _ptr(cnt), n.value,
-                                                  ctypes.byref(n)))
+        room = 1 << 18   # a skip list's size; a longer list is counted again with room for it
+        while True:
+            buf = np.empty(room * k, dtype=np.uint8)
+            cnt = np.empty(room, dtype=np.uint32)
+            rc = self._lib.oic_count_kmers(self._ctx, bgn, end, min_count, _ptr(buf), _ptr(cnt), room, ctypes.byref(n))
+            if rc != OIC_ERR_OVERFLOW or n.value <= room:
+                break
+            room = n.value
+        self._check(rc)
+        buf, cnt = buf[: n.value * k], cnt[: n.value].copy()
         s = buf.tobytes().decode()
         return [s[i * k:(i + 1) * k] for i in range(n.value)], cnt
 

@@ -1909,9 +1909,9 @@ int oic_count_kmers(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t minCo
   *nKmers = 0;
   if (n == 0) return OIC_OK;
   const uint32_t nr = (uint32_t)reads.size();
-  DevBuf dReads, dHist, dK, dV, dK2, dV2, dScr, dFlags, dPos, dRun, dSel, dSelPos, dOutK, dOutC;
+  DevBuf dReads, dHist, dK, dK2, dScr, dFlags, dPos, dRun, dSel, dSelPos, dOutK, dOutC;
   auto release = [&]() {
-    for (DevBuf *b : {&dReads, &dHist, &dK, &dV, &dK2, &dV2, &dScr, &dFlags, &dPos, &dRun, &dSel, &dSelPos, &dOutK, &dOutC})
+    for (DevBuf *b : {&dReads, &dHist, &dK, &dK2, &dScr, &dFlags, &dPos, &dRun, &dSel, &dSelPos, &dOutK, &dOutC})
       b->release();
   };
   int  rc   = OIC_OK;
@@ -1958,7 +1958,7 @@ int oic_count_kmers(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t minCo
   std::vector<uint64_t> outKeys;
   std::vector<uint32_t> outCounts;
   if (!rc && m &&
-      !(step(dK.ensure(m * 8)) && step(dV.ensure(m * 4)) && step(dK2.ensure(m * 8)) && step(dV2.ensure(m * 4)) &&
+      !(step(dK.ensure(m * 8)) && step(dK2.ensure(m * 8)) &&
         step(dScr.ensure(std::max(radix_sort_scratch(m), scan_u32_scratch(m)) + 256)) && step(dFlags.ensure(m * 4)) &&
         step(dPos.ensure(m * 4))))
     rc = rc ? rc : OIC_ERR_NOMEM;
@@ -1966,13 +1966,12 @@ int oic_count_kmers(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t minCo
     unsigned long long nPass = 0;
     if (!step(cudaMemsetAsync(ctr64(ctx) + kCellsSnap, 0, 8, ctx->st))) break;
     launch_canon_emit_part(ctx->R, dReads.as<uint32_t>(), nr, K, shift, passes[pi].first, passes[pi].second,
-                           dK.as<u64>(), dV.as<uint32_t>(), ctr64(ctx) + kCellsSnap, ctx->st);
+                           dK.as<u64>(), ctr64(ctx) + kCellsSnap, ctx->st);
     if (!step(cudaMemcpyAsync(&nPass, ctr64(ctx) + kCellsSnap, 8, cudaMemcpyDeviceToHost, ctx->st)) ||
         (rc = sync_check(ctx, "k-mer emission")))
       break;
     if (!nPass) continue;
-    if (!step(radix_sort_u64_u32(dK.as<u64>(), dV.as<uint32_t>(), dK2.as<u64>(), dV2.as<uint32_t>(), nPass, 2 * K,
-                                 dScr.p, ctx->st)))
+    if (!step(radix_sort_u64_u32(dK.as<u64>(), nullptr, dK2.as<u64>(), nullptr, nPass, 2 * K, dScr.p, ctx->st)))
       break;
     uint32_t nRuns = 0, nSel = 0;
     launch_run_starts(dK.as<u64>(), nPass, dFlags.as<uint32_t>(), ctx->st);
