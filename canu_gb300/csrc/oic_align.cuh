@@ -268,15 +268,22 @@ struct RowsOut {
 // Several warps of one CTA on one pair (the wide bins): warp 0 runs the pair logic and
 // hands each extension's row loop to the whole CTA through GroupShared.
 struct GroupJob {
-  SeqView A, T;
-  int     a0, t0;
-  int     m, n, errorLimit, u;
-  int    *rowA, *rowB;       // row buffers (rowA holds row 0)
+  SeqView    A, T;
+  int        a0, t0;
+  int        m, n, errorLimit, u;
+  int       *rowA, *rowB;    // row buffers (rowA holds row 0), bufW ints each
+  int       *rowsG;          // HBM row buffers, rowsGW ints each
+  int       *arena;
+  int4      *rowHdr;
+  const int *eml;
+  int        bufW, rowsGW, arenaCap, rowCap;
 };
 struct GroupShared {
-  GroupJob job;
-  int      cmd;              // kGroupRows or kGroupExit, posted by warp 0 before barrier 1
-  int      red[32][4];       // per-warp partial reductions of a row
+  __align__(16) int  red[2][32][4];   // per-warp partial reductions of a row, by its parity
+  GroupJob           job;
+  RowsOut            out;             // the row loop's result
+  unsigned long long slides;          // slide bases of the CTA's row loops
+  int                cmd;             // kGroupRows or kGroupExit, posted by warp 0 before barrier 1
 };
 enum { kGroupRows = 1, kGroupExit = 2 };
 
@@ -663,148 +670,185 @@ static __device__ __noinline__ bool no_path_within(WarpDP &w, const ReadView &Sr
 }
 
 // The row loop by every thread of the CTA (nThr threads, tid = threadIdx.x).  Thread t
-// takes U consecutive diagonals per pass, d0 = Lc + U*t + U*nThr*k, so the U+2
-// neighbour values of row e-1 are read once for U cells and U slides are in flight.
+// takes diagonals Lc + t, Lc + t + nThr, ..., U of them per pass, their loads together.
 // Every decision is made on CTA-reduced values, so all threads take the same path and
 // meet the same barriers.
-template <int U>
-static __device__ __noinline__ RowsOut group_rows(const GroupJob &j, const WarpScratch &sc, const AlignCaps &cap,
-                                                  const int *eml, int tid, int nThr, int (*red)[4],
-                                                  unsigned long long &slides) {
-  const int lane = tid & 31, wid = tid >> 5, nW = nThr >> 5;
-  const SeqView A = j.A, T = j.T;   // in registers for the slides
-  const int     a0 = j.a0, t0 = j.t0;
-  const int     m = j.m, n = j.n;
-  RowsOut o;
-  o.status = kRowsDone;
-  o.err = 0;
-  o.e = o.dEnd = o.eDone = o.Rc = o.rowEnd = o.ppEnd = 0;
-  o.cells = o.rows = 0;
-  // Every thread has read the job before warp 0 can post the next one.
-  group_bar(2, nThr);
-  int *prev = j.rowA, *cur = j.rowB;
-  int  bufW = cap.bandW;
-  int  used = 1, prevBase = 0, L = 0, R = 0;
-  for (int e = 1; e <= j.errorLimit; e++) {
-    if (e >= cap.rowCap) { o.status = kRowsErr; o.err = kErrRowsFull; break; }
+//
+// What bounds it is the latency of a row: shared-memory loads, the windows, a barrier and
+// the reduction behind it.  One barrier per row: the partial reductions go to slots of the
+// row's parity, neighbours outside the kept band are masked instead of overwritten, and the
+// kept band goes to the arena (with its largest value to the header) while the next row
+// reads it, as in row_loop.  A batch of 230 extensions of 60 kb reads with 4 % errors took
+// 39.6 ms with a sentinel write, a copy of the kept band and four barriers per row (and
+// one-warp rows in HBM first, for bands that end up here), 26.3 ms with one barrier, 19.4 ms
+// with the job read from shared memory, 14.2 ms with 512 threads instead of 256.  Two CTAs
+// of 512 threads per SM (64 registers) spill: 18.0 ms.
+template <int U, bool HASN>
+static __device__ __noinline__ void group_rows(GroupShared &gs, const int tid, const int nThr) {
+  const int lane = tid & 31, wid = tid >> 5;
+  const GroupJob &j = gs.job;
+  // The planes in registers for the slides (N masks are read from the job when needed).
+  const uint2 *const Ap = j.A.p + 0, *const Tp = j.T.p + 0;
+  const int a0 = j.a0, t0 = j.t0, m = j.m, n = j.n, errorLimit = j.errorLimit;
+  const int arenaCap = j.arenaCap, rowCap = j.rowCap;
+  int4 *const rowHdr = j.rowHdr;
+  int  *const arena  = j.arena;
+  const int *const eml = j.eml;
+  __builtin_assume(__isGlobal(rowHdr));
+  __builtin_assume(__isGlobal(arena));
+  __builtin_assume(__isGlobal(eml));
+  int *prev = j.rowA, *cur = j.rowB;   // diagonal d at index d - base + 2
+  int  bufW = j.bufW;
+  int  off = 0, base = 0, L = 0, R = 0;
+  int  lim = errorLimit >= 1 ? eml[1] : 0;
+  int  e = 1, status = kRowsDone;
+  u32  err = 0, cells = 0, slides = 0;
+  for (; e <= errorLimit; e++) {
+    if (e >= rowCap) { status = kRowsErr; err = kErrRowsFull; break; }
+    if (off + (R - L + 1) > arenaCap) { status = kRowsErr; err = kErrArenaFull; break; }
     const int Lc = max(L - 1, -e), Rc = min(R + 1, e);
     const int width = Rc - Lc + 1;
     if (width + 4 > bufW) {
-      if (bufW == cap.rowsGW || width + 4 > cap.rowsGW || !sc.rowsG) { o.status = kRowsErr; o.err = kErrBandWide; break; }
-      int *gA = sc.rowsG, *gB = sc.rowsG + cap.rowsGW;
-      for (int i = tid; i < bufW; i += nThr) gA[i] = prev[i];
+      int *const rowsG = j.rowsG;
+      const int  gw    = j.rowsGW;
+      if (bufW == gw || width + 4 > gw || !rowsG) { status = kRowsErr; err = kErrBandWide; break; }
+      for (int i = tid; i < bufW; i += nThr) rowsG[i] = prev[i];
       group_bar(2, nThr);
-      prev = gA;
-      cur  = gB;
-      bufW = cap.rowsGW;
+      prev = rowsG;
+      cur  = rowsG + gw;
+      bufW = gw;
     }
-    const int lim = eml[e];
-    if (tid < 4) prev[(tid < 2 ? L - 2 + tid : R - 1 + tid) - prevBase + 2] = -2;
-    group_bar(2, nThr);
-    const int *pv = prev + (2 - prevBase);
-    int       *cv = cur + (2 - Lc);
-    int myEnd = INT_MAX, myL = INT_MAX, myR = INT_MIN;
-    for (int d0 = Lc + tid * U; d0 <= Rc; d0 += nThr * U) {
-      int q[U + 2];   // row e-1 at d0-1 .. d0+U
-#pragma unroll
-      for (int k = 0; k < U + 2; k++) q[k] = (d0 - 1 + k <= Rc + 1) ? pv[d0 - 1 + k] : -2;
+    const int limNext = e < errorLimit ? eml[e + 1] : 0;
+    int myEnd = INT_MAX, myL = INT_MAX, myR = INT_MIN, prevMax = -1;
+    for (int c = Lc + tid; c <= Rc; c += nThr * U) {
+      int row[U];
 #pragma unroll
       for (int k = 0; k < U; k++) {
-        const int d = d0 + k;
+        const int d = c + k * nThr;
         if (d <= Rc) {
-          int row = 1 + q[k + 1];
-          if (q[k] > row) row = q[k];
-          if (1 + q[k + 2] > row) row = 1 + q[k + 2];
-          const int room = min(m - row, n - row - d);
-          if (room > 0) row += slide(A, a0, T, t0, row, d, room, slides);
-          cv[d] = row;
-          if ((row == m || row + d == n) && d < myEnd) myEnd = d;
-          if (!(row + max(d, 0) < lim)) {
-            if (myL == INT_MAX) myL = d;
+          // Row e-1 at d - 1, d, d + 1; -2 outside its kept band (forward.C:150-153).
+          const int *pv = prev + (2 - base) + d;
+          const int  pm = d > L ? pv[-1] : -2, p0 = d >= L && d <= R ? pv[0] : -2, pp = d < R ? pv[1] : -2;
+          if (d >= L && d <= R) arena[off - L + d] = p0;
+          prevMax = max(prevMax, p0);
+          row[k]  = max(max(p0, pp) + 1, pm);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int d = c + k * nThr;
+        if (d <= Rc) {
+          const int z = min(m, n - d);   // where the nearer end is
+          int r = row[k];
+          while (r < z) {
+            const uint2 x = load_planes(Ap, a0 + r), y = load_planes(Tp, t0 + d + r);
+            u32 mk = (x.x ^ y.x) | (x.y ^ y.y);
+            if (HASN) mk = drop_n(mk, j.A.nm, a0 + r, j.T.nm, t0 + d + r);
+            r += __clz((int)mk);
+            if (mk) break;
+          }
+          r = min(r, z);
+          slides += (u32)(r - row[k]);
+          cur[2 - Lc + d] = r;
+          if (r == z) myEnd = min(myEnd, d);
+          // pruneAlign (prefixEditDistance.H:249-258): extra = max(d, 0) on both band edges
+          if (r + max(d, 0) >= lim) {
+            myL = min(myL, d);
             myR = d;
           }
         }
       }
     }
+    int (*const slot)[4] = gs.red[e & 1];
     {
       const int wEnd = __reduce_min_sync(0xffffffffu, myEnd);
       const int wL   = __reduce_min_sync(0xffffffffu, myL);
       const int wR   = __reduce_max_sync(0xffffffffu, myR);
-      if (lane == 0) {
-        red[wid][0] = wEnd;
-        red[wid][1] = wL;
-        red[wid][2] = wR;
-      }
+      const int wV   = __reduce_max_sync(0xffffffffu, prevMax);
+      if (lane == 0) *(int4 *)slot[wid] = make_int4(wEnd, wL, wR, wV);
     }
     group_bar(2, nThr);
-    int dEnd = INT_MAX, L2 = INT_MAX, R2 = INT_MIN;
-    for (int i = 0; i < nW; i++) {
-      dEnd = min(dEnd, red[i][0]);
-      L2   = min(L2, red[i][1]);
-      R2   = max(R2, red[i][2]);
-    }
-    o.rows++;
+    // Every warp reduces the warps' results: lane i takes warp i's.
+    int4 w = make_int4(INT_MAX, INT_MAX, INT_MIN, -1);
+    if (lane < nThr >> 5) w = *(const int4 *)slot[lane];
+    const int dEnd = __reduce_min_sync(0xffffffffu, w.x);
+    const int L2   = __reduce_min_sync(0xffffffffu, w.y);
+    const int R2   = __reduce_max_sync(0xffffffffu, w.z);
+    prevMax        = __reduce_max_sync(0xffffffffu, w.w);
+    // Row e-1's header, with its largest value (forward.C:284-289) for max_score_rows.
+    if (tid == 0) rowHdr[e - 1] = make_int4(off, L, R, prevMax);
     if (dEnd != INT_MAX) {
-      o.cells += (unsigned long long)(dEnd - Lc + 1);
-      o.status   = kRowsEnd;
-      o.e        = e;
-      o.dEnd     = dEnd;
-      o.Rc       = Rc;
-      o.rowEnd   = cv[dEnd];
-      o.ppEnd    = pv[dEnd + 1];
+      cells += (u32)(dEnd - Lc + 1);
+      status = kRowsEnd;
+      if (tid == 0) {
+        gs.out.dEnd   = dEnd;
+        gs.out.Rc     = Rc;
+        gs.out.rowEnd = cur[2 - Lc + dEnd];
+        gs.out.ppEnd  = dEnd < R ? prev[2 - base + dEnd + 1] : -2;
+      }
       break;
     }
-    o.cells += (unsigned long long)width;
+    cells += (u32)width;
     if (L2 == INT_MAX) break;
-
-    // Keep the band for the traceback and take its largest value on the way.
-    const int cnt = R2 - L2 + 1;
-    if (used + cnt > cap.arenaCap) { o.status = kRowsErr; o.err = kErrArenaFull; break; }
-    int myV = -1;
-    for (int d = L2 + tid; d <= R2; d += nThr) {
-      const int v = cv[d];
-      myV         = max(myV, v);
-      sc.arena[used + d - L2] = v;
-    }
-    {
-      const int wV = __reduce_max_sync(0xffffffffu, myV);
-      if (lane == 0) red[wid][3] = wV;
-    }
-    group_bar(2, nThr);
-    int rowMax = -1;
-    for (int i = 0; i < nW; i++) rowMax = max(rowMax, red[i][3]);
-    if (tid == 0) sc.rowHdr[e] = make_int4(used, L2, R2, rowMax);
-    used += cnt;
+    off += R - L + 1;
     int *t = prev;
     prev   = cur;
     cur    = t;
-    prevBase = Lc;
-    L        = L2;
-    R        = R2;
-    o.eDone  = e;
-    group_bar(2, nThr);
+    base   = Lc;
+    L      = L2;
+    R      = R2;
+    lim    = limNext;
   }
-  return o;
+  if (e > errorLimit) {
+    // The error limit: the last row has not been kept yet.
+    if (off + (R - L + 1) > arenaCap) {
+      status = kRowsErr;
+      err    = kErrArenaFull;
+    } else {
+      int prevMax = -1;
+      for (int d = L + tid; d <= R; d += nThr) {
+        const int v = prev[2 - base + d];
+        arena[off + d - L] = v;
+        prevMax            = max(prevMax, v);
+      }
+      prevMax = __reduce_max_sync(0xffffffffu, prevMax);
+      if (lane == 0) gs.red[e & 1][wid][3] = prevMax;
+      group_bar(2, nThr);
+      for (int i = 0; i < nThr >> 5; i++) prevMax = max(prevMax, gs.red[e & 1][i][3]);
+      if (tid == 0) rowHdr[errorLimit] = make_int4(off, L, R, prevMax);
+    }
+  }
+  const unsigned long long sl = warp_sum64(slides);
+  if (lane == 0) atomicAdd(&gs.slides, sl);
+  if (tid == 0) {
+    gs.out.status = status;
+    gs.out.err    = err;
+    gs.out.e      = e;
+    gs.out.eDone  = e - 1;   // rows below e are kept
+    gs.out.cells  = cells;
+    gs.out.rows   = (unsigned)(e <= errorLimit && status != kRowsErr ? e : e - 1);
+  }
+  // Warp 0 goes on alone with the arena and the buffers: everything has been written.
+  __threadfence_block();
+  group_bar(2, nThr);
 }
 
-// The job a GroupJob names, with its compile-time tile.
-static __device__ __forceinline__ RowsOut group_rows_any(const GroupJob &j, const WarpScratch &sc,
-                                                         const AlignCaps &cap, const int *eml, int tid, int nThr,
-                                                         int (*red)[4], unsigned long long &slides) {
-  if (j.u == 4) return group_rows<4>(j, sc, cap, eml, tid, nThr, red, slides);
-  if (j.u == 2) return group_rows<2>(j, sc, cap, eml, tid, nThr, red, slides);
-  return group_rows<1>(j, sc, cap, eml, tid, nThr, red, slides);
+// The posted job, with its compile-time tile.
+static __device__ __forceinline__ void group_rows_any(GroupShared &gs, int tid, int nThr) {
+  const bool hasN = gs.job.A.nm || gs.job.T.nm;
+  const int  u    = gs.job.u;
+  if (hasN) group_rows<1, true>(gs, tid, nThr);
+  else if (u == 4) group_rows<4, false>(gs, tid, nThr);
+  else if (u == 2) group_rows<2, false>(gs, tid, nThr);
+  else group_rows<1, false>(gs, tid, nThr);
 }
 
 // Worker warps of a group CTA: run the row loops warp 0 posts until it posts exit.
-static __device__ __noinline__ void group_worker(GroupShared &gs, const WarpScratch &sc, const AlignCaps &cap,
-                                                 const int *eml, unsigned long long &slides) {
-  const int tid = threadIdx.x, nThr = blockDim.x;
+static __device__ __noinline__ void group_worker(GroupShared &gs) {
   while (true) {
-    group_bar(1, nThr);
+    group_bar(1, blockDim.x);
     if (gs.cmd != kGroupRows) break;
-    const GroupJob j = gs.job;
-    group_rows_any(j, sc, cap, eml, tid, nThr, gs.red, slides);
+    group_rows_any(gs, threadIdx.x, blockDim.x);
   }
 }
 
@@ -835,9 +879,7 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const int step, con
   RowsOut o;
   if (GROUP) {
     if (lane == 0) {
-      w.sc.arena[0]  = r0;
-      w.sc.rowHdr[0] = make_int4(0, 0, 0, 0);
-      w.smA[2]       = r0;
+      w.smA[2]     = r0;
       GroupJob &j  = w.gs->job;
       j.A          = A;
       j.T          = T;
@@ -849,12 +891,20 @@ static __device__ __noinline__ int warp_prefix_dp(WarpDP &w, const int step, con
       j.u          = w.gU;
       j.rowA       = w.smA;
       j.rowB       = w.smB;
+      j.rowsG      = w.sc.rowsG;
+      j.arena      = w.sc.arena;
+      j.rowHdr     = w.sc.rowHdr;
+      j.eml        = w.eml;
+      j.bufW       = w.cap.bandW;
+      j.rowsGW     = w.cap.rowsGW;
+      j.arenaCap   = w.cap.arenaCap;
+      j.rowCap     = w.cap.rowCap;
       w.gs->cmd    = kGroupRows;
     }
     __syncwarp();
     group_bar(1, w.gThreads);
-    const GroupJob j = w.gs->job;
-    o = group_rows_any(j, w.sc, w.cap, w.eml, lane, w.gThreads, w.gs->red, w.slides);
+    group_rows_any(*w.gs, lane, w.gThreads);
+    o = w.gs->out;
   } else {
     warp_rows(w, o, A, a0, m, T, t0, n, errorLimit, r0);
   }

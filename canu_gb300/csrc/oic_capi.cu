@@ -383,7 +383,8 @@ oic_tuning resolved_tuning(const oic_ctx *c) {
   if (!t.narrowArena) t.narrowArena = 1u << 20;
   if (!t.wideMinLen) t.wideMinLen = 0xffffffffu;
   if (t.forceWide) t.wideMinLen = 0;
-  if (!t.wideThreads) t.wideThreads = 256;
+  // 128 / 256 / 512 threads: 27.9 / 19.4 / 14.2 ms for 230 extensions of 60 kb noisy reads.
+  if (!t.wideThreads) t.wideThreads = 512;
   if (!t.wideTile) t.wideTile = 1;
   if (!t.wideBandW) t.wideBandW = 12288;
   if (!t.wideCtas) t.wideCtas = resolved_tuning_ctas(c, t);
@@ -1807,6 +1808,7 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
     if (pass == 0) {
       AlignConfig ac = align_normal(ctx);
       ac.caps.arenaCap = (int)tn.narrowArena;
+      ac.caps.rowsGW   = ac.caps.bandW;   // a band wider than the shared-memory rows is the CTA's
       WarpScratch ws;
       if ((rc = ensure_align_scratch(ctx, ac, false, ws))) break;
       launch_extend_batch(ctx->R, ctx->dp, ctx->dEml.as<int>(), dP.as<ExtendProblem>(), nAlign, ws,

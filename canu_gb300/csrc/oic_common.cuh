@@ -139,20 +139,6 @@ __device__ __forceinline__ int match_run32(const SeqView &A, int a, const SeqVie
   return __clz((int)m);
 }
 
-// Bases that agree from A[row] / T[row+d] on, capped at `lim` (> 0).
-__device__ __forceinline__ int slide(const SeqView &A, int a0, const SeqView &T, int t0, int row, int d, int lim,
-                                     unsigned long long &slides) {
-  int run = 0;
-  while (run < lim) {
-    const int r = match_run32(A, a0 + row + run, T, t0 + row + d + run);
-    run += r;
-    if (r < 32) break;
-  }
-  if (run > lim) run = lim;
-  slides += (unsigned long long)run;
-  return run;
-}
-
 __device__ __forceinline__ u64 mix64(u64 x) {
   x ^= x >> 33;
   x *= 0xff51afd7ed558ccdull;

@@ -78,11 +78,10 @@ static __global__ void __launch_bounds__(512, 1) extend_group_kernel(ReadsDev R,
                                                                       unsigned long long *stats, int U) {
   __shared__ GroupShared gs;
   const WarpScratch sc = warp_scratch(scBase, cap, blockIdx.x);
+  if (threadIdx.x == 0) gs.slides = 0;
+  __syncthreads();
   if (threadIdx.x >= 32) {
-    unsigned long long slides = 0;
-    group_worker(gs, sc, cap, eml, slides);
-    slides = warp_sum64(slides);
-    if ((threadIdx.x & 31) == 0 && slides) atomicAdd(&stats[1], slides);
+    group_worker(gs);
     return;
   }
   WarpDP w;
@@ -94,7 +93,7 @@ static __global__ void __launch_bounds__(512, 1) extend_group_kernel(ReadsDev R,
   const unsigned long long slidesWarp = warp_sum64(w.slides);
   if (threadIdx.x == 0) {
     atomicAdd(&stats[0], w.cells);
-    atomicAdd(&stats[1], slidesWarp);
+    atomicAdd(&stats[1], slidesWarp + gs.slides);
     gs.cmd = kGroupExit;
   }
   __syncwarp();

@@ -866,11 +866,10 @@ __global__ void __launch_bounds__(512, 1) align_group_kernel(ReadsDev R, TableDe
   __shared__ PairSmem    pairSmem;
   __shared__ GroupShared gs;
   const WarpScratch sc = warp_scratch(scBase, cap, blockIdx.x);
+  if (threadIdx.x == 0) gs.slides = 0;
+  __syncthreads();
   if (threadIdx.x >= 32) {
-    unsigned long long slides = 0;
-    group_worker(gs, sc, cap, eml, slides);
-    slides = warp_sum64(slides);
-    if ((threadIdx.x & 31) == 0 && slides) atomicAdd(&out.stats[kStSlides], slides);
+    group_worker(gs);
     return;
   }
   WarpDP w;
@@ -879,7 +878,10 @@ __global__ void __launch_bounds__(512, 1) align_group_kernel(ReadsDev R, TableDe
   w.gThreads = blockDim.x;
   w.gU       = U;
   align_loop<true>(w, pairSmem, R, Tb, pairs, work, nWork, workCounter, nodes, out);
-  if (threadIdx.x == 0) gs.cmd = kGroupExit;
+  if (threadIdx.x == 0) {
+    gs.cmd = kGroupExit;
+    if (gs.slides) atomicAdd(&out.stats[kStSlides], gs.slides);
+  }
   __syncwarp();
   group_bar(1, blockDim.x);
 }
