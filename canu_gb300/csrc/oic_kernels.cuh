@@ -53,10 +53,10 @@ struct PairRec {
   u32 flags;      // bit0 reverse strand, bit1 consistent, bit2 S left-end screened, bit3 S right-end screened
 };
 
-struct PairAcc {   // seed-replay state of one pair
-  u32 T;
+struct alignas(16) PairAcc {   // seed-replay state of one pair; the replay reads and writes the first 16 bytes
   int head;
   int diagCt, diagBgn, diagEnd;
+  u32 T;
   int consistent;
   int slot;
   int pad;

@@ -18,22 +18,28 @@
 // live in the CTA's HBM scratch; a warp finds the partners it has seen lately in a small
 // shared-memory table, and a lane keeps its pair's newest run in registers.
 //
+// A buffer meets two barriers: one when its owners are counted (by then every warp has
+// replayed the seeds before), one when its seeds are in place.  A warp lays out consecutive
+// chunks of 32 seeds, so that the counts are 8 x 8 and each warp scans them for itself, and
+// it finds the offsets of 32 consecutive seeds with one vote: the ends of the next 32
+// offsets, which are all different, as bits of a word.
+//
 // What bounds it is latency: a lookup, its occurrences, the pair, its newest run, one after
-// another, and the warps of a CTA waiting for the one with most seeds (half of the stall
-// cycles).  A strand on one warp took 11 ms for 8 kb and 25 ms for 15 kb, whatever else ran;
-// eight warps and one step per run of seeds bring that to 4 and 7 ms.  With many strands
-// (150 Mbp, 1.8 G seeds) the stage went from 53 to 46 ms: 760 to 1,216 strands in flight
-// keep their pairs and runs in L2 where 4,864 did not (37 B of HBM per seed, from 55), and
-// a seed costs 19 warp instructions.  5 / 6 / 8 CTAs per SM: 53 / 49 / 46 ms.  Seeds one by
-// one in the lane loop: 122 ms.  Dealing partners to the warps in order of appearance
-// instead of by hash, or laying the seeds out by offset instead of by a search per seed,
-// changed less than the spread.
+// another, and the warps of a CTA waiting for the slowest (two fifths of the stall cycles).
+// A strand on one warp took 11 ms for 8 kb and 25 ms for 15 kb, whatever else ran; eight
+// warps and one step per run of seeds bring that to 4 and 7 ms.  With many strands
+// (150 Mbp, 1.8 G seeds) the stage went from 53 ms (a warp per strand) to 46 and, with two
+// barriers per buffer in place of five, the vote in place of a search per seed, and a
+// binary search in place of a scan of the occurrences, to 36.5 ms, of which 26 are the
+// lookups and the laying out.  760 to 1,216 strands in flight keep their pairs and runs in
+// L2 where 4,864 did not.  5 / 6 / 7 / 8 CTAs per SM: 43.7 / 40.3 / 38.8 / 36.5 ms; a
+// buffer of 512 seeds 38.3.  Seeds one by one in the lane loop: 122 ms (of 46).  Fetching
+// the next offsets' table slots ahead of the replay: 39.6.  Dealing partners to the warps in
+// order of appearance instead of by hash changed less than the spread.
 //
 // A table probe is one 16-byte load of a (key, value) slot.  The qualifying
 // occurrences of a k-mer (partner ID above the ref read's) are the tail of its run,
-// which ascends by partner: runs of up to kScanMax entries are counted by a backward
-// scan, eight entries per step -- the entries the replay reads next -- and longer runs
-// by binary search.
+// which ascends by partner.
 #include "oic_kernels.cuh"
 #include "oic_prims.cuh"
 
@@ -44,23 +50,25 @@ namespace {
 constexpr int kSeedThreads = 256;
 constexpr int kSeedCtas    = 8;      // CTAs per SM
 constexpr int kSeedWarps   = kSeedThreads / 32;
-constexpr int kScanMax     = 64;     // occurrence runs up to this long are scanned backwards
 constexpr int kSeedBuf     = 1024;   // seeds laid out at a time
-constexpr int kSeedPer     = kSeedBuf / kSeedThreads;
-constexpr int kSeedChunks  = kSeedBuf / 32;
-static_assert(kSeedChunks == 32 && kSeedWarps == 8, "one lane per chunk; owners have three bits");
+constexpr int kSeedPer     = kSeedBuf / kSeedThreads;   // 32-seed chunks a warp lays out
+static_assert(kSeedWarps == 8 && 32 * kSeedPer <= 256, "owners have three bits, ranks a byte");
+constexpr int kOffBits     = 24;     // a packed seed: the ref offset above its 256, the partner's offset below
+static_assert(kSeedThreads <= 256 && kMaxReadLenBits <= kOffBits, "both offsets share a word");
 constexpr int kSeedRecent  = 64;     // recently seen partners per warp
 
 struct SeedSmem {
   u64 recent[kSeedWarps][kSeedRecent];   // partner << 32 | pair index (all ones: none)
-  u32 tStr[kSeedBuf];                    // the seeds: partner, its offset, the ref strand's offset
-  int tOff[kSeedBuf];
-  int sOff[kSeedBuf];
-  u32 incl[kSeedThreads];                // inclusive scan of the offsets' seed counts
-  u32 qEnd[kSeedThreads];
-  unsigned short cnt[kSeedWarps][kSeedChunks];   // seeds of a warp in 32 consecutive ones, then their places
-  u32 part[kSeedWarps];                  // seeds of a warp in the buffer
-  u32 warpSum[kSeedWarps];
+  u32 tStr[kSeedBuf];                    // the seeds: partner, packed offsets
+  u32 off[kSeedBuf];
+  // The offsets with seeds, in order: seeds up to and with this offset, the place of its seed 0
+  // in the occurrence array plus the seeds before it, and the offset.
+  u32 end[kSeedThreads];
+  u32 from[kSeedThreads];
+  unsigned char at[kSeedThreads];
+  u32 cnt[kSeedWarps][kSeedWarps / 2];   // seeds per owner and laying warp, two warps to a word
+  u32 warpSum[2][kSeedWarps];
+  u32 warpCnt[2][kSeedWarps];
   u32 seg;
   u32 base[2];                           // output places of the strand's nodes and pairs
   int nPairs, nNodes, overflow, screened;
@@ -122,12 +130,12 @@ __device__ __forceinline__ u32 block_incl_scan(SeedSmem &sm, u32 v, u32 &total) 
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const u32 inc = warp_incl_scan_u32(v);
   __syncthreads();
-  if (lane == 31) sm.warpSum[wib] = inc;
+  if (lane == 31) sm.warpSum[0][wib] = inc;
   __syncthreads();
   u32 before = 0, all = 0;
 #pragma unroll
   for (int w = 0; w < kSeedWarps; w++) {
-    const u32 x = sm.warpSum[w];
+    const u32 x = sm.warpSum[0][w];
     before += w < wib ? x : 0;
     all += x;
   }
@@ -137,22 +145,23 @@ __device__ __forceinline__ u32 block_incl_scan(SeedSmem &sm, u32 v, u32 &total) 
 
 // Replays the seeds of one round (lane's seed at place `at` of the buffer, -1: none).
 __device__ __forceinline__ void replay_round(SeedSmem &sm, const SeedCaps &cap, int *slotKey, int *slotVal,
-                                             PairAcc *pairs, int4 *nodes, int at, int K) {
+                                             PairAcc *pairs, int4 *nodes, int at, int i0, int K) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const u32 tStr = at >= 0 ? sm.tStr[at] : (0x80000000u | lane);
-  const int myS  = at >= 0 ? sm.sOff[at] : 0, myT = at >= 0 ? sm.tOff[at] : 0;
+  const u32 off  = at >= 0 ? sm.off[at] : 0;
   const unsigned peers = __match_any_sync(0xffffffffu, tStr);
   // Seeds that follow their predecessor in the group: next offset, same diagonal.
   const unsigned before = peers & ((1u << lane) - 1);
   const int      pl = before ? 31 - __clz((int)before) : lane;
-  const int      ps = __shfl_sync(0xffffffffu, myS, pl), pt = __shfl_sync(0xffffffffu, myT, pl);
-  const unsigned follows = __ballot_sync(0xffffffffu, before && myS == ps + 1 && myT == pt + 1);
+  const u32      po = __shfl_sync(0xffffffffu, off, pl);
+  const unsigned follows = __ballot_sync(0xffffffffu, before && off == po + (1u << kOffBits) + 1);
   const int  at0  = at - lane;   // lane 0's place: the round's seeds are consecutive
   const bool lead = at >= 0 && before == 0 && !*(volatile int *)&sm.overflow;
   if (lead) {
     // Find or create the pair (Add_Ref, Find_Overlaps.C:104-150).
-    const u32 h = (u32)(mix64(tStr));
-    u64 &rec    = sm.recent[wib][(h >> 16) & (kSeedRecent - 1)];
+    u32 h = tStr * 0x9e3779b1u;
+    h ^= h >> 15;
+    u64 &rec    = sm.recent[wib][(h >> 4) & (kSeedRecent - 1)];
     const u64 r = rec;
     int pi      = (u32)(r >> 32) == tStr ? (int)(u32)r : -1;
     if (pi < 0) {
@@ -186,65 +195,65 @@ __device__ __forceinline__ void replay_round(SeedSmem &sm, const SeedCaps &cap, 
     }
     if (pi < 0) sm.overflow = 1;
     else {
-      PairAcc pa  = pairs[pi];
-      int4    hd  = make_int4(0, 0, 0, 0);    // the newest run, and whether it has grown here
-      bool    dirty = false;
-      if (pa.head) hd = nodes[pa.head];
+      int4 *const acc = (int4 *)(pairs + pi);
+      const int4 a0 = *acc;
+      int  head = a0.x, diagCt = a0.y, diagBgn = a0.z, diagEnd = a0.w, consistent = 1;
+      int4 hd   = make_int4(0, 0, 0, 0);    // the newest run, and whether it has grown here
+      bool dirty = false;
+      if (head) hd = nodes[head];
       unsigned m = peers;
       while (m) {
         const int q    = __ffs((int)m) - 1;
-        const int sOff = sm.sOff[at0 + q], tOff = sm.tOff[at0 + q];
+        const u32 o    = sm.off[at0 + q];
+        const int sOff = i0 + (int)(o >> kOffBits), tOff = (int)(o & ((1u << kOffBits) - 1));
         // Seed q, and the `more` seeds of the group that follow it one by one.
         const unsigned brk = m & ~follows & ~((2u << q) - 1);
         const unsigned run = brk ? m & ((brk & (0u - brk)) - 1) : m;
         int more = __popc(run) - 1;
         m &= m - 1;
-        pa.diagCt++;
-        if (pa.diagBgn > sOff) pa.diagBgn = sOff;
-        if (pa.diagEnd < sOff) pa.diagEnd = sOff;
+        diagCt++;
+        if (diagBgn > sOff) diagBgn = sOff;
+        if (diagEnd < sOff) diagEnd = sOff;
         // Add_Match's first node (Find_Overlaps.C:25-96): most seeds extend it.
         const int expected = hd.z + hd.y - K + 1, diag = hd.x - hd.z, newDiag = tOff - sOff;
-        if (pa.head && expected >= sOff) {
+        if (head && expected >= sOff) {
           if (expected == sOff && newDiag == diag) {
             hd.y++;
             dirty = true;
           } else {
-            if (dirty) nodes[pa.head].y = hd.y;
+            if (dirty) nodes[head].y = hd.y;
             dirty = false;
-            if (!add_match(nodes, sm, cap.nodeCap, pa.head, tOff, sOff, pa.consistent, K)) break;
-            hd = nodes[pa.head];
+            if (!add_match(nodes, sm, cap.nodeCap, head, tOff, sOff, consistent, K)) break;
+            hd = nodes[head];
             // Unless the seed's run is now the first node, the next seed walks the list too.
             if (hd.z + hd.y - K != sOff || hd.x - hd.z != newDiag) more = 0;
           }
         } else {
           // The walk stops at the first node: a new run.
-          if (pa.head && (abs(diag - newDiag) > 3 || sOff < expected + K - 2)) pa.consistent = 0;
+          if (head && (abs(diag - newDiag) > 3 || sOff < expected + K - 2)) consistent = 0;
           const int id = atomicAdd(&sm.nNodes, 1);
           if (id >= cap.nodeCap) {
             sm.overflow = 1;
             break;
           }
-          if (dirty) nodes[pa.head].y = hd.y;
+          if (dirty) nodes[head].y = hd.y;
           dirty     = false;
-          hd        = make_int4(tOff, K, sOff, pa.head);
+          hd        = make_int4(tOff, K, sOff, head);
           nodes[id] = hd;
-          pa.head   = id;
+          head   = id;
         }
         if (more) {
           // Each of them extends the first node by one.
           hd.y += more;
           dirty = true;
-          pa.diagCt += more;
-          if (pa.diagEnd < sOff + more) pa.diagEnd = sOff + more;
+          diagCt += more;
+          if (diagEnd < sOff + more) diagEnd = sOff + more;
           m &= ~run;
         }
       }
-      if (dirty) nodes[pa.head].y = hd.y;
-      pairs[pi].head       = pa.head;
-      pairs[pi].diagCt     = pa.diagCt;
-      pairs[pi].diagBgn    = pa.diagBgn;
-      pairs[pi].diagEnd    = pa.diagEnd;
-      pairs[pi].consistent = pa.consistent;
+      if (dirty) nodes[head].y = hd.y;
+      *acc = make_int4(head, diagCt, diagBgn, diagEnd);
+      if (!consistent) pairs[pi].consistent = 0;
     }
   }
   __syncwarp();
@@ -262,6 +271,7 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
   const int K      = P.kmerLen;
   const u64 kmask  = (K >= 32) ? ~0ull : ((1ull << (2 * K)) - 1);
   unsigned long long nSeeds = 0, nSegs = 0;
+  int par = 0;   // which half of warpSum and warpCnt the next 256 offsets take
 
   for (int i = tid; i < cap.slotCap; i += kSeedThreads) slotKey[i] = -1;
 
@@ -287,7 +297,8 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
     const u64 *Sn   = R.hasN[sRead] ? (dir ? R.nrc : R.nfwd) + wo : nullptr;
     const int sLen  = (int)R.len[sRead];
     const int nK    = sLen - K + 1;
-    const i64 thr   = (i64)(sRead + 1) - (i64)T.firstID;   // T qualifies iff tStr > thr
+    // A partner qualifies from this string on.
+    const u32 from = sRead + 2 > T.firstID ? sRead + 2 - T.firstID : 0;
     unsigned long long segSeeds = 0;   // counted once the segment completes in this configuration
 
     for (int i0 = 0; i0 < nK; i0 += kSeedThreads) {
@@ -308,103 +319,112 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
             }
             if (scr) atomicOr(&sm.screened, scr);
           } else {
+            // The qualifying occurrences are the run's end: it ascends by partner.
             const u32 start = (u32)(val & 0xffffffffull);
-            const u32 cnt   = (u32)((val >> 32) & 0x7fffffffull);
-            const u32 end   = start + cnt;
-            if (cnt <= (u32)kScanMax) {
-              while (n < cnt) {
-                u64 o[8];
-#pragma unroll
-                for (int k = 0; k < 8; k++) o[k] = (n + k < cnt) ? __ldg(T.occ + (end - 1 - n - k)) : 0ull;
-                u32 q = 0;
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                  if (q == (u32)k && n + k < cnt && (i64)(o[k] >> 32) > thr) q++;
-                n += q;
-                if (q < 8) break;
-              }
-            } else {
-              // first occurrence whose string is past thr
-              u32 lo = start, hi = end;
-              while (lo < hi) {
-                u32 mid = (lo + hi) >> 1;
-                if ((i64)(T.occ[mid] >> 32) > thr) hi = mid;
-                else lo = mid + 1;
-              }
-              n = end - lo;
+            qEnd            = start + (u32)((val >> 32) & 0x7fffffffull);
+            u32 lo = start, hi = qEnd;
+            while (lo < hi) {
+              const u32 mid = (lo + hi) >> 1;
+              if (__ldg((const u32 *)T.occ + 2 * (u64)mid + 1) >= from) hi = mid;
+              else lo = mid + 1;
             }
-            qEnd = end;
+            n = qEnd - lo;
           }
         }
       }
-      u32 total;
-      sm.qEnd[tid] = qEnd;
-      sm.incl[tid] = block_incl_scan(sm, n, total);
+      // The offsets that have seeds, in order.
+      const unsigned has = __ballot_sync(0xffffffffu, n > 0);
+      const u32 inc = warp_incl_scan_u32(n);
+      if (lane == 31) {
+        sm.warpSum[par][wib] = inc;
+        sm.warpCnt[par][wib] = __popc(has);
+      }
+      __syncthreads();
+      // Only a replay sets the flag, and none runs between this barrier and the next: all warps
+      // read the same.  (So it is after the buffer's counts below.)
+      if (sm.overflow) break;
+      u32 end = inc, total = 0;
+      int c = __popc(has & ((1u << lane) - 1)), nOff = 0;
+#pragma unroll
+      for (int w = 0; w < kSeedWarps; w++) {
+        const u32 x = sm.warpSum[par][w], y = sm.warpCnt[par][w];
+        end += w < wib ? x : 0;
+        c += w < wib ? y : 0;
+        total += x;
+        nOff += y;
+      }
+      par ^= 1;
+      if (total == 0) continue;
+      if (n) {
+        sm.end[c]  = end;
+        sm.from[c] = qEnd - 1 + (end - n);
+        sm.at[c]   = (unsigned char)tid;
+      }
       segSeeds += (tid == 0) ? total : 0;
+      __syncthreads();
 
       for (u32 b = 0; b < total; b += kSeedBuf) {
-        __syncthreads();
-        // Seeds b .. b + kSeedBuf, in reference order: thread tid has those at 256 k + tid.
-        u32 tS[kSeedPer];
-        int tO[kSeedPer], sO[kSeedPer], rank[kSeedPer];
+        // Seeds b .. b + kSeedBuf, in reference order; this warp lays out `per` chunks of 32.
+        const u32 stop = total - b < (u32)kSeedBuf ? total : b + kSeedBuf;
+        const int per  = (int)((stop - b + 32 * kSeedWarps - 1) / (32 * kSeedWarps));
+        u32 s0 = b + 32 * per * wib;
+        u32 tS[kSeedPer], off[kSeedPer], ranks = 0, run = 0;
+        // The first offset with seeds past s0.
+        int c0 = 0;
+        if (s0 < stop) {
+          c0 = 8 * __popc(__ballot_sync(0xffffffffu, 8 * lane + 7 < nOff && sm.end[8 * lane + 7] <= s0));
+          c0 += __popc(__ballot_sync(0xffffffffu, lane < 8 && c0 + lane < nOff && sm.end[c0 + lane] <= s0));
+        }
 #pragma unroll
         for (int k = 0; k < kSeedPer; k++) {
-          const u32  s  = b + kSeedThreads * k + tid;
-          const bool ok = s < total;
-          tS[k] = 0;
-          tO[k] = sO[k] = 0;
+          if (k >= per || s0 >= stop) break;
+          // The ends of the next 32 offsets, as bits: seed s0 + l is past those below bit l.
+          const u32 d = c0 + lane < nOff ? sm.end[c0 + lane] - s0 : 33;
+          const unsigned ends = __reduce_or_sync(0xffffffffu, d <= 32 ? 1u << (d - 1) : 0);
+          const int  j  = c0 + __popc(ends & ((1u << lane) - 1));
+          const bool ok = s0 + lane < stop;
+          tS[k] = off[k] = 0;
           if (ok) {
-            int lo = 0, hi = kSeedThreads - 1;   // first offset with incl > s
-            while (lo < hi) {
-              const int mid = (lo + hi) >> 1;
-              if (sm.incl[mid] > s) hi = mid;
-              else lo = mid + 1;
-            }
-            const u32 j = s - (lo ? sm.incl[lo - 1] : 0);
-            const u64 o = __ldg(T.occ + (sm.qEnd[lo] - 1 - j));   // newest occurrence first
-            tS[k] = (u32)(o >> 32);
-            tO[k] = (int)(u32)o;
-            sO[k] = i0 + lo;
+            const u64 o = __ldg(T.occ + (u32)(sm.from[j] - (s0 + lane)));   // newest occurrence first
+            tS[k]  = (u32)(o >> 32);
+            off[k] = (u32)sm.at[j] << kOffBits | (u32)o;
           }
-          // Its owner, and its rank among the owner's seeds of these 32.
+          // Its owner, and its rank among the owner's seeds of this warp; lane w counts owner w's.
           const u32 w = (tS[k] * 0x9e3779b1u) >> 29;
           const unsigned v0 = __ballot_sync(0xffffffffu, w & 1), v1 = __ballot_sync(0xffffffffu, w & 2),
                          v2 = __ballot_sync(0xffffffffu, w & 4), in = __ballot_sync(0xffffffffu, ok);
           const unsigned same = (w & 1 ? v0 : ~v0) & (w & 2 ? v1 : ~v1) & (w & 4 ? v2 : ~v2) & in;
-          rank[k] = ok ? __popc(same & ((1u << lane) - 1)) : -1;
-          const int chunk = kSeedWarps * k + wib;
-          if (lane < kSeedWarps)
-            sm.cnt[lane][chunk] = (unsigned short)__popc((lane & 1 ? v0 : ~v0) & (lane & 2 ? v1 : ~v1) &
-                                                         (lane & 4 ? v2 : ~v2) & in);
+          ranks |= (__shfl_sync(0xffffffffu, run, w) + __popc(same & ((1u << lane) - 1))) << (8 * k);
+          run += __popc((lane & 1 ? v0 : ~v0) & (lane & 2 ? v1 : ~v1) & (lane & 4 ? v2 : ~v2) & in);
+          c0 += __popc(ends);
+          s0 += 32;
         }
-        __syncthreads();
-        {
-          // Warp w turns its row of counts into places inside its part.
-          const u32 c   = sm.cnt[wib][lane];   // kSeedChunks == 32
-          const u32 inc = warp_incl_scan_u32(c);
-          sm.cnt[wib][lane] = (unsigned short)(inc - c);
-          if (lane == 31) sm.part[wib] = inc;
-        }
-        __syncthreads();
-        u32 first = 0;                          // this warp's part of the buffer
-        for (int w = 0; w < wib; w++) first += sm.part[w];
-        const int mine = (int)sm.part[wib];
+        if (lane < kSeedWarps) ((unsigned short *)sm.cnt[lane])[wib] = (unsigned short)run;
+        __syncthreads();   // every warp has replayed its part of the seeds before these
+        if (sm.overflow) break;
+        // Places: by owner, then by laying warp.
+        const u32 x   = (&sm.cnt[0][0])[lane];
+        const u32 sum = (x & 0xffff) + (x >> 16);
+        const u32 up  = warp_incl_scan_u32(sum);
+        const u32 place = up - sum + (wib & 1 ? x & 0xffff : 0);
+        const int first = (int)__shfl_sync(0xffffffffu, up - sum, 4 * wib);
+        const int last  = (int)__shfl_sync(0xffffffffu, up, 4 * wib + 3);
+        s0 = b + 32 * per * wib;
 #pragma unroll
-        for (int k = 0; k < kSeedPer; k++)
-          if (rank[k] >= 0) {
-            const u32 w = (tS[k] * 0x9e3779b1u) >> 29;
-            u32 p = sm.cnt[w][kSeedWarps * k + wib] + rank[k];
-            for (u32 x = 0; x < w; x++) p += sm.part[x];
+        for (int k = 0; k < kSeedPer; k++) {
+          if (k >= per || s0 >= stop) break;
+          const u32 w = (tS[k] * 0x9e3779b1u) >> 29;
+          const u32 p = __shfl_sync(0xffffffffu, place, 4 * w + (wib >> 1)) + ((ranks >> (8 * k)) & 0xff);
+          if (s0 + lane < stop) {
             sm.tStr[p] = tS[k];
-            sm.tOff[p] = tO[k];
-            sm.sOff[p] = sO[k];
+            sm.off[p]  = off[k];
           }
+          s0 += 32;
+        }
         __syncthreads();
-        for (int r = 0; r < mine; r += 32)
-          replay_round(sm, cap, slotKey, slotVal, pairs, nodes, r + lane < mine ? (int)first + r + lane : -1, K);
-        if (__syncthreads_or(sm.overflow)) break;
+        for (int r = first; r < last; r += 32)
+          replay_round(sm, cap, slotKey, slotVal, pairs, nodes, r + lane < last ? r + lane : -1, i0, K);
       }
-      if (__syncthreads_or(sm.overflow)) break;
     }
     __syncthreads();
     const int  nPairs = min(sm.nPairs, cap.pairCap);
