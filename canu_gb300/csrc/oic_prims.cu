@@ -127,6 +127,7 @@ constexpr int kUpItems     = 16;
 constexpr int kSortThreads = 512;                         // downsweep
 constexpr int kSortWarps   = kSortThreads / 32;
 constexpr int kSortItems   = 8;
+constexpr int kSortCtas    = 2;                           // per SM
 constexpr int kSortTile    = kSortThreads * kSortItems;   // 4096
 constexpr int kDigits      = 256;
 static_assert(kUpThreads * kUpItems == kSortTile && kUpThreads == kDigits, "one histogram per downsweep tile");
@@ -144,11 +145,17 @@ __global__ void __launch_bounds__(kUpThreads) radix_upsweep_kernel(const unsigne
   }
   for (int i = threadIdx.x; i < (kUpThreads / 32) * kDigits; i += kUpThreads) (&h[0][0])[i] = 0;
   __syncthreads();
-#pragma unroll 4
-  for (int k = 0; k < kUpItems; k++) {
-    uint64_t i = base + (uint64_t)k * kUpThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[wid][(keys[i] >> shift) & 0xff], 1u);
+  // All of a thread's loads in flight before the first count: 62 M keys in 76 us (6.6 TB/s;
+  // four at a time 128 us).
+  unsigned long long k[kUpItems];
+#pragma unroll
+  for (int it = 0; it < kUpItems; it++) {
+    const uint64_t i = base + (uint64_t)it * kUpThreads + threadIdx.x;
+    k[it] = i < n ? keys[i] : 0;
   }
+#pragma unroll
+  for (int it = 0; it < kUpItems; it++)
+    if (base + (uint64_t)it * kUpThreads + threadIdx.x < n) atomicAdd(&h[wid][(uint32_t)(k[it] >> shift) & 0xff], 1u);
   __syncthreads();
   for (int d = threadIdx.x; d < kDigits; d += kUpThreads) {
     uint32_t s = 0;
@@ -165,92 +172,109 @@ __global__ void __launch_bounds__(kUpThreads) radix_upsweep_kernel(const unsigne
 //
 // The lanes with the same digit are found with eight ballots: match_any walks a warp's
 // distinct digits one by one, and 8 warps x 16 keys of them waited for it two thirds of the
-// time (97 G keys/s).
+// time (97 G keys/s); marking the lanes in a word per digit in shared memory is as fast as
+// the ballots.  62 M keys and values took 385 us (161 G keys/s, 3.8 TB/s) while the tile's
+// output ranges were read between two barriers and 8 warps went over the counts twice; read
+// ahead, and with two digits to a word, 348 us.  More CTAs on an SM are slower, not faster
+// (3 with 40 registers, or tiles of 3,072: +7 %): the output's lines, of 256 runs per tile
+// in flight, are what L2 has to hold.
 template <bool VALS>
-__global__ void __launch_bounds__(kSortThreads) radix_downsweep_kernel(const unsigned long long *keysIn, const uint32_t *valsIn,
-                                                                       unsigned long long *keysOut, uint32_t *valsOut, uint64_t n,
-                                                                       int shift, const uint32_t *offsets,
-                                                                       uint32_t nTiles, const uint32_t *nDev) {
+__global__ void __launch_bounds__(kSortThreads, kSortCtas)
+    radix_downsweep_kernel(const unsigned long long *keysIn, const uint32_t *valsIn, unsigned long long *keysOut,
+                           uint32_t *valsOut, uint64_t n, int shift, const uint32_t *offsets, uint32_t nTiles,
+                           const uint32_t *nDev) {
   extern __shared__ __align__(16) unsigned char sortDyn[];
   unsigned long long *sk = (unsigned long long *)sortDyn;           // kSortTile keys
   uint32_t           *sv = (uint32_t *)(sk + kSortTile);             // kSortTile values
-  __shared__ uint16_t cnt[kSortWarps][kDigits];
+  __shared__ __align__(4) uint16_t cnt[kSortWarps][kDigits];
   __shared__ uint32_t tileBase[kDigits];     // output position of the tile's first key of each digit ...
-  __shared__ uint32_t warpSums[kDigits / 32];
+  __shared__ uint32_t warpSums[kDigits / 64];
   if (nDev && *nDev < n) n = *nDev;
   const uint64_t tile0 = (uint64_t)blockIdx.x * kSortTile;
   if (tile0 >= n) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kSortWarps * kDigits / 2; i += kSortThreads) ((uint32_t *)&cnt[0][0])[i] = 0;
-  __syncthreads();
-
-  const uint64_t base = tile0 + (uint64_t)wid * (32 * kSortItems);
+  const uint32_t tot = (uint32_t)(n - tile0 < kSortTile ? n - tile0 : kSortTile);   // the tile's keys
+  const uint32_t l0  = (uint32_t)wid * (32 * kSortItems) + lane;                    // this thread's first
   const unsigned ltMask = (1u << lane) - 1;
   unsigned long long k[kSortItems];
   uint32_t v[kSortItems];
-  uint32_t rank[kSortItems];
+  uint32_t rank[kSortItems / 2];             // two 16-bit ranks to a word
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
-    uint64_t i = base + (uint64_t)it * 32 + lane;
-    bool     ok = i < n;
-    k[it]       = ok ? keysIn[i] : 0;
-    if (VALS) v[it] = ok ? valsIn[i] : 0;
+    const bool ok = l0 + it * 32 < tot;
+    k[it] = ok ? keysIn[tile0 + l0 + it * 32] : 0;
+    if (VALS) v[it] = ok ? valsIn[tile0 + l0 + it * 32] : 0;
   }
+  // Digits 2 t and 2 t + 1 are thread t's; their output ranges come while the keys are ranked.
+  const int t = threadIdx.x;
+  uint32_t out0 = 0, out1 = 0;
+  if (t < kDigits / 2) {
+    out0 = offsets[(uint64_t)(2 * t) * nTiles + blockIdx.x];
+    out1 = offsets[(uint64_t)(2 * t + 1) * nTiles + blockIdx.x];
+  }
+  for (int i = lane; i < kDigits / 2; i += 32) ((uint32_t *)cnt[wid])[i] = 0;
+  __syncwarp();
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
-    const bool ok = base + (uint64_t)it * 32 + lane < n;
+    const bool ok = l0 + it * 32 < tot;
     const uint32_t d = (uint32_t)(k[it] >> shift) & 0xff;
     unsigned peers = __ballot_sync(0xffffffffu, ok);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
-      const unsigned m = __ballot_sync(0xffffffffu, (d >> b) & 1);
-      peers &= (d >> b) & 1 ? m : ~m;
+      const bool bit = (d & (1u << b)) != 0;
+      const unsigned m = __ballot_sync(0xffffffffu, bit);
+      peers &= bit ? m : ~m;
     }
-    const uint32_t c = cnt[wid][d];
-    rank[it]  = c + __popc(peers & ltMask);
+    const uint32_t c = cnt[wid][d], below = (uint32_t)__popc(peers & ltMask);
+    if (it & 1) rank[it / 2] |= (c + below) << 16;
+    else rank[it / 2] = c + below;
     __syncwarp();
-    if (ok && (peers & ltMask) == 0) cnt[wid][d] = (uint16_t)(c + __popc(peers));
+    if (ok && below == 0) cnt[wid][d] = (uint16_t)(c + __popc(peers));
     __syncwarp();
   }
   __syncthreads();
-  // Per digit: the warps' exclusive prefix, then the digit's start inside the tile.
-  uint32_t s = 0, incl = 0;
-  const int d0 = threadIdx.x;
-  if (d0 < kDigits) {
+  // Per digit: the warps' exclusive prefix and the digit's start inside the tile, for two
+  // digits in one word (no half passes 4,096).
+  uint32_t c[kSortWarps], s = 0, incl = 0;
+  if (t < kDigits / 2) {
 #pragma unroll
     for (int w = 0; w < kSortWarps; w++) {
-      const uint32_t c = cnt[w][d0];
-      cnt[w][d0]       = (uint16_t)s;
-      s += c;
+      c[w] = ((uint32_t *)cnt[w])[t];
+      s += c[w];
     }
-    incl = warp_incl_scan(s);
+    incl = warp_incl_scan((s & 0xffff) + (s >> 16));
     if (lane == 31) warpSums[wid] = incl;
   }
   __syncthreads();
-  if (d0 < kDigits) {
-    uint32_t start = incl - s;
+  if (t < kDigits / 2) {
+    uint32_t start = incl - (s & 0xffff) - (s >> 16);
     for (int w = 0; w < wid; w++) start += warpSums[w];
+    const uint32_t next = start + (s & 0xffff);
+    uint32_t at = start | next << 16;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; w++) cnt[w][d0] = (uint16_t)(cnt[w][d0] + start);
-    tileBase[d0] = offsets[(uint64_t)d0 * nTiles + blockIdx.x] - start;   // ... minus its place in the tile
+    for (int w = 0; w < kSortWarps; w++) {
+      ((uint32_t *)cnt[w])[t] = at;
+      at += c[w];
+    }
+    tileBase[2 * t]     = out0 - start;       // ... minus its place in the tile
+    tileBase[2 * t + 1] = out1 - next;
   }
   __syncthreads();
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
-    if (base + (uint64_t)it * 32 + lane < n) {
-      const uint32_t p = cnt[wid][(uint32_t)(k[it] >> shift) & 0xff] + rank[it];
+    if (l0 + it * 32 < tot) {
+      const uint32_t p = cnt[wid][(uint32_t)(k[it] >> shift) & 0xff] + ((rank[it / 2] >> (16 * (it & 1))) & 0xffff);
       sk[p] = k[it];
       if (VALS) sv[p] = v[it];
     }
   }
   __syncthreads();
-  const uint32_t tot = (uint32_t)(n - tile0 < kSortTile ? n - tile0 : kSortTile);
 #pragma unroll
   for (int it = 0; it < kSortItems; it++) {
     const uint32_t p = it * kSortThreads + threadIdx.x;
     if (p < tot) {
       const unsigned long long key = sk[p];
-      const uint64_t pos = (uint64_t)(uint32_t)(tileBase[(uint32_t)(key >> shift) & 0xff] + p);
+      const uint32_t pos = tileBase[(uint32_t)(key >> shift) & 0xff] + p;
       keysOut[pos] = key;
       if (VALS) valsOut[pos] = sv[p];
     }
