@@ -889,10 +889,9 @@ int align_stage_graph(oic_ctx *ctx, uint32_t nPairs, uint32_t nNodes, const oic_
     cudaMemsetAsync(ctr64(ctx) + kAlignStatBase, 0, kStCount * sizeof(unsigned long long), s);
     launch_work_keys(ctx->dPairs.as<PairRec>(), cap, logit, ctx->filterLogitThr, ctx->R.len, ctx->T.sread,
                      tn.wideMinLen, ctr32(ctx) + cKeep, ctx->dWorkK.as<u64>(), ctx->dWork.as<uint32_t>(), s,
-                     ctr32(ctx) + cPairCount);
+                     ctr32(ctx) + cPairCount, ctx->dCnt.as<uint32_t>());
     radix_sort_u64_u32(ctx->dWorkK.as<u64>(), ctx->dWork.as<uint32_t>(), ctx->dWorkK2.as<u64>(),
                        ctx->dWorkV2.as<uint32_t>(), cap, 32, ctx->dWorkScratch.p, s, ctr32(ctx) + cPairCount);
-    cudaMemsetAsync(ctx->dCnt.p, 0, (size_t)cap * sizeof(uint32_t), s);
     if (coll) {
       cudaMemsetAsync(ctx->dPairCells.p, 0, (size_t)cap * sizeof(uint32_t), s);
       cudaMemsetAsync(ctx->dPairExt.p, 0, (size_t)cap * sizeof(int4), s);
@@ -910,9 +909,9 @@ int align_stage_graph(oic_ctx *ctx, uint32_t nPairs, uint32_t nNodes, const oic_
     launch_cta_bin(ctx, tn, bG, ctas, ctx->dWork.as<uint32_t>(), 0, aoW, s);
     cudaEventRecordWithFlags(ctx->gEv[2], s, cudaEventRecordExternal);   // recorded at every replay
     scan_u32(ctx->dCnt.as<uint32_t>(), ctx->dRecPos.as<uint32_t>(), cap, ctr32(ctx) + cRecTotal,
-             ctx->dScanScratch.p, s);
+             ctx->dScanScratch.p, s, ctr32(ctx) + cPairCount);
     launch_compact_records(ctx->dRec.as<uint32_t>(), ctx->dCnt.as<uint32_t>(), ctx->dRecPos.as<uint32_t>(), cap,
-                           ctx->dRecOut.as<uint32_t>(), s);
+                           ctx->dRecOut.as<uint32_t>(), s, ctr32(ctx) + cPairCount);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
     g_launches    = launches0;
@@ -979,9 +978,9 @@ int align_stage_graph(oic_ctx *ctx, uint32_t nPairs, uint32_t nNodes, const oic_
                        ctx->dNodes.as<int4>(), wsH, capsH, ao, ctx->st);
     cudaEventRecord(h1, ctx->st);
     CK(scan_u32(ctx->dCnt.as<uint32_t>(), ctx->dRecPos.as<uint32_t>(), cap, ctr32(ctx) + cRecTotal,
-                ctx->dScanScratch.p, ctx->st));
+                ctx->dScanScratch.p, ctx->st, ctr32(ctx) + cPairCount));
     launch_compact_records(ctx->dRec.as<uint32_t>(), ctx->dCnt.as<uint32_t>(), ctx->dRecPos.as<uint32_t>(), cap,
-                           ctx->dRecOut.as<uint32_t>(), ctx->st);
+                           ctx->dRecOut.as<uint32_t>(), ctx->st, ctr32(ctx) + cPairCount);
     CK(cudaMemcpyAsync(h, ctx->dCtr.p, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->st));
     rc = sync_check(ctx, "align kernel (large arena)");
     float hm = 0;

@@ -154,10 +154,10 @@ void launch_extend_batch(ReadsDev R, DevParams P, const int *eml, const ExtendPr
 // Sort keys (32 bits) of the work list: by bin -- 0 one-warp DP, 1 CTA DP (shorter read
 // >= wideMinLen bases), 2 dropped by the filter (logit non-null, below logitThr) -- and
 // inside a bin the pairs with the most match nodes first.  binCount[0..1] (zeroed by
-// the caller) get the sizes of bins 0 and 1.
+// the caller) get the sizes of bins 0 and 1; cnt, when given, is zeroed.
 void launch_work_keys(const PairRec *pairs, u32 n, const float *logit, float logitThr, const u32 *readLen,
                       const u32 *strRead, u32 wideMinLen, u32 *binCount, unsigned long long *keys, u32 *vals,
-                      cudaStream_t st, const u32 *nDev = nullptr);
+                      cudaStream_t st, const u32 *nDev = nullptr, u32 *cnt = nullptr);
 // Append the one-warp overflow behind the CTA bin's own pairs on the device (see
 // append_overflow_kernel in oic_pairs.cu).
 void launch_append_overflow(u32 *work, const u32 *binCount, const u32 *ovf, u32 *ovfCount, u32 *wideN,
@@ -190,7 +190,8 @@ void launch_run_compact(const u64 *keys, const u64 *runStart, u32 nRuns, u64 nVa
                         u64 *outKey, u32 *outCount, cudaStream_t st);
 
 // Compact per-pair record slots into a dense record array.
-void launch_compact_records(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst, cudaStream_t st);
+void launch_compact_records(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst, cudaStream_t st,
+                            const u32 *nDev = nullptr);
 
 int align_warps_per_block();
 

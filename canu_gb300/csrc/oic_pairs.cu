@@ -1208,7 +1208,7 @@ __global__ void __launch_bounds__(kSpecWarps * 32, 3) align_spec_kernel(
 // of bins 0 and 1.
 __global__ void work_keys_kernel(const PairRec *pairs, u32 n, const float *logit, float logitThr, const u32 *readLen,
                                  const u32 *strRead, u32 wideMinLen, u32 *binCount, unsigned long long *keys,
-                                 u32 *vals, const u32 *nDev) {
+                                 u32 *vals, const u32 *nDev, u32 *cnt) {
   if (nDev && *nDev < n) n = *nDev;
   const u32 stride = gridDim.x * blockDim.x;
   const int lane   = threadIdx.x & 31;
@@ -1225,6 +1225,7 @@ __global__ void work_keys_kernel(const PairRec *pairs, u32 n, const float *logit
       const u32 nc = pr.nodeCnt < 0x3fffffffu ? pr.nodeCnt : 0x3fffffffu;
       keys[i]      = ((unsigned long long)bin << 30) | (0x3fffffffu - nc);
       vals[i]      = i;
+      if (cnt) cnt[i] = 0;
     }
     const unsigned b0 = __ballot_sync(0xffffffffu, bin == 0), b1 = __ballot_sync(0xffffffffu, bin == 1);
     if (lane == 0) {
@@ -1264,7 +1265,9 @@ __global__ void list_keys_kernel(const PairRec *pairs, const u32 *list, u32 n, u
   }
 }
 
-__global__ void compact_records_kernel(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst) {
+__global__ void compact_records_kernel(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst,
+                                       const u32 *nDev) {
+  if (nDev && *nDev < nPairs) nPairs = *nDev;
   for (u32 p = blockIdx.x * blockDim.x + threadIdx.x; p < nPairs; p += gridDim.x * blockDim.x) {
     const u32 c = cnt[p];
     for (u32 j = 0; j < c * 6; j++) dst[(u64)pos[p] * 6 + j] = rec[(u64)p * 18 + j];
@@ -1337,14 +1340,19 @@ void launch_extend_group(int threads, int U, int bandW, int ctas, ReadsDev R, De
   g_launches++;
 }
 
+// Blocks of 256 threads that go through n pairs, or through the device's count of them (up to
+// n: as many blocks as fill the chip, the threads take the pairs in turn).
+static unsigned pair_blocks(u32 n, const u32 *nDev) {
+  const u64 g = ((u64)n + 255) / 256, most = nDev ? 1216 : 65535u * 8;
+  return (unsigned)(g < most ? g : most);
+}
+
 void launch_work_keys(const PairRec *pairs, u32 n, const float *logit, float logitThr, const u32 *readLen,
                       const u32 *strRead, u32 wideMinLen, u32 *binCount, unsigned long long *keys, u32 *vals,
-                      cudaStream_t st, const u32 *nDev) {
+                      cudaStream_t st, const u32 *nDev, u32 *cnt) {
   if (n == 0) return;
-  unsigned g = (n + 255) / 256;
-  if (g > 65535u * 8) g = 65535u * 8;
-  work_keys_kernel<<<g, 256, 0, st>>>(pairs, n, logit, logitThr, readLen, strRead, wideMinLen, binCount, keys, vals,
-                                      nDev);
+  work_keys_kernel<<<pair_blocks(n, nDev), 256, 0, st>>>(pairs, n, logit, logitThr, readLen, strRead, wideMinLen,
+                                                         binCount, keys, vals, nDev, cnt);
   g_launches++;
 }
 
@@ -1363,11 +1371,10 @@ void launch_list_keys(const PairRec *pairs, const u32 *list, u32 n, unsigned lon
   g_launches++;
 }
 
-void launch_compact_records(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst, cudaStream_t st) {
+void launch_compact_records(const u32 *rec, const u32 *cnt, const u32 *pos, u32 nPairs, u32 *dst, cudaStream_t st,
+                            const u32 *nDev) {
   if (nPairs == 0) return;
-  unsigned g = (nPairs + 255) / 256;
-  if (g > 65535u * 8) g = 65535u * 8;
-  compact_records_kernel<<<g, 256, 0, st>>>(rec, cnt, pos, nPairs, dst);
+  compact_records_kernel<<<pair_blocks(nPairs, nDev), 256, 0, st>>>(rec, cnt, pos, nPairs, dst, nDev);
   g_launches++;
 }
 

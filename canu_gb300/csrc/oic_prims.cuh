@@ -16,8 +16,9 @@ extern thread_local unsigned long long g_launches;
 // Scratch bytes oic_scan_u32 needs for n elements.
 size_t scan_u32_scratch(uint64_t n);
 // out[i] = sum(in[0..i)) for i < n, and *total (device pointer, may be null) = sum(in).
-// `in` and `out` may alias.  n < 2^32.
-cudaError_t scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *total, void *scratch, cudaStream_t st);
+// `in` and `out` may alias.  n < 2^32.  With nDev non-null it scans the first min(n, *nDev).
+cudaError_t scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *total, void *scratch, cudaStream_t st,
+                     const uint32_t *nDev = nullptr);
 
 // Scratch bytes radix_sort needs for n elements (double buffers are separate).
 size_t radix_sort_scratch(uint64_t n);
