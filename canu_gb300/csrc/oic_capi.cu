@@ -1194,6 +1194,7 @@ int oic_create(const oic_params *p, int device, oic_ctx **out) {
         dp.kmerExpect * (double)((uint64_t)(int64_t)ctx->P.minOlapLen - (uint64_t)ctx->P.kmerLen + 1));
   dp.kmerLen    = (int)ctx->P.kmerLen;
   dp.partial    = ctx->P.partial ? 1 : 0;
+  dp.collect = dp.pad = 0;
   dp.unique     = ctx->P.uniqueOlapPerPair ? 1 : 0;
   dp.hopeless   = ctx->P.useHopelessCheck ? 1 : 0;
   dp.minOlapLen = ctx->P.minOlapLen;
@@ -1741,7 +1742,8 @@ int oic_set_filter(oic_ctx *ctx, const uint16_t *params, float threshold, float 
 
 int oic_collect_pairs(oic_ctx *ctx, int mode) {
   if (!ctx || mode < 0 || mode > 2) return OIC_ERR_ARG;
-  ctx->collect = mode;
+  ctx->collect    = mode;
+  ctx->dp.collect = mode != 0;
   return OIC_OK;
 }
 

@@ -189,6 +189,8 @@ struct DevParams {
   int    hopeless;
   int    minOlapLen;
   int    maxErrors;            // MAX_ERRORS (prefixEditDistance.C:27)
+  int    collect;              // pairs are collected
+  int    pad;
 };
 
 __device__ __forceinline__ int error_bound(int i, double maxErate) {

@@ -300,6 +300,7 @@ __device__ __forceinline__ void extend_node(WarpDP &w, const ReadView &S, int sL
 // stays readable).
 enum { kSlotFree = 0, kSlotRunning = 1, kSlotDone = 2, kSlotCancelled = 3 };
 constexpr unsigned char kNodeDead = 0, kNodeOpen = 1, kNodeOwner = 2, kNodeHelper = 3;   // kNodeHelper + h: helper h
+constexpr unsigned char kNodeProved = 255;   // collected pairs only: shown to have no overlap, still to be counted
 
 struct TeamPair {            // a pair open to helpers
   int            lock;
@@ -475,12 +476,12 @@ static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, const ReadVie
                                                         const int4 *nodes, int cnt, volatile unsigned char *alive,
                                                         float extCells, float extRows, Team *tm, int me, bool open) {
   const int lane = threadIdx.x & 31;
-  const int next = best_node(nodes, alive, cnt, kNodeOpen, 255);
+  const int next = best_node(nodes, alive, cnt, kNodeOpen, kNodeProved - 1);
   if (next < 0) return true;
   const int dc = nodes[next].x - nodes[next].z;
   int dlo = INT_MAX, dhi = INT_MIN, E = 0, n = 0;
   for (int i = lane; i < cnt; i += 32)
-    if (alive[i] != kNodeDead) {
+    if (alive[i] != kNodeDead && alive[i] != kNodeProved) {
       const int4 q = nodes[i];
       const int  d = q.x - q.z;
       if (abs(d - dc) <= kProofSpan) {
@@ -508,8 +509,8 @@ static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, const ReadVie
   for (int i = lane; i < cnt; i += 32) {
     const int st = alive[i];
     const int d  = nodes[i].x - nodes[i].z;
-    if (st == kNodeDead || d < dlo || d > dhi) continue;
-    alive[i] = kNodeDead;
+    if (st == kNodeDead || st == kNodeProved || d < dlo || d > dhi) continue;
+    alive[i] = w.P.collect ? kNodeProved : kNodeDead;
     was += st == kNodeOpen;
     if (open && st >= kNodeHelper) team_drop(*tm, st - kNodeHelper);
   }
@@ -633,8 +634,10 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     if (open && !team_lock(tm->pair[me])) { w.err |= kErrInternal; break; }
     const int li = best_node(nodes, alive, cnt, kNodeOpen, 255);
     int h = -1;
+    // A node shown to have no overlap has its turn among the pair's extensions, and is gone.
+    const bool proved = P.collect && li >= 0 && alive[li] == kNodeProved;
     if (open) {
-      if (li >= 0) {
+      if (li >= 0 && !proved) {
         h = (int)alive[li] - kNodeHelper;
         __syncwarp();
         if (h < 0 && lane == 0) {
@@ -645,6 +648,15 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
       team_unlock(tm->pair[me]);
     }
     if (li < 0) break;
+    if (proved) {
+      __syncwarp();
+      if (lane == 0) {
+        alive[li] = kNodeDead;
+        ps.nExt++;
+      }
+      __syncwarp();
+      continue;
+    }
 
     ExtRes    &res = ps.res;
     const int *dl  = w.sc.deltaL;
@@ -714,7 +726,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
         const int st = rm ? (int)alive[i] : (int)kNodeDead;
         if (rm) {
           alive[i] = kNodeDead;
-          if (st >= kNodeHelper && i != li) team_drop(*tm, st - kNodeHelper);
+          if (st >= kNodeHelper && st != kNodeProved && i != li) team_drop(*tm, st - kNodeHelper);
         }
         const unsigned was = __ballot_sync(0xffffffffu, st == kNodeOpen);
         if (lane == 0) tm->pair[me].open -= __popc(was);

@@ -200,10 +200,10 @@ typedef struct oic_pair_info {
   uint32_t seeds;      /* k-mer seeds of the pair (diag_ct) */
   uint32_t nodes;      /* match runs of the pair (its nodes in oic_get_pairs' node array) */
   uint32_t overlaps;   /* records the DP emitted for the pair */
-  uint32_t cells;      /* DP cells spent on the pair (saturating) */
+  uint32_t cells;      /* DP cells spent on the pair (saturating); as dpCells of oic_stats, work done */
   float    score;      /* filter logit (0 when no filter is set) */
-  uint32_t extensions; /* Extend_Alignment calls made for the pair */
-  int32_t  firstHit;   /* index of the first extension that added an overlap, -1 none */
+  uint32_t extensions; /* the reference's Extend_Alignment calls for the pair */
+  int32_t  firstHit;   /* index of the first of them that added an overlap, -1 none */
   uint32_t cellsFirst; /* DP cells of the pair's first extension */
   uint32_t extLimit;   /* 1 when the filter's single-extension tier applied, else 0 */
 } oic_pair_info;
@@ -262,7 +262,8 @@ int oic_mlp_adam(float *dMaster, float *dM, float *dV, float *dGrad, uint16_t *d
 /* ---------------------------------------------------------------------------------
  * DP launch configuration.  No counterpart in the reference (its DP runs one pair per
  * OpenMP thread).  Candidate pairs go to one of two bins:
- *   one-warp bin   one warp per pair, 8 warps per CTA, 512-int shared-memory rows
+ *   one-warp bin   one warp per pair, 24 warps per CTA, which extend nodes of one
+ *                  another's pairs when they have none; 512-int shared-memory rows
  *                  (wider bands continue in HBM rows up to 16384), at most narrowArena
  *                  kept DP cells per extension;
  *   CTA bin        one pair per CTA of wideThreads threads (32 x warps per pair); each

@@ -124,3 +124,31 @@ def test_hopeless_groups_keep_records(err, erate, with_n, built):
         assert sa[k] == sb[k], k
     if erate <= 0.02:
         assert sa["extensions"] < sb["extensions"]   # groups were dropped
+
+
+@pytest.mark.parametrize("erate", [0.01, 0.02])
+def test_collected_pairs_count_the_reference_extensions(erate, built):
+    """The extensions and the first hit of a collected pair do not depend on which of its
+    match nodes were shown to have no overlap without extending them."""
+    r = np.random.default_rng(14)
+    rep = rand_seq(r, 2500)
+    g = rand_seq(r, 6000) + rep + rand_seq(r, 9000) + mutate(r, rep, 0.01) + rand_seq(r, 6000)
+    seqs = []
+    for _ in range(40):
+        n = int(r.integers(2500, 8000))
+        p = int(r.integers(0, len(g) - n))
+        seqs.append(mutate(r, g[p:p + n], 0.55 * erate).encode())
+    off = np.cumsum([0] + [len(x) for x in seqs])
+    got = []
+    for wide in (0, 1):
+        with oic.Overlapper(oic.default_params(kmerLen=K, hashBits=18, maxErate=erate, minOlapLen=500)) as ov:
+            ov.set_reads(np.ones(len(seqs)), [len(x) for x in seqs], off[:-1], np.frombuffer(b"".join(seqs), np.uint8))
+            ov.set_tuning(forceWide=wide)
+            ov.collect_pairs(1)
+            ov.run()
+            info = ov.pairs()[0]
+            got.append((info[np.lexsort((info["flags"], info["bID"], info["aID"]))], ov.stats()["extensions"]))
+    (a, na), (b, nb) = got
+    assert na < nb   # groups were dropped
+    for k in ("aID", "bID", "flags", "nodes", "overlaps", "extensions", "firstHit"):
+        assert np.array_equal(a[k], b[k]), k
