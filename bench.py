@@ -514,17 +514,17 @@ def main():
     alg_bytes = pairs * (32 + 72 + 4 + 2 * mean_len / 4) + nodes * 16
     achieved = alg_bytes / (ms_align / 1000.0) / 1e9
     # DRAM bytes per DP cell of the one-warp DP kernel, from one ncu capture of a 1/50
-    # scale c2 launch (10.54 GB read + 22.94 GB written for 6.598 G cells; the figures and
+    # scale c2 launch (2.113 GB read + 4.293 GB written for 0.966 G cells; the figures and
     # the command are in profiles/align_kernel_c2_scale0.02_ncu.md), scaled to this job.
-    traffic = 5.074 * cells
+    traffic = 6.632 * cells
     sm_mhz = clk.get("sm_mhz") or peaks.get("sm_max_mhz", 2070.0)
     int_peak = 152 * INT_LANES_PER_SM * sm_mhz * 1e6 / 1e12
     int_ops = 6 * cells + slides / 16.0
-    # Instruction issue, the one-warp DP's binding resource: 15.85 warp instructions per
-    # DP cell (ncu smsp__inst_executed.sum of the same 1/50-scale c2 launch) against 152
-    # SMs x 4 schedulers x one warp instruction per cycle.
+    # Instruction issue: 406 warp instructions per DP error row (ncu smsp__inst_executed.sum
+    # of the same 1/50-scale c2 launch, 8.207 G for 20.23 M rows, the proofs that spare
+    # extensions included) against 152 SMs x 4 schedulers x one warp instruction per cycle.
     issue_peak = 152 * 4 * sm_mhz * 1e6 / 1e9
-    issue_ach = 15.85 * cells / (ms_align / 1000.0) / 1e9
+    issue_ach = 406 * float(st0.get("dpRows", 0)) / (ms_align / 1000.0) / 1e9
     # The memory stages by the byte model of the hash build and probe: build 0.25 B per
     # base read + 12 B per k-mer written (8 B key, 4 B position), and separately the sort
     # passes (6 passes x 24 B per k-mer); probe 2 strands x (0.25 B per base + one 32 B
@@ -568,19 +568,19 @@ def main():
                                           "INT32 lanes x median SM clock"},
                      "issue": {"achieved_g_warp_inst_per_s": issue_ach, "peak_g_warp_inst_per_s": issue_peak,
                                "frac": issue_ach / issue_peak,
-                               "basis": "15.85 warp instructions per DP cell (ncu, one-warp DP kernel, 1/50-scale "
-                                        "c2 launch: profiles/align_kernel_c2_scale0.02_ncu.md) x this job's DP "
-                                        "cells / DP stage time; peak = 152 SMs x 4 schedulers x median SM clock"},
+                               "basis": "406 warp instructions per DP error row (ncu, one-warp DP kernel, 1/50-scale "
+                                        "c2 launch: profiles/align_kernel_c2_scale0.02_ncu.md) x this job's error "
+                                        "rows / DP stage time; peak = 152 SMs x 4 schedulers x median SM clock"},
                      "hash": stage_roof(hash_bytes, ms_hash, "0.25 B/base + 12 B/k-mer (sort passes excluded)"),
                      "hash_with_sort": stage_roof(hash_bytes + sort_passes * 24 * n_kmers, ms_hash,
                                                   f"as hash + {sort_passes} radix passes x 24 B/k-mer",
-                                                  sort_passes * 24.1 * n_kmers,
-                                                  "radix passes only: ncu 24.1 B DRAM per key and pass "
-                                                  "(profiles/radix_downsweep_c2_scale0.25_ncu.md)"),
+                                                  sort_passes * 23.9 * n_kmers,
+                                                  "radix passes only: ncu 23.9 B DRAM per key and pass "
+                                                  "(profiles/radix_downsweep_c2_scale0.1_ncu.md)"),
                      "seed": stage_roof(seed_bytes, ms_seed, "2 strands x (0.25 B/base + 32 B/lookup) + 12 B/seed",
-                                        54.9 * float(st0["seeds"]),
-                                        "ncu 54.9 B DRAM per seed of a 1/4-scale c2 launch x this job's seeds "
-                                        "(profiles/seed_kernel_c2_scale0.25_ncu.md)")},
+                                        47.7 * float(st0["seeds"]),
+                                        "ncu 47.7 B DRAM per seed of a 1/50-scale c2 launch x this job's seeds "
+                                        "(profiles/seed_kernel_c2_scale0.02_ncu.md)")},
         "gpu_launches": int(sum(r[0]["kernelLaunches"] for r in res)),
         "clocks": clk,
     }
