@@ -1403,9 +1403,10 @@ int oic_load_hash_block(oic_ctx *ctx, uint32_t bgnID, uint32_t endID, uint32_t *
   CK(cudaMemcpyAsync(ctx->dStrKmers.p, strKmers.data(), nCand * 4, cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemcpyAsync(ctx->dFlat.p, flat.data(), (size_t)(nCand + 1) * 8, cudaMemcpyHostToDevice, ctx->st));
   CK(cudaMemsetAsync(ctx->dNewKeys.p, 0, (size_t)nCand * 4 + 4, ctx->st));
-  // With no more k-mers than the entry limit no read can meet it: the block is every
-  // candidate string, and the strings' new k-mers need not be known one by one.
-  const bool whole = nFlat <= entryLim;
+  // With fewer k-mers than the entry limit no read can meet it: the block is every
+  // candidate string, and the strings' new k-mers need not be known one by one.  (With as
+  // many, strings without k-mers after the last one that has some are left out.)
+  const bool whole = nFlat < entryLim;
   if (nCand) launch_chunk_str(ctx->dFlat.as<u64>(), nCand, nFlat, ctx->dChunkStr.as<uint32_t>(), ctx->st);
 
   const size_t n = (size_t)nFlat;
