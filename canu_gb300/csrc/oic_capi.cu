@@ -1810,7 +1810,11 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
     if (pass == 0) {
       AlignConfig ac = align_normal(ctx);
       ac.caps.arenaCap = (int)tn.narrowArena;
-      ac.caps.rowsGW   = ac.caps.bandW;   // a band wider than the shared-memory rows is the CTA's
+      // Few problems: a band wider than the shared-memory rows is the CTA's at once.  Many
+      // keep every warp busy, and wide rows in HBM then cost less than a CTA per problem.
+      // 230 / 1,000 / 4,000 noisy extensions of 30 kb reads: 7.2 / 18.1 / 55.5 ms by the CTA,
+      // 20.1 / 21.2 / 47.1 by the warps; of 15 kb reads 3.4 / 6.6 / 18.9 and 6.1 / 7.3 / 10.1.
+      if (nAlign <= 8u * (uint32_t)ctx->nSM) ac.caps.rowsGW = ac.caps.bandW;
       WarpScratch ws;
       if ((rc = ensure_align_scratch(ctx, ac, false, ws))) break;
       launch_extend_batch(ctx->R, ctx->dp, ctx->dEml.as<int>(), dP.as<ExtendProblem>(), nAlign, ws,

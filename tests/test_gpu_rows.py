@@ -152,3 +152,26 @@ def test_collected_pairs_count_the_reference_extensions(erate, built):
     assert na < nb   # groups were dropped
     for k in ("aID", "bID", "flags", "nodes", "overlaps", "extensions", "firstHit"):
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("erate", [0.12])
+def test_wide_bands_by_warps_and_by_ctas(erate, built):
+    """Bands wider than the shared-memory rows: a small batch hands them to the CTA kernel, a
+    large one keeps them on a warp; the results are the same."""
+    r = np.random.default_rng(15)
+    seqs, prob = [], []
+    for i in range(9):
+        g = rand_seq(r, 9000 + 1500 * i)
+        seqs += [mutate(r, g, 0.05).encode(), mutate(r, g, 0.05).encode()]
+        anchor = next((p, q) for p in range(2000, 8000) for q in [seqs[-1].find(seqs[-2][p:p + K])] if q >= 0)
+        prob.append((2 * i + 1, 0, 2 * i + 2, anchor[0], anchor[1], K))
+    off = np.cumsum([0] + [len(x) for x in seqs])
+    with oic.Overlapper(oic.default_params(kmerLen=K, maxErate=erate)) as ov:
+        ov.set_reads(np.ones(len(seqs)), [len(x) for x in seqs], off[:-1], np.frombuffer(b"".join(seqs), np.uint8))
+        a = np.array(prob)
+        small = ov.extend_batch(*[a[:, j] for j in range(6)])
+        b = np.tile(a, (300, 1))                 # 2,700 problems: more than eight per SM
+        large = ov.extend_batch(*[b[:, j] for j in range(6)])
+    assert (small[1] == 3).any()                 # some reach both ends
+    for s, l in zip(small, large):
+        assert (np.tile(s, (300,) + (1,) * (s.ndim - 1)) == l).all()
