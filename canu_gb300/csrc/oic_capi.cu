@@ -1839,7 +1839,11 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
       AlignCaps   caps;
       WarpScratch ws;
       if ((rc = ensure_group_scratch(ctx, tn, pass == 2, ctas, caps, ws))) break;
-      const int threads = pass == 2 ? (int)std::max<uint32_t>(tn.wideThreads, 512) : (int)tn.wideThreads;
+      // More problems than three per SM: two CTAs of 256 threads on one where the default is
+      // 512 (noisy extensions: 4,000 of 15 kb reads 15.3 against 23.3 ms, 1,000 of 30 kb reads
+      // 16.4 and 18.3, but 400 of them 8.9 and 8.5 and 230 of 60 kb reads 19.4 and 14.2).
+      int threads = pass == 2 ? (int)std::max<uint32_t>(tn.wideThreads, 512) : (int)tn.wideThreads;
+      if (pass == 1 && !ctx->tune.wideThreads && ns > 3u * (uint32_t)ctx->nSM) threads = 256;
       launch_extend_group(threads, (int)tn.wideTile, caps.bandW, (int)std::min<uint32_t>(ctas, ns), ctx->R, ctx->dp,
                           ctx->dEml.as<int>(), sp, ns, ws, caps, so, sk, sd, ss, ctr64(ctx) + kExtStatBase, ctx->st);
       std::vector<int32_t> o5((size_t)ns * 5), ok(ns), od(ns);

@@ -279,7 +279,8 @@ int oic_mlp_adam(float *dMaster, float *dM, float *dV, float *dGrad, uint16_t *d
 typedef struct oic_tuning {
   uint32_t narrowArena;   /* kept DP cells per extension in the one-warp bin (default 1 << 20) */
   uint32_t wideMinLen;    /* length-bin boundary, bases of the shorter read (default: none) */
-  uint32_t wideThreads;   /* threads per CTA of the CTA bin: 64 .. 512, a multiple of 32 (default 512) */
+  uint32_t wideThreads;   /* threads per CTA of the CTA bin: 64 .. 512, a multiple of 32 (default 512;
+                             256 in a batch of more extensions than three per SM) */
   uint32_t wideTile;      /* diagonals per thread per pass in the CTA bin: 1, 2 or 4 (default 1) */
   uint32_t wideBandW;     /* shared-memory row width of the CTA bin, ints (default 12288) */
   uint32_t wideCtas;      /* CTAs of the CTA bin (default: 2 per SM) */

@@ -157,7 +157,8 @@ def test_collected_pairs_count_the_reference_extensions(erate, built):
 @pytest.mark.parametrize("erate", [0.12])
 def test_wide_bands_by_warps_and_by_ctas(erate, built):
     """Bands wider than the shared-memory rows: a small batch hands them to the CTA kernel, a
-    large one keeps them on a warp; the results are the same."""
+    large one keeps them on a warp, or on smaller CTAs when these are asked for; the results
+    are the same."""
     r = np.random.default_rng(15)
     seqs, prob = [], []
     for i in range(9):
@@ -172,6 +173,9 @@ def test_wide_bands_by_warps_and_by_ctas(erate, built):
         small = ov.extend_batch(*[a[:, j] for j in range(6)])
         b = np.tile(a, (300, 1))                 # 2,700 problems: more than eight per SM
         large = ov.extend_batch(*[b[:, j] for j in range(6)])
+        ov.set_tuning(forceWide=1)
+        forced = ov.extend_batch(*[b[:, j] for j in range(6)])
     assert (small[1] == 3).any()                 # some reach both ends
-    for s, l in zip(small, large):
-        assert (np.tile(s, (300,) + (1,) * (s.ndim - 1)) == l).all()
+    for s, l, f in zip(small, large, forced):
+        want = np.tile(s, (300,) + (1,) * (s.ndim - 1))
+        assert (want == l).all() and (want == f).all()
