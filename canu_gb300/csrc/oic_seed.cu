@@ -41,11 +41,18 @@
 // occurrences of a k-mer (partner ID above the ref read's) are the tail of its run,
 // which ascends by partner.
 #include "oic_kernels.cuh"
+#include "oic_occurrences.h"
 #include "oic_prims.cuh"
 
 namespace oic {
 
 namespace {
+
+// The block string of occurrence p (the high half of its word).
+struct OccStr {
+  const u64 *occ;
+  __device__ __forceinline__ u32 operator()(u32 p) const { return __ldg((const u32 *)occ + 2 * (u64)p + 1); }
+};
 
 constexpr int kSeedThreads = 256;
 constexpr int kSeedCtas    = 8;      // CTAs per SM
@@ -322,13 +329,7 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
             // The qualifying occurrences are the run's end: it ascends by partner.
             const u32 start = (u32)(val & 0xffffffffull);
             qEnd            = start + (u32)((val >> 32) & 0x7fffffffull);
-            u32 lo = start, hi = qEnd;
-            while (lo < hi) {
-              const u32 mid = (lo + hi) >> 1;
-              if (__ldg((const u32 *)T.occ + 2 * (u64)mid + 1) >= from) hi = mid;
-              else lo = mid + 1;
-            }
-            n = qEnd - lo;
+            n = qEnd - first_occurrence_from(start, qEnd, from, OccStr{T.occ});
           }
         }
       }
