@@ -14,6 +14,7 @@
 
 #include "oic_gpu.h"
 #include "oic_kernels.cuh"
+#include "oic_occurrences.h"
 #include "oic_prims.cuh"
 #include "oic_internal.h"
 
@@ -252,7 +253,7 @@ SeedConfig seed_wide(const oic_ctx *c) {
   s.ctas         = c->nSM;
   s.caps.slotCap = 1 << 17;
   s.caps.pairCap = 1 << 16;
-  s.caps.nodeCap = 1 << 22;
+  s.caps.nodeCap = kSeedNodeCapMax;
   return s;
 }
 

@@ -61,6 +61,9 @@ constexpr int kSeedBuf     = 1024;   // seeds laid out at a time
 constexpr int kSeedPer     = kSeedBuf / kSeedThreads;   // 32-seed chunks a warp lays out
 static_assert(kSeedWarps == 8 && 32 * kSeedPer <= 256, "owners have three bits, ranks a byte");
 constexpr int kOffBits     = 24;     // a packed seed: the ref offset above its 256, the partner's offset below
+static_assert((u64)kSeedThreads * kSeedNodeCapMax <= 1ull << 32, "the seeds of kSeedThreads offsets are counted in 32 bits");
+constexpr u32 kTooMany     = 1u << 16;   // in warpCnt: an offset of the warp has more seeds than there are nodes
+static_assert(kSeedThreads < kTooMany, "the offsets with seeds are counted below the flag");
 static_assert(kSeedThreads <= 256 && kMaxReadLenBits <= kOffBits, "both offsets share a word");
 constexpr int kSeedRecent  = 64;     // recently seen partners per warp
 
@@ -329,21 +332,19 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
             // The qualifying occurrences are the run's end: it ascends by partner.
             const u32 start = (u32)(val & 0xffffffffull);
             qEnd            = start + (u32)((val >> 32) & 0x7fffffffull);
-            n = qEnd - first_occurrence_from(start, qEnd, from, OccStr{T.occ});
+            n = offset_seeds(start, qEnd, from, (u32)cap.nodeCap, OccStr{T.occ});
           }
         }
       }
       // The offsets that have seeds, in order.
       const unsigned has = __ballot_sync(0xffffffffu, n > 0);
       const u32 inc = warp_incl_scan_u32(n);
+      const bool tooMany = __any_sync(0xffffffffu, n == kTooManySeeds);
       if (lane == 31) {
         sm.warpSum[par][wib] = inc;
-        sm.warpCnt[par][wib] = __popc(has);
+        sm.warpCnt[par][wib] = __popc(has) | (tooMany ? kTooMany : 0);
       }
       __syncthreads();
-      // Only a replay sets the flag, and none runs between this barrier and the next: all warps
-      // read the same.  (So it is after the buffer's counts below.)
-      if (sm.overflow) break;
       u32 end = inc, total = 0;
       int c = __popc(has & ((1u << lane) - 1)), nOff = 0;
 #pragma unroll
@@ -355,6 +356,11 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
         nOff += y;
       }
       par ^= 1;
+      // Only a replay sets the flag, and none runs between this barrier and the next: all warps
+      // read the same.  (So it is after the buffer's counts below.)  Where an offset has too
+      // many seeds, all warps see it here and stop here.
+      if (nOff >= (int)kTooMany) sm.overflow = 1;
+      if (sm.overflow) break;
       if (total == 0) continue;
       if (n) {
         sm.end[c]  = end;

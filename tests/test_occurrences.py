@@ -34,6 +34,18 @@ def test_search_finds_the_first_partner_anywhere_in_the_array(base, positions):
             start = base + int(r.integers(0, 5000 - length + 1))
             end = start + length
             for from_ in {0, start // div, (start + length // 2) // div, (start + length // 2) // div + 1, end // div + 1}:
-                queries.append((start, end, from_, div))
+                queries.append(("s", start, end, from_, div))
                 want.append((min(max(start, from_ * div), end), 0))
     assert positions(queries) == want
+
+
+def test_seeds_of_256_offsets_do_not_wrap(positions):
+    """The 32-bit sum of the seeds of 256 ref offsets is the 64-bit one for every run up to the
+    longest that the widest configuration can hold; longer runs are refused, each of them
+    (16,777,216 seeds an offset made the sum 0, and a little more a small number)."""
+    cap = 1 << 22
+    counts = [0, 1, cap - 1, cap, cap + 1, (1 << 24) - 1, 1 << 24, (1 << 24) + 1, (1 << 31) - 1]
+    got = positions([("o", 1000, 1000 + n, 0, 7) for n in counts])
+    assert got == [(256 * n, 0) if n < cap else (0, 256) for n in counts]
+    # Only the occurrences from the first qualifying string on count: the last 70 of 4 strings.
+    assert positions([("o", 0, 280, 3, 70), ("o", 0, 280, 4, 70)]) == [(256 * 70, 0), (0, 0)]
