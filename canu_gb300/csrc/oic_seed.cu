@@ -62,8 +62,6 @@ constexpr int kSeedPer     = kSeedBuf / kSeedThreads;   // 32-seed chunks a warp
 static_assert(kSeedWarps == 8 && 32 * kSeedPer <= 256, "owners have three bits, ranks a byte");
 constexpr int kOffBits     = 24;     // a packed seed: the ref offset above its 256, the partner's offset below
 static_assert((u64)kSeedThreads * kSeedNodeCapMax <= 1ull << 32, "the seeds of kSeedThreads offsets are counted in 32 bits");
-constexpr u32 kTooMany     = 1u << 16;   // in warpCnt: an offset of the warp has more seeds than there are nodes
-static_assert(kSeedThreads < kTooMany, "the offsets with seeds are counted below the flag");
 static_assert(kSeedThreads <= 256 && kMaxReadLenBits <= kOffBits, "both offsets share a word");
 constexpr int kSeedRecent  = 64;     // recently seen partners per warp
 
@@ -79,6 +77,7 @@ struct SeedSmem {
   u32 cnt[kSeedWarps][kSeedWarps / 2];   // seeds per owner and laying warp, two warps to a word
   u32 warpSum[2][kSeedWarps];
   u32 warpCnt[2][kSeedWarps];
+  int tooMany[2];                        // one of these offsets has more seeds than there are nodes
   u32 seg;
   u32 base[2];                           // output places of the strand's nodes and pairs
   int nPairs, nNodes, overflow, screened;
@@ -293,6 +292,7 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
       sm.nNodes   = 1;
       sm.overflow = 0;
       sm.screened = 0;
+      sm.tooMany[0] = sm.tooMany[1] = 0;
     }
     for (int i = tid; i < kSeedWarps * kSeedRecent; i += kSeedThreads) (&sm.recent[0][0])[i] = ~0ull;
     __syncthreads();
@@ -333,18 +333,25 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
             const u32 start = (u32)(val & 0xffffffffull);
             qEnd            = start + (u32)((val >> 32) & 0x7fffffffull);
             n = offset_seeds(start, qEnd, from, (u32)cap.nodeCap, OccStr{T.occ});
+            if (n == kTooManySeeds) {
+              n               = 0;
+              sm.tooMany[par] = 1;
+            }
           }
         }
       }
       // The offsets that have seeds, in order.
       const unsigned has = __ballot_sync(0xffffffffu, n > 0);
       const u32 inc = warp_incl_scan_u32(n);
-      const bool tooMany = __any_sync(0xffffffffu, n == kTooManySeeds);
       if (lane == 31) {
         sm.warpSum[par][wib] = inc;
-        sm.warpCnt[par][wib] = __popc(has) | (tooMany ? kTooMany : 0);
+        sm.warpCnt[par][wib] = __popc(has);
       }
       __syncthreads();
+      // Only a replay sets the flag, and none runs between this barrier and the next: all warps
+      // read the same.  (So it is after the buffer's counts below.)  tooMany is written before
+      // the barrier, its other half before the next one.
+      if (sm.overflow | sm.tooMany[par]) break;
       u32 end = inc, total = 0;
       int c = __popc(has & ((1u << lane) - 1)), nOff = 0;
 #pragma unroll
@@ -356,11 +363,6 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
         nOff += y;
       }
       par ^= 1;
-      // Only a replay sets the flag, and none runs between this barrier and the next: all warps
-      // read the same.  (So it is after the buffer's counts below.)  Where an offset has too
-      // many seeds, all warps see it here and stop here.
-      if (nOff >= (int)kTooMany) sm.overflow = 1;
-      if (sm.overflow) break;
       if (total == 0) continue;
       if (n) {
         sm.end[c]  = end;
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(kSeedThreads, kSeedCtas) seed_kernel(ReadsDev 
     }
     __syncthreads();
     const int  nPairs = min(sm.nPairs, cap.pairCap);
-    const bool ovf    = sm.overflow != 0;
+    const bool ovf    = (sm.overflow | sm.tooMany[0] | sm.tooMany[1]) != 0;
     const bool lscr = sm.screened & 1, rscr = sm.screened & 2;
     if (!ovf) nSeeds += segSeeds;
 
