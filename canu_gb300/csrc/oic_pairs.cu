@@ -346,6 +346,18 @@ __device__ __forceinline__ void team_unlock(TeamPair &p) {
 }
 __device__ __forceinline__ int team_read(const int &v) { return *(const volatile int *)&v; }
 
+// Whether pair p has nodes to claim (by a helper, under its lock).  The owner opens a pair
+// without the lock, its fields first: behind the fence they are the open pair's.
+__device__ __forceinline__ bool team_open(const TeamPair &p) {
+  int open = 0;
+  if ((threadIdx.x & 31) == 0) {
+    open = team_read(p.open);
+    __threadfence_block();
+  }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, open, 0) > 0;
+}
+
 // The best node (length descending, index ascending) whose state lies in [lo, hi]; -1: none.
 __device__ __forceinline__ int best_node(const int4 *nodes, const volatile unsigned char *alive, int cnt, int lo, int hi) {
   int myLen = -1, myIdx = INT_MAX;
@@ -405,7 +417,7 @@ static __device__ __noinline__ void team_help(WarpDP &w, Team &tm, int me) {
       const int      o     = __ffs((int)(above ? above : open)) - 1;
       TeamPair      &p     = tm.pair[o];
       if (team_lock(p)) {
-        if (__shfl_sync(0xffffffffu, team_read(p.open), 0) > 0)
+        if (team_open(p))
           node = best_node(p.nodes, p.alive, p.cnt, kNodeOpen, kNodeOpen);
         if (node >= 0) {
           S    = p.S;
