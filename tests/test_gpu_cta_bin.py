@@ -1,0 +1,70 @@
+"""The CTA bin with more pairs than it has resident CTAs."""
+import numpy as np
+import pytest
+
+import canu_gb300 as oic
+pytestmark = pytest.mark.gpu
+
+
+def noisy(r, g, err):
+    """A copy of g with substitutions, insertions and deletions, a third each."""
+    x = r.random(len(g))
+    out = np.where(x < err / 3, (g + r.integers(1, 4, len(g))) % 4, g)
+    count = 1 + (x >= 2 * err / 3).astype(int) * (x < err) - (x >= err / 3).astype(int) * (x < 2 * err / 3)
+    rid = np.repeat(np.arange(len(g)), count)
+    out = out[rid]
+    extra = np.flatnonzero(rid[1:] == rid[:-1]) + 1
+    out[extra] = r.integers(0, 4, len(extra))
+    return np.frombuffer(b"ACGT", np.uint8)[out].tobytes()
+
+
+def pairs_of_reads(r, n, length, err):
+    """n pairs of reads, each pair of a template of its own."""
+    seqs = []
+    for _ in range(n):
+        g = r.integers(0, 4, length)
+        seqs += [noisy(r, g, err), noisy(r, g, err)]
+    return seqs
+
+
+def run(seqs, reps=1, **tuning):
+    off = np.cumsum([0] + [len(x) for x in seqs])
+    with oic.Overlapper(oic.default_params(kmerLen=22, hashBits=20, maxErate=0.12, minOlapLen=300)) as ov:
+        ov.set_reads(np.ones(len(seqs)), [len(x) for x in seqs], off[:-1], np.frombuffer(b"".join(seqs), np.uint8))
+        ov.set_tuning(**tuning)
+        ms = []
+        for _ in range(reps):
+            ov.clear()
+            ov.run()
+            ms.append(ov.stats()["msWide"])
+        return oic.sort_records(ov.overlaps()), ov.stats(), min(ms)
+
+
+@pytest.fixture(scope="module")
+def reads():
+    r = np.random.default_rng(21)
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    # One long pair more than there are SMs, and short ones that keep every SM busy about as
+    # long as a long pair takes.
+    return sms, pairs_of_reads(r, sms + 1, 7000, 0.05) + pairs_of_reads(r, 2500, 900, 0.05)
+
+
+def test_records_do_not_depend_on_the_bin(reads, built):
+    sms, seqs = reads
+    warps, sw, _ = run(seqs)
+    ctas, sc, _ = run(seqs, forceWide=1)
+    assert sc["pairsWide"] > 2 * 2 * sms and len(ctas) > 2500
+    assert np.array_equal(warps, ctas)
+    for k in ("kmerHitsWithoutOlap", "kmerHitsWithOlap", "totalOverlaps", "containedOverlaps", "dovetailOverlaps"):
+        assert sw[k] == sc[k], k
+
+
+def test_longest_pairs_start_first_whatever_the_number_of_ctas(reads, built):
+    """CTAs that wait for an SM hold no pair meanwhile: three CTAs for each SM take no longer
+    than one (a long pair dealt to a waiting CTA starts when the short ones are done: half as
+    long again)."""
+    sms, seqs = reads
+    _, _, one = run(seqs, 4, forceWide=1, wideCtas=sms)
+    _, _, three = run(seqs, 4, forceWide=1, wideCtas=3 * sms)
+    assert three < 1.15 * one, (one, three)
