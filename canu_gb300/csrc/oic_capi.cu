@@ -1094,11 +1094,11 @@ int ensure_pair_caps(oic_ctx *ctx) {
   return OIC_OK;
 }
 
-// CTAs of the CTA bin: as many per SM (at most 2) as the row buffers leave room for
-// in the SM's 227 KB of shared memory.
+// CTAs of the CTA bin: as many as the SMs hold at a time, at most 2 each -- one of the
+// default 512 threads, two of 256.  (Two per SM whatever the threads left half of the CTAs,
+// 77 MB of arena, rows and headers each, waiting for a place: 11.8 GB.)
 uint32_t resolved_tuning_ctas(const oic_ctx *c, const oic_tuning &t) {
-  const size_t per = (size_t)2 * t.wideBandW * sizeof(int) + 4096;
-  const int    k   = (int)std::max<size_t>(1, std::min<size_t>(2, (227u << 10) / per));
+  const int k = std::max(1, std::min(2, group_ctas_per_sm((int)t.wideThreads, (int)t.wideBandW)));
   return (uint32_t)(k * c->nSM);
 }
 
@@ -1836,16 +1836,21 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
       int *so = (int *)(sp + ns), *sk = so + 5 * (size_t)ns, *sd = sk + ns;
       uint32_t *ss = (uint32_t *)(sd + ns);
       CK(cudaMemcpyAsync(sp, sub.data(), ns * sizeof(ExtendProblem), cudaMemcpyHostToDevice, ctx->st));
-      uint32_t    ctas = 0;
-      AlignCaps   caps;
-      WarpScratch ws;
-      if ((rc = ensure_group_scratch(ctx, tn, pass == 2, ctas, caps, ws))) break;
       // More problems than three per SM: two CTAs of 256 threads on one where the default is
       // 512 (noisy extensions: 4,000 of 15 kb reads 15.3 against 23.3 ms, 1,000 of 30 kb reads
       // 16.4 and 18.3, but 400 of them 8.9 and 8.5 and 230 of 60 kb reads 19.4 and 14.2).
-      int threads = pass == 2 ? (int)std::max<uint32_t>(tn.wideThreads, 512) : (int)tn.wideThreads;
-      if (pass == 1 && !ctx->tune.wideThreads && ns > 3u * (uint32_t)ctx->nSM) threads = 256;
-      launch_extend_group(threads, (int)tn.wideTile, caps.bandW, (int)std::min<uint32_t>(ctas, ns), ctx->R, ctx->dp,
+      oic_tuning tg = tn;
+      if (pass == 2) tg.wideThreads = std::max<uint32_t>(tn.wideThreads, 512);
+      else if (!ctx->tune.wideThreads && ns > 3u * (uint32_t)ctx->nSM) tg.wideThreads = 256;
+      // Two CTAs per SM (where an SM has room for the rows of two), although one of 512 threads
+      // lives on it: the problems are dealt to the CTAs, and a CTA for each problem starts when
+      // a place is free (230 extensions of 60 kb reads by 230 CTAs 15.6 ms, by 152 CTAs 19.3).
+      if (!ctx->tune.wideCtas) tg.wideCtas = (tn.wideBandW <= 14000 ? 2u : 1u) * (uint32_t)ctx->nSM;
+      uint32_t    ctas = 0;
+      AlignCaps   caps;
+      WarpScratch ws;
+      if ((rc = ensure_group_scratch(ctx, tg, pass == 2, ctas, caps, ws))) break;
+      launch_extend_group((int)tg.wideThreads, (int)tg.wideTile, caps.bandW, (int)std::min<uint32_t>(ctas, ns), ctx->R, ctx->dp,
                           ctx->dEml.as<int>(), sp, ns, ws, caps, so, sk, sd, ss, ctr64(ctx) + kExtStatBase, ctx->st);
       std::vector<int32_t> o5((size_t)ns * 5), ok(ns), od(ns);
       std::vector<uint32_t> os(ns);

@@ -129,6 +129,9 @@ void launch_align_group(int threads, int U, int bandW, int ctas, ReadsDev R, Tab
                         const PairRec *pairs, const u32 *work, u32 nWork, u32 *workCounter, const int4 *nodes,
                         WarpScratch sc, AlignCaps cap, AlignOut out, cudaStream_t st);
 
+// CTAs of the CTA bin that an SM holds at a time, with bandW-int shared-memory rows.
+int group_ctas_per_sm(int threads, int bandW);
+
 // Speculative CTA bin: one pair per CTA of align_spec_warps() warps, each warp running
 // whole extensions (one-warp DP, HBM rows up to cap.rowsGW) of the pair's next alive match nodes, replayed in the reference's order.
 // sc/cap describe ctas * align_spec_warps() warp scratches; a pair's alive flags use the

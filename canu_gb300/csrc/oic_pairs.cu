@@ -1335,6 +1335,14 @@ void launch_align_group(int threads, int U, int bandW, int ctas, ReadsDev R, Tab
   g_launches++;
 }
 
+int group_ctas_per_sm(int threads, int bandW) {
+  const size_t smem = (size_t)2 * bandW * sizeof(int);
+  int k = 0;
+  cudaFuncSetAttribute(align_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, align_group_kernel, threads, smem) != cudaSuccess) return 0;
+  return k;
+}
+
 void launch_align_spec(int ctas, ReadsDev R, TableDev T, DevParams P, const int *eml, const PairRec *pairs,
                        const u32 *work, u32 nWork, u32 *workCounter, const int4 *nodes, WarpScratch sc, AlignCaps cap,
                        AlignOut out, cudaStream_t st) {

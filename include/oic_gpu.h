@@ -283,7 +283,9 @@ typedef struct oic_tuning {
                              256 in a batch of more extensions than three per SM) */
   uint32_t wideTile;      /* diagonals per thread per pass in the CTA bin: 1, 2 or 4 (default 1) */
   uint32_t wideBandW;     /* shared-memory row width of the CTA bin, ints (default 12288) */
-  uint32_t wideCtas;      /* CTAs of the CTA bin (default: 2 per SM) */
+  uint32_t wideCtas;      /* CTAs of the CTA bin (default: as many as the SMs hold at a time, at
+                             most 2 per SM -- 1 of 512 threads, 2 of 256; 2 per SM in a batch of
+                             extensions) */
   uint64_t wideArena;     /* kept DP cells per CTA of the CTA bin (default: 2^24, less if memory is short) */
   uint32_t forceWide;     /* testing: every pair goes to the CTA bin (0 / 1) */
   uint32_t noGraph;       /* 1: launch the DP stage kernel by kernel with host-read sizes instead of

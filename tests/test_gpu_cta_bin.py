@@ -68,3 +68,16 @@ def test_longest_pairs_start_first_whatever_the_number_of_ctas(reads, built):
     _, _, one = run(seqs, 4, forceWide=1, wideCtas=sms)
     _, _, three = run(seqs, 4, forceWide=1, wideCtas=3 * sms)
     assert three < 1.15 * one, (one, three)
+
+
+@pytest.mark.parametrize("tuning,per_sm", [({}, 1), ({"wideThreads": 256}, 2), ({"wideThreads": 64}, 2),
+                                           ({"wideThreads": 256, "wideBandW": 25600}, 1)])
+def test_default_ctas_are_those_the_sms_hold(tuning, per_sm, built):
+    """No CTA of the default grid waits for an SM with its arena, rows and headers idle:
+    128 registers a thread let one CTA of 512 threads, or two of 256, live on an SM, and
+    200 KB of rows one."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    with oic.Overlapper(oic.default_params(kmerLen=22)) as ov:
+        ov.set_tuning(**tuning)
+        assert ov.tuning()["wideCtas"] == per_sm * sms
