@@ -1806,16 +1806,18 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
   // tuning forces the CTA bin, else those that overflowed); pass 2: the large arena.
   DevBuf dSub;
   std::vector<uint32_t> idx;
+  // Few problems: a band wider than the shared-memory rows is the CTA's at once.  Many
+  // keep every warp busy, and wide rows in HBM then cost less than a CTA per problem.
+  // 230 / 1,000 / 4,000 noisy extensions of 30 kb reads: 7.2 / 18.1 / 55.5 ms by the CTA,
+  // 20.1 / 21.2 / 47.1 by the warps; of 15 kb reads 3.4 / 6.6 / 18.9 and 6.1 / 7.3 / 10.1.
+  bool wideByWarps = nAlign > 8u * (uint32_t)ctx->nSM;
+  const uint64_t cells0 = ctx->stats.dpCells, slides0 = ctx->stats.slideBases;
   for (int pass = tn.forceWide ? 1 : 0; pass < 3 && rc == OIC_OK; pass++) {
     CK(cudaMemsetAsync(ctr64(ctx) + kExtStatBase, 0, 2 * sizeof(unsigned long long), ctx->st));
     if (pass == 0) {
       AlignConfig ac = align_normal(ctx);
       ac.caps.arenaCap = (int)tn.narrowArena;
-      // Few problems: a band wider than the shared-memory rows is the CTA's at once.  Many
-      // keep every warp busy, and wide rows in HBM then cost less than a CTA per problem.
-      // 230 / 1,000 / 4,000 noisy extensions of 30 kb reads: 7.2 / 18.1 / 55.5 ms by the CTA,
-      // 20.1 / 21.2 / 47.1 by the warps; of 15 kb reads 3.4 / 6.6 / 18.9 and 6.1 / 7.3 / 10.1.
-      if (nAlign <= 8u * (uint32_t)ctx->nSM) ac.caps.rowsGW = ac.caps.bandW;
+      if (!wideByWarps) ac.caps.rowsGW = ac.caps.bandW;
       WarpScratch ws;
       if ((rc = ensure_align_scratch(ctx, ac, false, ws))) break;
       launch_extend_batch(ctx->R, ctx->dp, ctx->dEml.as<int>(), dP.as<ExtendProblem>(), nAlign, ws,
@@ -1849,7 +1851,19 @@ int oic_extend_batch(oic_ctx *ctx, uint32_t nAlign, const uint32_t *sRead, const
       uint32_t    ctas = 0;
       AlignCaps   caps;
       WarpScratch ws;
-      if ((rc = ensure_group_scratch(ctx, tg, pass == 2, ctas, caps, ws))) break;
+      rc = ensure_group_scratch(ctx, tg, pass == 2, ctas, caps, ws);
+      if (rc == OIC_ERR_NOMEM && pass == 1 && !wideByWarps && !tn.forceWide) {
+        // No memory for the CTAs' arenas: the warps' HBM rows hold most wide bands too.
+        cudaGetLastError();
+        ctx->dArena2.release();
+        ctx->stats.dpCells    = cells0;
+        ctx->stats.slideBases = slides0;
+        wideByWarps = true;
+        rc          = OIC_OK;
+        pass        = -1;   // from the one-warp pass again
+        continue;
+      }
+      if (rc) break;
       launch_extend_group((int)tg.wideThreads, (int)tg.wideTile, caps.bandW, (int)std::min<uint32_t>(ctas, ns), ctx->R, ctx->dp,
                           ctx->dEml.as<int>(), sp, ns, ws, caps, so, sk, sd, ss, ctr64(ctx) + kExtStatBase, ctx->st);
       std::vector<int32_t> o5((size_t)ns * 5), ok(ns), od(ns);
