@@ -24,6 +24,7 @@
 #include "oic_gpu.h"
 #include "oic_common.cuh"
 #include "oic_prims.cuh"
+#include "oic_store_layout.h"
 
 namespace oic {
 namespace {
@@ -142,18 +143,11 @@ unsigned grid_of(u64 n) {
   return (unsigned)(g ? g : 1);
 }
 
-// The call's device memory: one allocation, freed on scope exit, laid out by take().
-struct Arena {
-  char  *p    = nullptr;
-  size_t used = 0;
-  ~Arena() {
+// Device memory freed on scope exit.
+struct DevMem {
+  char *p = nullptr;
+  ~DevMem() {
     if (p) cudaFree(p);
-  }
-  size_t room(size_t n) { return (n + 255) & ~(size_t)255; }
-  template <class T> T *take(size_t bytes) {
-    char *q = p + used;
-    used += room(bytes);
-    return (T *)q;
   }
 };
 
@@ -182,33 +176,32 @@ extern "C" int oic_store_sort(int device, const uint32_t *words, uint64_t nRecor
     cudaError_t e_ = (x);                                                                       \
     if (e_ != cudaSuccess) return e_ == cudaErrorMemoryAllocation ? OIC_ERR_NOMEM : OIC_ERR_CUDA; \
   } while (0)
-  Arena mem;
-  const size_t ids = ((size_t)maxID + 2) * 4;
-  TRY(cudaMalloc(&mem.p, mem.room(nRecords * 24) + 2 * mem.room(n2 * 24) + 3 * mem.room(n2 * 8) + 2 * mem.room(n2 * 4) +
-                             2 * mem.room((n2 + 1) * 4) + mem.room(scr) + mem.room(8 * 8 + 4 * 4) + 2 * mem.room(ids)));
-  uint32_t           *dIn   = mem.take<uint32_t>(nRecords * 24);
-  uint32_t           *dRec  = mem.take<uint32_t>(n2 * 24);
-  uint32_t           *dOut  = mem.take<uint32_t>(n2 * 24);
-  u64                *dKeys = mem.take<u64>(n2 * 8);
-  u64                *dK2   = mem.take<u64>(n2 * 8);
-  u64                *dK3   = mem.take<u64>(n2 * 8);
-  uint32_t           *dIdx  = mem.take<uint32_t>(n2 * 4);
-  uint32_t           *dIdx2 = mem.take<uint32_t>(n2 * 4);
-  uint32_t           *dKeep = mem.take<uint32_t>((n2 + 1) * 4);
-  uint32_t           *dPos  = mem.take<uint32_t>((n2 + 1) * 4);
-  void               *dScr  = mem.take<char>(scr);
-  unsigned long long *cnt   = mem.take<unsigned long long>(8 * 8 + 4 * 4);   // 8 counters, then the compaction total
+  const StoreLayout at  = store_layout(nRecords, maxID, scr);
+  const size_t      ids = ((size_t)maxID + 2) * 4;
+  DevMem mem;
+  TRY(cudaMalloc(&mem.p, at.bytes));
+  uint32_t           *dIn   = (uint32_t *)(mem.p + at.in);
+  u64                *dKeys = (u64 *)(mem.p + at.keys);
+  uint32_t           *dKeep = (uint32_t *)(mem.p + at.keep);
+  uint32_t           *dPos  = (uint32_t *)(mem.p + at.pos);
+  uint32_t           *dRec  = (uint32_t *)(mem.p + at.rec);
+  u64                *dK2   = (u64 *)(mem.p + at.k2);
+  u64                *dK3   = (u64 *)(mem.p + at.k3);
+  uint32_t           *dIdx  = (uint32_t *)(mem.p + at.idx);
+  uint32_t           *dIdx2 = (uint32_t *)(mem.p + at.idx2);
+  void               *dScr  = mem.p + at.scr;
+  unsigned long long *cnt   = (unsigned long long *)(mem.p + at.cnt);
   uint32_t           *total = (uint32_t *)(cnt + 8);
-  uint32_t           *dA    = mem.take<uint32_t>(ids);
-  uint32_t           *dAOff = mem.take<uint32_t>(ids);
+  uint32_t           *dA    = (uint32_t *)(mem.p + at.a);
+  uint32_t           *dAOff = (uint32_t *)(mem.p + at.aOff);
+  uint32_t           *dOut  = (uint32_t *)(mem.p + at.out);   // over dIn, dKeys, dKeep and dPos
   TRY(cudaMemsetAsync(cnt, 0, 8 * 8 + 4 * 4, st));
   TRY(cudaMemsetAsync(dA, 0, ids, st));
   TRY(cudaMemsetAsync(dKeep + n2, 0, 4, st));
   if (nRecords) TRY(cudaMemcpyAsync(dIn, words, nRecords * 24, cudaMemcpyHostToDevice, st));
 
   if (nRecords) {
-    store_expand_kernel<<<grid_of(nRecords), 256, 0, st>>>(dIn, nRecords, maxID, maxEvalue, idBits,
-                                                           dRec, dKeys, dKeep,
+    store_expand_kernel<<<grid_of(nRecords), 256, 0, st>>>(dIn, nRecords, maxID, maxEvalue, idBits, dRec, dKeys, dKeep,
                                                            cnt);
     g_launches++;
   }
@@ -219,19 +212,16 @@ extern "C" int oic_store_sort(int device, const uint32_t *words, uint64_t nRecor
   uint32_t m = 0;
   if (n2) {
     TRY(scan_u32(dKeep, dPos, n2, total, dScr, st));
-    store_compact_kernel<<<grid_of(n2), 256, 0, st>>>(dKeys, dKeep, dPos, n2,
-                                                      dK2, dIdx);
+    store_compact_kernel<<<grid_of(n2), 256, 0, st>>>(dKeys, dKeep, dPos, n2, dK2, dIdx);
     g_launches++;
     TRY(cudaMemcpyAsync(&m, total, 4, cudaMemcpyDeviceToHost, st));
     TRY(cudaStreamSynchronize(st));
   }
   if (m) {
-    TRY(radix_sort_u64_u32((unsigned long long *)dK2, dIdx, (unsigned long long *)dK3,
-                           dIdx2, m, 2 * idBits, dScr, st));
+    TRY(radix_sort_u64_u32((unsigned long long *)dK2, dIdx, (unsigned long long *)dK3, dIdx2, m, 2 * idBits, dScr, st));
     store_ties_kernel<<<grid_of(m), 256, 0, st>>>(dK2, dIdx, dRec, m);
     g_launches++;
-    store_gather_kernel<<<grid_of(m), 256, 0, st>>>(dRec, dIdx, m, dOut,
-                                                    dA);
+    store_gather_kernel<<<grid_of(m), 256, 0, st>>>(dRec, dIdx, m, dOut, dA);
     g_launches++;
     TRY(cudaMemcpyAsync(out, dOut, (size_t)m * 24, cudaMemcpyDeviceToHost, st));
   }
