@@ -621,6 +621,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
   const ReadView S = make_view(R, sRead, rev);
   const ReadView T = make_view(R, tRead, 0);
   const unsigned long long cells0 = w.cells, slides0 = w.slides, rows0 = w.rows;
+  const unsigned long long slidesCta0 = GROUP ? w.gs->slides : 0;   // the CTA's row loops count theirs there
 
   // Pairs that run one extension, or stop after a few without an overlap, are not opened.
   const bool open = !GROUP && cnt > 1 && !cons && extLimit == 0;
@@ -760,6 +761,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     w.cells  = cells0;
     w.slides = slides0;
     w.rows   = rows0;
+    if (GROUP && lane == 0) w.gs->slides = slidesCta0;   // the other warps wait for a row loop
     return false;
   }
 

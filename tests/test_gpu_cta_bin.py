@@ -81,3 +81,17 @@ def test_default_ctas_are_those_the_sms_hold(tuning, per_sm, built):
     with oic.Overlapper(oic.default_params(kmerLen=22)) as ov:
         ov.set_tuning(**tuning)
         assert ov.tuning()["wideCtas"] == per_sm * sms
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_reruns_leave_no_counts_behind(graph, built):
+    """Pairs whose extension does not fit a CTA's arena are discarded and run again in the
+    large one: cells, rows and slide bases are those of a run whose arenas are large enough."""
+    r = np.random.default_rng(23)
+    seqs = pairs_of_reads(r, 3, 30000, 0.05) + pairs_of_reads(r, 20, 2000, 0.05)
+    small, ss, _ = run(seqs, forceWide=1, noGraph=1 - graph, wideArena=1 << 20)
+    large, sl, _ = run(seqs, forceWide=1, noGraph=1 - graph)
+    assert ss["pairsWide"] > sl["pairsWide"]          # pairs were run again
+    assert len(large) == 23 and np.array_equal(small, large)
+    for k in ("dpCells", "dpRows", "extensions", "slideBases"):
+        assert ss[k] == sl[k], (k, ss[k], sl[k])
