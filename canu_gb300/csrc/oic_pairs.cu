@@ -193,6 +193,7 @@ struct PairSmem {
   int                nExt;       // extensions run for the pair in flight
   int                firstHit;   // index of its first extension that added an overlap, -1 none
   unsigned long long cellsFirst; // DP cells of its first extension
+  long long          cellsInfo;  // collected pairs: DP cells of its extensions beyond those counted as work
   ExtRes             res;        // its latest extension
   PairCounts         pc;    // counts of the pair in flight
   PairCounts         acc;   // committed counts of the warp
@@ -277,6 +278,23 @@ __device__ __forceinline__ void extend_node(WarpDP &w, const ReadView &S, int sL
   __syncwarp();
 }
 
+// Collected pairs: extends a node shown to have no overlap, for the pair's own figures (how
+// many extensions, and their cells); the work counters are those of a run that does not
+// collect.  Returns false on a capacity overflow.
+static __device__ __noinline__ bool extend_proved(WarpDP &w, PairSmem &ps, const ReadView &S, int sLen,
+                                                  const ReadView &T, int tLen, int4 lm,
+                                                  volatile unsigned char &alive) {
+  extend_node(w, S, sLen, T, tLen, lm, ps.res);
+  w.err |= ps.res.err;
+  if ((threadIdx.x & 31) == 0) {
+    alive = 0;   // kNodeDead
+    ps.nExt++;
+    ps.cellsInfo += (long long)ps.res.cells;
+  }
+  __syncwarp();
+  return w.err == 0;
+}
+
 // ---------------------------------------------------------------------------------
 // The team of a one-warp DP CTA.  Each warp takes pairs of its own; a warp that finds the
 // work list empty helps the others of its CTA.  Process_Matches extends, one after
@@ -300,7 +318,7 @@ __device__ __forceinline__ void extend_node(WarpDP &w, const ReadView &S, int sL
 // stays readable).
 enum { kSlotFree = 0, kSlotRunning = 1, kSlotDone = 2, kSlotCancelled = 3 };
 constexpr unsigned char kNodeDead = 0, kNodeOpen = 1, kNodeOwner = 2, kNodeHelper = 3;   // kNodeHelper + h: helper h
-constexpr unsigned char kNodeProved = 255;   // collected pairs only: shown to have no overlap, still to be counted
+constexpr unsigned char kNodeProved = 255;   // collected pairs only: shown to have no overlap, still to be extended for the pair's figures
 
 struct TeamPair {            // a pair open to helpers
   int            lock;
@@ -484,7 +502,7 @@ __device__ __forceinline__ bool team_wait(Team &tm, int h) {
 // It is tried when its cells are estimated at less than half the work of extending the
 // group, from the last extension's cells and rows and the measured instructions of each.
 constexpr int kProofSpan = 64;
-static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, const ReadView &S, int sLen, const ReadView &T, int tLen,
+static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, PairSmem &ps, const ReadView &S, int sLen, const ReadView &T, int tLen,
                                                         const int4 *nodes, int cnt, volatile unsigned char *alive,
                                                         float extCells, float extRows, Team *tm, int me, bool open) {
   const int lane = threadIdx.x & 31;
@@ -512,7 +530,10 @@ static __device__ __noinline__ bool drop_hopeless_group(WarpDP &w, const ReadVie
   if (min(dhi + E, tLen - 1) - max(dlo - E, 1 - sLen) + 1 > kProofDiags) return true;
   const float proof = (float)E * (60.0f + 3.0f * (1.5f * (float)E + (float)(dhi - dlo)));
   if (2.0f * proof > (float)n * (3000.0f + 150.0f * extRows + 6.0f * extCells)) return true;
-  if (!no_path_within(w, S, sLen, T, tLen, dlo, dhi, E)) return false;
+  const unsigned long long cells0 = w.cells;
+  const bool none = no_path_within(w, S, sLen, T, tLen, dlo, dhi, E);
+  if (lane == 0) ps.cellsInfo -= (long long)(w.cells - cells0);   // no extension's
+  if (!none) return false;
   if (open && !team_lock(tm->pair[me])) {
     w.err |= kErrInternal;
     return false;
@@ -550,6 +571,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     ps.nExt       = 0;
     ps.firstHit   = -1;
     ps.cellsFirst = 0;
+    ps.cellsInfo  = 0;
   }
   __syncwarp();
   nRec = 0;
@@ -647,7 +669,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     if (open && !team_lock(tm->pair[me])) { w.err |= kErrInternal; break; }
     const int li = best_node(nodes, alive, cnt, kNodeOpen, 255);
     int h = -1;
-    // A node shown to have no overlap has its turn among the pair's extensions, and is gone.
+    // A node shown to have no overlap has its turn among the collected pair's extensions.
     const bool proved = P.collect && li >= 0 && alive[li] == kNodeProved;
     if (open) {
       if (li >= 0 && !proved) {
@@ -661,13 +683,8 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
       team_unlock(tm->pair[me]);
     }
     if (li < 0) break;
-    if (proved) {
-      __syncwarp();
-      if (lane == 0) {
-        alive[li] = kNodeDead;
-        ps.nExt++;
-      }
-      __syncwarp();
+    if (!GROUP && proved) {
+      if (!extend_proved(w, ps, S, sLen, T, tLen, nodes[li], alive[li])) break;
       continue;
     }
 
@@ -750,7 +767,7 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
     if (h >= 0 && lane == 0) atomicExch(&tm->slot[h].state, kSlotFree);   // the deltas have been read
     __syncwarp();
     if (!GROUP && !dov && extLimit == 0 && proofs > 0) {
-      if (!drop_hopeless_group(w, S, sLen, T, tLen, nodes, cnt, alive, (float)(w.cells - cellsExt),
+      if (!drop_hopeless_group(w, ps, S, sLen, T, tLen, nodes, cnt, alive, (float)(w.cells - cellsExt),
                                (float)(w.rows - rowsExt), tm, me, open))
         proofs--;
       if (w.err) break;
@@ -836,7 +853,7 @@ static __device__ __forceinline__ void align_loop(WarpDP &w, PairSmem &ps, const
         if (nRec == 0) ps.pc.v[kStCellsNoOlap] += w.cells - cellsBefore;
         out.cnt[pi] = nRec;
         if (out.cells) {
-          const unsigned long long c = w.cells - cellsBefore;
+          const unsigned long long c = w.cells - cellsBefore + (unsigned long long)ps.cellsInfo;
           out.cells[pi] = c > 0xffffffffull ? 0xffffffffu : (u32)c;
           out.ext[pi]   = make_int4(ps.nExt, ps.firstHit,
                                     ps.cellsFirst > 0x7fffffffull ? 0x7fffffff : (int)ps.cellsFirst, extLimit);

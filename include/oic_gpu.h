@@ -200,9 +200,11 @@ typedef struct oic_pair_info {
   uint32_t seeds;      /* k-mer seeds of the pair (diag_ct) */
   uint32_t nodes;      /* match runs of the pair (its nodes in oic_get_pairs' node array) */
   uint32_t overlaps;   /* records the DP emitted for the pair */
-  uint32_t cells;      /* DP cells spent on the pair (saturating); as dpCells of oic_stats, work done */
+  uint32_t cells;      /* DP cells of the pair's extensions (saturating) */
   float    score;      /* filter logit (0 when no filter is set) */
-  uint32_t extensions; /* the reference's Extend_Alignment calls for the pair */
+  uint32_t extensions; /* the reference's Extend_Alignment calls for the pair; a run that collects
+                          also extends the match nodes shown to have no overlap together, which
+                          oic_stats counts as it does without collection */
   int32_t  firstHit;   /* index of the first of them that added an overlap, -1 none */
   uint32_t cellsFirst; /* DP cells of the pair's first extension */
   uint32_t extLimit;   /* 1 when the filter's single-extension tier applied, else 0 */
