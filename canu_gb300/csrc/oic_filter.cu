@@ -28,6 +28,7 @@
 // Tensor-core use: mma.sync.m16n8k16 (FP16 in, FP32 accumulate) with ldmatrix
 // fragment loads from shared memory.  One warp owns 16 samples at a time; layer 1's
 // accumulator fragments are repacked in registers as layer 2's A fragments.
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
 #include "oic_gpu.h"
@@ -35,6 +36,8 @@
 #include "oic_prims.cuh"
 
 namespace oic {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -78,6 +81,10 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const u32 (&a)[4], u32 b
 __device__ __forceinline__ u32 pack_h2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<u32 *>(&h);
+}
+// acc += the two halves of v, each converted exactly and added in FP32.
+__device__ __forceinline__ void add_halves(float &acc, u32 v) {
+  asm("{.reg .f16 l, h; mov.b32 {l, h}, %1; add.rn.f32.f16 %0, l, %0; add.rn.f32.f16 %0, h, %0;}" : "+f"(acc) : "r"(v));
 }
 __device__ __forceinline__ float2 unpack_h2(u32 v) {
   __half2 h = *reinterpret_cast<__half2 *>(&v);
@@ -398,30 +405,37 @@ __global__ void __launch_bounds__(kBwdWarps * 32) mlp_bwd_hidden_kernel(const __
 }
 
 // grad W[m][c] += sum_s G[s][m] * H[s][c]   (M = 128, N = NC columns of H)
-// grad b[m]    += sum_s G[s][m]             (as the product with a column of ones)
+// grad b[m]    += sum_s G[s][m]             (in FP32)
 // for both layers in one launch: blocks of y 0 take layer 2 (G2, H1), of y 1 layer 1 (G1, X).
 // Each block takes a contiguous range of samples in steps of 64.
 //
 // What bounds it is the latency of a step and the FP32 atomics of a block's 128 x NC sums.
 // One launch per layer in blocks of at least 1,024 samples put 32 blocks on 152 SMs (87 + 81
 // us at 32,768 samples; now 25 us for both), and a serial sum over the rows for the bias was
-// half of a step.
+// half of a step.  The bias is added up from the A fragments by all lanes, in FP32 with the
+// mixed-precision add (a product with a column of ones takes as long, but the tensor cores'
+// sums are less exact; converting first costs 3 to 9 us more), and over the eight blocks of a
+// cluster before it goes to memory: an atomic per 256 samples rounded the whole sum four
+// times as often as one per 1,024.  Rms error over the sum of magnitudes at 1,000 / 32,768 /
+// 60,000 samples: product and atomics 1.2 / 1.4 / 1.6e-7, one thread a column over blocks of
+// 1,024 samples 1.2 / 0.8 / 0.9e-7, this 0.2 / 0.3 / 0.4e-7.
 constexpr int kWgWarps = 8;
 constexpr int kWgRows  = 64;
 constexpr u32 kWgMin   = 256;
+constexpr int kWgCluster = 8;
 
 struct WgSmem {
   __half g[kWgRows * kHS];
   __half h[kWgRows * kHS];
+  float  bias[kHid];
 };
 
 template <int NC>
 __device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __half *H, u32 n, u32 perBlock,
                                             float *gradW, float *gradB) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  constexpr int NT   = NC / 8;
-  constexpr u32 kOne = 0x3c003c00u;   // two FP16 ones
-  float acc[NT][4], bsum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  constexpr int NT = NC / 8;
+  float acc[NT][4], b0 = 0.0f, b1 = 0.0f, c0 = 0.0f, c1 = 0.0f;   // b, c: rows g and g + 8 of the fragments, this lane's samples
 #pragma unroll
   for (int i = 0; i < NT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
   const u64 s0 = (u64)blockIdx.x * perBlock;
@@ -437,7 +451,10 @@ __device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __
       // A[m][k] = G[k][m]: stored [k][m], transposed ldmatrix.
       u32 a[4];
       ldsm_x4_t(a, s.g + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * kHS + m0 + ((lane >> 3) & 1) * 8);
-      mma16816(bsum, a, kOne, kOne);
+      add_halves(b0, a[0]);
+      add_halves(c0, a[2]);
+      add_halves(b1, a[1]);
+      add_halves(c1, a[3]);
 #pragma unroll
       for (int np = 0; np < NT / 2; np++) {
         u32 b[4];
@@ -448,21 +465,40 @@ __device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __
     }
   }
   const int g = lane >> 2, t = lane & 3;
+  // Bias: the four lanes of a row, then the cluster's blocks (its first block adds them up).
+  b0 += c0;
+  b1 += c1;
 #pragma unroll
-  for (int nt = 0; nt < NT; nt++) {
-    const int c = nt * 8 + 2 * t;
-    atomicAdd(&gradW[(m0 + g) * NC + c], acc[nt][0]);
-    atomicAdd(&gradW[(m0 + g) * NC + c + 1], acc[nt][1]);
-    atomicAdd(&gradW[(m0 + g + 8) * NC + c], acc[nt][2]);
-    atomicAdd(&gradW[(m0 + g + 8) * NC + c + 1], acc[nt][3]);
+  for (int o = 1; o < 4; o <<= 1) {
+    b0 += __shfl_xor_sync(0xffffffffu, b0, o);
+    b1 += __shfl_xor_sync(0xffffffffu, b1, o);
   }
-  if (t == 0) {   // every column of the product with ones is the sum
-    atomicAdd(&gradB[m0 + g], bsum[0]);
-    atomicAdd(&gradB[m0 + g + 8], bsum[2]);
+  if (t == 0) {
+    s.bias[m0 + g]     = b0;
+    s.bias[m0 + g + 8] = b1;
   }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();
+  if (s0 < n) {
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) {
+      const int c = nt * 8 + 2 * t;
+      atomicAdd(&gradW[(m0 + g) * NC + c], acc[nt][0]);
+      atomicAdd(&gradW[(m0 + g) * NC + c + 1], acc[nt][1]);
+      atomicAdd(&gradW[(m0 + g + 8) * NC + c], acc[nt][2]);
+      atomicAdd(&gradW[(m0 + g + 8) * NC + c + 1], acc[nt][3]);
+    }
+  }
+  cluster.barrier_wait();
+  if (cluster.block_rank() == 0 && threadIdx.x < kHid) {
+    float sum = 0.0f;
+    for (int r = 0; r < kWgCluster; r++) sum += *cluster.map_shared_rank(&s.bias[threadIdx.x], r);
+    atomicAdd(&gradB[threadIdx.x], sum);
+  }
+  cluster.sync();   // no block leaves while its sums are read
 }
 
-__global__ void __launch_bounds__(kWgWarps * 32) mlp_wgrad_kernel(const __half *G2, const __half *H1, const __half *G1,
+__global__ void __cluster_dims__(kWgCluster, 1, 1) __launch_bounds__(kWgWarps * 32) mlp_wgrad_kernel(const __half *G2, const __half *H1, const __half *G1,
                                                                  const __half *X, u32 n, u32 perBlock, float *grad) {
   __shared__ __align__(16) WgSmem s;
   if (blockIdx.y == 0) wgrad_block<kHid>(s, G2, H1, n, perBlock, grad + kOffW2, grad + kOffB2);
@@ -546,7 +582,8 @@ cudaError_t launch_mlp_backward(const void *prm, const void *X, const void *H1, 
   // with at least 128 / 256 / 512: 98 / 90 / 89 us; 256 keeps smaller batches spread).
   u32 per = kWgMin;
   while ((u64)per * num_sms() * 2 < n) per *= 2;
-  const dim3 wb((unsigned)(((u64)n + per - 1) / per), 2);
+  const u64  blocks1 = ((u64)n + per - 1) / per;
+  const dim3 wb((unsigned)((blocks1 + kWgCluster - 1) / kWgCluster * kWgCluster), 2);
   mlp_wgrad_kernel<<<wb, kWgWarps * 32, 0, st>>>((const __half *)G2, (const __half *)H1, (const __half *)G1,
                                                  (const __half *)X, n, per, grad);
   g_launches++;
