@@ -275,14 +275,12 @@ int ensure_seed_scratch(oic_ctx *ctx, const SeedConfig &sc, bool wide, SeedScrat
 }
 
 struct AlignConfig {
-  int bandW;
   int warps;
   AlignCaps caps;
 };
 
 AlignConfig align_normal(const oic_ctx *c) {
   AlignConfig a;
-  a.bandW         = 512;
   a.warps         = c->nSM * align_warps_per_block();
   a.caps.arenaCap = 1 << 20;
   a.caps.rowCap   = 1 << 14;
@@ -417,7 +415,6 @@ int ensure_group_scratch(oic_ctx *ctx, const oic_tuning &t, bool huge, uint32_t 
   if (cells < (1u << 20)) return fail(ctx, OIC_ERR_NOMEM, "not enough device memory for the CTA-bin DP arena");
   caps.arenaCap = (int)std::min<uint64_t>(cells, 0x7fff0000ull);
   AlignConfig ac;
-  ac.bandW = caps.bandW;
   ac.warps = (int)ctas;
   ac.caps  = caps;
   if (ctx->dArena2.cap < (size_t)ctas * caps.arenaCap * sizeof(int)) ctx->dArena2.release();
@@ -450,7 +447,6 @@ int ensure_spec_scratch(oic_ctx *ctx, const oic_tuning &t, uint32_t &ctas, Align
   if (cells < (uint64_t)sw << 17) return fail(ctx, OIC_ERR_NOMEM, "not enough device memory for the CTA-bin DP arena");
   caps.arenaCap = (int)std::min<uint64_t>(cells / sw, 0x7fff0000ull);
   AlignConfig ac;
-  ac.bandW = caps.bandW;
   ac.warps = (int)ctas * sw;
   ac.caps  = caps;
   if (ctx->dArena2.cap < (size_t)ac.warps * caps.arenaCap * sizeof(int)) ctx->dArena2.release();
