@@ -315,7 +315,8 @@ static __device__ __noinline__ bool extend_proved(WarpDP &w, PairSmem &ps, const
 //
 // Every wait is bounded: an owner that waits too long for a result extends the node
 // itself, a helper that waits too long for its result to be taken leaves (its scratch
-// stays readable).
+// stays readable), and an owner that cannot close its pair leaves it, and the pairs that it
+// takes after it, to the CTA bin: a helper may still be in it.
 enum { kSlotFree = 0, kSlotRunning = 1, kSlotDone = 2, kSlotCancelled = 3 };
 constexpr unsigned char kNodeDead = 0, kNodeOpen = 1, kNodeOwner = 2, kNodeHelper = 3;   // kNodeHelper + h: helper h
 constexpr unsigned char kNodeProved = 255;   // collected pairs only: shown to have no overlap, still to be extended for the pair's figures
@@ -340,7 +341,13 @@ struct Team {
   TeamSlot slot[kAlignWarps];
 };
 
-constexpr int kLockTries = 1 << 22, kWaitTries = 1 << 24;
+#ifndef OIC_LOCK_TRIES
+#define OIC_LOCK_TRIES (1 << 22)   // of 64 ns at the least
+#endif
+#ifndef OIC_WAIT_TRIES
+#define OIC_WAIT_TRIES (1 << 24)   // of 100 ns or more
+#endif
+constexpr int kLockTries = OIC_LOCK_TRIES, kWaitTries = OIC_WAIT_TRIES;
 
 // Lock of a pair, taken by a warp (bounded: false when it could not be had).
 __device__ __forceinline__ bool team_lock(TeamPair &p) {
@@ -401,7 +408,8 @@ __device__ __forceinline__ void team_drop(Team &tm, int h) {
 }
 
 // Closes warp `me`'s pair: no new claims, outstanding ones dropped.  False when the lock
-// could not be had (the pair is closed all the same; its helpers give up by themselves).
+// could not be had: a helper may still claim a node of the pair, so neither the pair's fields
+// nor its node flags may be used again.
 __device__ __forceinline__ bool team_close(Team &tm, int me) {
   TeamPair &p   = tm.pair[me];
   const int lane = threadIdx.x & 31;
@@ -773,7 +781,10 @@ __device__ bool process_pair(WarpDP &w, PairSmem &ps, const ReadsDev &R, const T
       if (w.err) break;
     }
   }
-  if (open && !team_close(*tm, me)) w.err |= kErrInternal;
+  if (open && !team_close(*tm, me)) {
+    w.err |= kErrInternal;
+    w.cap.nodeCap = -1;   // no room for any pair from now on
+  }
   if (w.err) {
     w.cells  = cells0;
     w.slides = slides0;
