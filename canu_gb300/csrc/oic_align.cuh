@@ -1,11 +1,11 @@
 // oic_align.cuh -- warp-cooperative banded prefix edit distance (furthest-reaching
 // diagonals) and the per-read-pair driver around it.
 //
-// One warp owns one read pair.  Lanes own diagonals of the current error row, 32 at a
-// time; the previous row lives in a shared-memory buffer, every kept row is appended to
+// One warp owns one read pair.  Lanes own diagonals of the current error row, two each per
+// step of 64; the previous row lives in a shared-memory buffer, every kept row is appended to
 // the warp's traceback arena in HBM, and the slides compare 32 bases per step on the reads'
-// bit planes.  The arithmetic is the reference's exactly -- integer rows, the same band pruning against Edit_Match_Limit,
-// the same first-index tie breaks, and the branch-point test in IEEE double with
+// bit planes.  The arithmetic is the reference's exactly -- integer rows, the same band
+// pruning against Edit_Match_Limit, the same first-index tie breaks, and the branch-point test in IEEE double with
 // explicitly rounded multiply / subtract / divide (no FMA contraction), as an x86-64
 // build of canu computes it.
 #pragma once

@@ -6,8 +6,9 @@
 // reverse complement -- plus a parallel mask array with 0b11 at every N.  The DP reads the
 // same bases as bit planes (word i: the low bits of bases 32i .. 32i+31, then their high
 // bits, base 32i topmost), in which a comparison of 32 bases is four funnel shifts and two
-// logic instructions, and the first difference a count of leading zeros.  Reads start on a word boundary and are separated by one zero guard word,
-// so a 32-base window that runs off either end of a read stays inside the arrays.
+// logic instructions, and the first difference a count of leading zeros.  Reads start on a
+// word boundary and are separated by one zero guard word, so a 32-base window that runs off
+// either end of a read stays inside the arrays.
 #pragma once
 
 #include <cstdint>

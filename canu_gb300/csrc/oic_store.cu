@@ -11,8 +11,8 @@
 //
 // Here: one thread per input record writes both copies and their keep flags; a scan
 // compacts the kept copies; the library's radix sort orders them by (a_iid, b_iid) as
-// one key of as many bits as two IDs need (stable; 60,000 reads: 4 passes instead of 8); the rare runs of equal (a_iid, b_iid) are then ordered by the
-// data words; a gather writes the records in that order, and a histogram + scan of
+// one key of as many bits as two IDs need (stable; 60,000 reads: 4 passes instead of 8); the
+// rare runs of equal (a_iid, b_iid) are then ordered by the data words; a gather writes the records in that order, and a histogram + scan of
 // a_iid gives the first record of every read.
 //
 // Record words (ovFile's full record): a_iid, b_iid, dat0 >> 32, dat0, dat1 >> 32,
