@@ -291,8 +291,10 @@ __global__ void __launch_bounds__(kFwdWarps * 32) mlp_forward_kernel(const __hal
 // more tiles per warp.  The sums of w3, b3 and the loss go to memory once per cluster of four
 // blocks: an atomic per 128 samples rounded the whole sum four times as often as one per 512
 // (w3 at 60,000 samples: rms error over the sum of magnitudes 2.2e-7 and 1.2e-7, now 0.6e-7).
-// A step of 32,768 samples 82.7 -> 78.9 us, of 60,000 125.1 -> 126.2, of 1,000 51.7 -> 54.5
-// (waiting for the cluster's other blocks).
+// A step of 32,768 samples 82.7 -> 77.7 us, of 60,000 124.8 -> 123.2, of 1,000 51.5 -> 54.2
+// (two launches in clusters).  The blocks write their sums into the first one's shared memory
+// and leave; with the first one reading theirs, and a second barrier behind that, a step of
+// 32,768 samples took 1.4 us more.
 constexpr int kBwdWarps   = 8;
 constexpr int kBwdCluster = 4;
 
@@ -302,6 +304,7 @@ struct BwdSmem {
   float  dw3[kHid];
   float  db3;
   float  loss;
+  float  sums[kBwdCluster][kHid + 2];   // dw3, db3 and loss of the cluster's blocks, in its first
 };
 
 __global__ void __cluster_dims__(kBwdCluster, 1, 1) __launch_bounds__(kBwdWarps * 32)
@@ -309,6 +312,8 @@ __global__ void __cluster_dims__(kBwdCluster, 1, 1) __launch_bounds__(kBwdWarps 
                           const float *weight, u32 n, __half *G2, __half *G1, float *grad, float *loss) {
   extern __shared__ __align__(16) unsigned char bwdRaw[];
   BwdSmem &s     = *reinterpret_cast<BwdSmem *>(bwdRaw);
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();   // this block has started: its shared memory may be written
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   stage_rows(s.w2, kHS, prm + kOffW2, kHid, 0, kHid, kHid, threadIdx.x, blockDim.x);
   for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
@@ -403,19 +408,23 @@ __global__ void __cluster_dims__(kBwdCluster, 1, 1) __launch_bounds__(kBwdWarps 
     atomicAdd(&s.loss, lsum);
   }
   // Then over the cluster's blocks, by its first.
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  if (cluster.block_rank() == 0) {
-    const auto sum = [&](float *p) {
-      float v = 0.0f;
-      for (int r = 0; r < kBwdCluster; r++) v += *cluster.map_shared_rank(p, r);
-      return v;
-    };
-    for (int i = threadIdx.x; i < kHid; i += blockDim.x) atomicAdd(&grad[kOffW3 + i], sum(&s.dw3[i]));
-    if (threadIdx.x == 0) atomicAdd(&grad[kOffB3], sum(&s.db3));
-    if (threadIdx.x == 32 && loss) atomicAdd(loss, sum(&s.loss));
+  cluster.barrier_wait();
+  __syncthreads();
+  const int i = threadIdx.x;
+  if (i < kHid + 2)
+    cluster.map_shared_rank(s.sums[cluster.block_rank()], 0)[i] = i < kHid ? s.dw3[i] : i == kHid ? s.db3 : s.loss;
+  __syncwarp();
+  cluster.barrier_arrive();
+  if (cluster.block_rank() != 0) return;
+  cluster.barrier_wait();
+  if (i < kHid + 2) {
+    float v = 0.0f;
+#pragma unroll
+    for (int r = 0; r < kBwdCluster; r++) v += s.sums[r][i];
+    if (i < kHid) atomicAdd(&grad[kOffW3 + i], v);
+    else if (i == kHid) atomicAdd(&grad[kOffB3], v);
+    else if (loss) atomicAdd(loss, v);
   }
-  cluster.sync();   // no block leaves while its sums are read
 }
 
 // grad W[m][c] += sum_s G[s][m] * H[s][c]   (M = 128, N = NC columns of H)
@@ -441,7 +450,7 @@ constexpr int kWgCluster = 8;
 struct WgSmem {
   __half g[kWgRows * kHS];
   __half h[kWgRows * kHS];
-  float  bias[kHid];
+  float  bias[kWgCluster][kHid];   // of the cluster's blocks, in its first
 };
 
 template <int NC>
@@ -449,6 +458,8 @@ __device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __
                                             float *gradW, float *gradB) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   constexpr int NT = NC / 8;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();   // this block has started: its shared memory may be written
   float acc[NT][4], b0 = 0.0f, b1 = 0.0f, c0 = 0.0f, c1 = 0.0f;   // b, c: rows g and g + 8 of the fragments, this lane's samples
 #pragma unroll
   for (int i = 0; i < NT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
@@ -487,11 +498,13 @@ __device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __
     b0 += __shfl_xor_sync(0xffffffffu, b0, o);
     b1 += __shfl_xor_sync(0xffffffffu, b1, o);
   }
+  cluster.barrier_wait();
   if (t == 0) {
-    s.bias[m0 + g]     = b0;
-    s.bias[m0 + g + 8] = b1;
+    float *first  = cluster.map_shared_rank(s.bias[cluster.block_rank()], 0);
+    first[m0 + g]     = b0;
+    first[m0 + g + 8] = b1;
   }
-  cg::cluster_group cluster = cg::this_cluster();
+  __syncwarp();
   cluster.barrier_arrive();
   if (s0 < n) {
 #pragma unroll
@@ -503,13 +516,14 @@ __device__ __forceinline__ void wgrad_block(WgSmem &s, const __half *G, const __
       atomicAdd(&gradW[(m0 + g + 8) * NC + c + 1], acc[nt][3]);
     }
   }
+  if (cluster.block_rank() != 0) return;
   cluster.barrier_wait();
-  if (cluster.block_rank() == 0 && threadIdx.x < kHid) {
+  if (threadIdx.x < kHid) {
     float sum = 0.0f;
-    for (int r = 0; r < kWgCluster; r++) sum += *cluster.map_shared_rank(&s.bias[threadIdx.x], r);
+#pragma unroll
+    for (int r = 0; r < kWgCluster; r++) sum += s.bias[r][threadIdx.x];
     atomicAdd(&gradB[threadIdx.x], sum);
   }
-  cluster.sync();   // no block leaves while its sums are read
 }
 
 __global__ void __cluster_dims__(kWgCluster, 1, 1) __launch_bounds__(kWgWarps * 32) mlp_wgrad_kernel(const __half *G2, const __half *H1, const __half *G1,
